@@ -114,7 +114,7 @@ typedef struct {
                          * > 1 (HDR, e.g. 16) needs VCT_STORAGE_RGBA16F      */
   int32_t shadow_from_maps; /* 0 (default): shadow cones of the texture-unit
                          * sampler read packed alpha-only copies of the six
-                         * maps' chains (two fetches per step instead of
+                         * maps' chains (one fetch per step instead of
                          * three, identical values); 1: the six maps       */
   int32_t full_march;   /* 1: cones march their full length also outside the
                          * grid, as the reference's loop does; 0 (default):
@@ -134,9 +134,9 @@ typedef struct {
                          * marches all of its cones (the reference's rule).
                          * The FP32 software sampler always marches per
                          * pixel                                           */
-  int32_t trace_tile_rows; /* shared-far-field tracer: rows of a CTA's
-                         * 16-pixel-wide tile, 8, 16 or 32; 0 (default): 16.
-                         * The frame is the same for every value          */
+  int32_t trace_tile_rows; /* 0, 8, 16 or 32: accepted and without effect
+                         * (the tracer has one tile shape; the frame never
+                         * depended on it)                                */
   int32_t reserved[2];
 } vct_config;
 
@@ -482,18 +482,16 @@ void vct_batch_config_default(vct_batch_config* cfg);
  * binning, brick and trace launches (trace 1-3, or 0: one launch with one
  * CTA per 16 x 16 tile of every scene, not persistent), the persistent
  * trace's tile scheduling (1 = atomic tile queue, 0 = static stride), the
- * trace's form: 0 = one launch over all scenes, 1 = one launch of the
- * one-scene trace kernel per scene, spread over parallel streams (graph
- * branches), and the tile of the per-scene shared-far-field trace.  Every
- * shape renders the same frames. */
+ * trace's form: 0 = one launch over all scenes, 1 = the one-scene trace
+ * (two launches) per scene, spread over parallel streams (graph branches).
+ * Every shape renders the same frames. */
 typedef struct {
   int32_t bin_ctas_per_sm;
   int32_t bricks_ctas_per_sm;
   int32_t trace_ctas_per_sm;
   int32_t trace_dynamic;
   int32_t trace_per_scene;
-  int32_t trace_tile_rows;  /* per-scene shared-far-field trace: CTA tile 16 x 8,
-                             * 16 x 16 or 16 x 32 pixels (the same frame) */
+  int32_t trace_tile_rows;  /* 8, 16 or 32: accepted and without effect */
 } vct_batch_shape;
 
 typedef struct vct_batch vct_batch;

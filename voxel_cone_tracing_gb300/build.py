@@ -23,7 +23,7 @@ ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC,-ffp-contract=off", "-I", CSRC]
 # Per-file flags: the cone tracer fuses products and sums only where its
 # code says so, so that its frames do not change with the code's arrangement.
-FILE_FLAGS = {"k_trace.cu": ["-fmad=false"]}
+FILE_FLAGS = {"k_trace.cu": ["-fmad=false"], "k_trace_frame.cu": ["-fmad=false"]}
 # Extra nvcc flags (e.g. -DVCT_TRACE_MIN_BLOCKS=3 for tuning sweeps); the
 # library is rebuilt when they differ from the ones it was built with.
 EXTRA = os.environ.get("VCT_NVCC_FLAGS", "").split()

@@ -85,6 +85,10 @@ struct vct_batch {
   DevBuf<unsigned long long> vis;
   DevBuf<float4> gb_pos, gb_nrm;
   DevBuf<uchar4> frame;
+  // TraceWork of the per-scene trace, a slice per scene
+  DevBuf<float4> trace_far, trace_diffuse, trace_specular, trace_refracted;
+  DevBuf<float> trace_shadow;
+  std::vector<size_t> far_base, shadow_base;
   DevBuf<FrameStatus> d_status;
   HostBuf<FrameStatus> h_status;
   // execution
@@ -221,10 +225,11 @@ struct vct_batch {
       for (size_t i = 0; i < trace_order.size(); ++i) {
         const int s = trace_order[i];
         const SceneRes& r = *scenes[s];
-        TraceParams tp = r.tp;
-        tp.tile_rows = shape.trace_tile_rows;
-        VCT_CUDA(launch_trace(r.sp, h_cams.p[s], r.maps.ms, tp, gb_pos.p + px_base[s], gb_nrm.p + px_base[s],
-                              frame.p + px_base[s], nullptr, side[i % kSide], &launches));
+        const TraceWork tw = {trace_far.p ? trace_far.p + far_base[s] : nullptr, trace_diffuse.p + px_base[s],
+                              trace_specular.p + px_base[s], trace_refracted.p + px_base[s],
+                              trace_shadow.p + shadow_base[s]};
+        VCT_CUDA(launch_trace(r.sp, h_cams.p[s], r.maps.ms, r.tp, gb_pos.p + px_base[s], gb_nrm.p + px_base[s],
+                              frame.p + px_base[s], nullptr, r.maps.sched, tw, side[i % kSide], &launches));
       }
       for (int k = 0; k < kSide; ++k) {
         VCT_CUDA(cudaEventRecord(join_ev[k], side[k]));
@@ -453,7 +458,7 @@ vct_status build_batch(vct_batch* b, const vct_batch_scene* descs, uint32_t n) {
       for (int d = 0; d < 6; ++d)
         for (int l = 1; l <= 3; ++l) bm.surf[d][l] = ms.surf[d][l];
       bm.has_alpha = ms.alpha_tex[0] != 0;
-      for (int k = 0; k < 2 && bm.has_alpha; ++k)
+      for (int k = 0; k < kMaxAlpha && bm.has_alpha; ++k)
         for (int l = 1; l <= 3; ++l) bm.alpha[k][l] = ms.alpha_surf[k][l];
       for (int l = 1; l <= 3 && ms.skip_empty; ++l) bm.occ_raw[l] = ms.occ_raw[l];
     }
@@ -510,6 +515,19 @@ vct_status build_batch(vct_batch* b, const vct_batch_scene* descs, uint32_t n) {
   VCT_CHECK(b->gb_pos.ensure(px));
   VCT_CHECK(b->gb_nrm.ensure(px));
   VCT_CHECK(b->frame.ensure(px));
+  size_t far = 0, shadow = 0;
+  for (uint32_t i = 0; i < n; ++i) {
+    const SceneRes& r = *b->scenes[i];
+    b->far_base.push_back(far);
+    b->shadow_base.push_back(shadow);
+    far += trace_far_slots(r.W, r.H);
+    shadow += (size_t)r.W * r.H * std::max(r.sp.n_lights, 1);
+  }
+  if (b->cfg.far_share) VCT_CHECK(b->trace_far.ensure(far));
+  VCT_CHECK(b->trace_diffuse.ensure(px));
+  VCT_CHECK(b->trace_specular.ensure(px));
+  VCT_CHECK(b->trace_refracted.ensure(px));
+  VCT_CHECK(b->trace_shadow.ensure(shadow));
   VCT_CHECK(b->d_status.ensure(1));
   VCT_CHECK(b->h_status.ensure(1));
   std::memset(b->h_status.p, 0, sizeof(FrameStatus));
@@ -731,20 +749,15 @@ extern "C" vct_status vct_batch_autotune(vct_batch* b, int32_t frames, vct_batch
     }
     return VCT_OK;
   };
-  // The trace's form first, from the same starting point: one launch per
-  // scene (16x8 or, with shared far fields, 16x16 or 16x32 tiles), one
+  // The trace's form first, from the same starting point: per scene, one
   // launch with one CTA per tile, or one persistent launch (2 or 3 CTAs
   // per SM).
   {
     const BatchShape start = cur;
-    BatchShape forms[6];
+    BatchShape forms[4];
     int nf = 0;
-    for (int rows = 8; rows <= 32; rows *= 2) {
-      if (rows > 8 && !b->cfg.far_share) continue;
-      forms[nf] = start;
-      forms[nf].trace_per_scene = 1;
-      forms[nf++].trace_tile_rows = rows;
-    }
+    forms[nf] = start;
+    forms[nf++].trace_per_scene = 1;
     for (int c : {0, 2, 3}) {
       forms[nf] = start;
       forms[nf].trace_per_scene = 0;

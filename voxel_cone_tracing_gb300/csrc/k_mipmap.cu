@@ -113,13 +113,13 @@ __device__ __forceinline__ void aniso6_rgba16f(const uint2* ch, uint2* out) {
   }
 }
 
-// Texel (x, y, z) of level `level` of the alpha-only chains from the six
-// maps' RGBA8 texels v[0], v[stride], ..., v[5 * stride].
-__device__ __forceinline__ void write_alpha(const MapSet& ms, int level, int x, int y, int z, const uint32_t* v,
-                                            int stride) {
-  surf3Dwrite(make_uchar4(v[0] >> 24, v[stride] >> 24, v[2 * stride] >> 24, v[3 * stride] >> 24),
-              ms.alpha_surf[0][level], x * 4, y, z);
-  surf3Dwrite(make_uchar2(v[4 * stride] >> 24, v[5 * stride] >> 24), ms.alpha_surf[1][level], x * 2, y, z);
+// Texel (x, y, z) of level `level` of the alpha chains from the six maps'
+// texels v[0], v[stride], ..., v[5 * stride].
+template <class T>
+__device__ __forceinline__ void write_alpha(const MapSet& ms, int level, int x, int y, int z, const T* v, int stride) {
+#pragma unroll
+  for (int c = 0; c < kMaxAlpha; ++c)
+    surf3Dwrite(alpha_texel(v, stride, c), ms.alpha_surf[c][level], x * (int)sizeof(T), y, z);
 }
 
 // One pass: source level `src_level` (0 = the shared level 0) -> levels
@@ -261,8 +261,7 @@ __device__ __forceinline__ void mip_reduce(const MapSet& ms, int src_level, int 
           out[6 * b3 + r] = v;
           surf3Dwrite(v, ms.surf[6][dl], ((ox >> 1) + x) * Texel<STORAGE>::kBytes, (oy >> 1) + y, (oz >> 1) + z);
         }
-        if constexpr (STORAGE == VCT_STORAGE_RGBA8)
-          if (ms.alpha_tex[0]) write_alpha(ms, dl, (ox >> 1) + x, (oy >> 1) + y, (oz >> 1) + z, v6, 1);
+        if (ms.alpha_tex[0]) write_alpha(ms, dl, (ox >> 1) + x, (oy >> 1) + y, (oz >> 1) + z, v6, 1);
       }
       __syncthreads();
       cur = out;
@@ -283,7 +282,7 @@ __device__ __forceinline__ void mip_reduce(const MapSet& ms, int src_level, int 
       surf3Dwrite(v, ms.surf[d][dl], ((ox >> l) + x) * Texel<STORAGE>::kBytes, (oy >> l) + y, (oz >> l) + z);
     }
     __syncthreads();
-    if constexpr (NMAPS >= 6 && STORAGE == VCT_STORAGE_RGBA8) {
+    if constexpr (NMAPS >= 6) {
       if (ms.alpha_tex[0]) {
         // The alpha copies of this level, from the six maps in shared memory
         // (read only; the next level writes past them).
@@ -432,7 +431,7 @@ __global__ void __launch_bounds__(kThreads) k_mip_level_batch(BatchWork w, int l
       v[d] = reduce<STORAGE>(ch, d, NMAPS == 1);
       surf3Dwrite(v[d], ms.surf[d][level], x * Texel<STORAGE>::kBytes, y, z);
     }
-    if constexpr (NMAPS == 6 && STORAGE == VCT_STORAGE_RGBA8)
+    if constexpr (NMAPS == 6)
       if (ms.alpha_tex[0]) write_alpha(ms, level, x, y, z, v, 1);
   }
 }

@@ -848,7 +848,7 @@ __device__ __forceinline__ void brick_accumulate(const SceneParams& sp, int N, c
 // The brick holds whole 4^3, 2^3 and 1^3 blocks of levels 1-3, so its CTA
 // writes them from its level-0 texels in shared memory with the MipBuilder's
 // rule (vct_mip.cuh: exact integers for RGBA8, one fixed FP32 evaluation for
-// RGBA16F), plus the alpha-only chains (RGBA8) and the occupancy bytes of
+// RGBA16F), plus the alpha chains and the occupancy bytes of
 // those levels (a cell is occupied when its block of level 0 holds a
 // non-zero texel); the MipBuilder then starts from level 3.  This replaces
 // the first pass's re-read of level 0 (and the linear copy it read).
@@ -866,11 +866,12 @@ typedef BrickMipScratchT<VCT_STORAGE_RGBA8> BrickMipScratch;
 __device__ __forceinline__ bool texel_nonzero(uint32_t v) { return v != 0u; }
 __device__ __forceinline__ bool texel_nonzero(uint2 v) { return (v.x | v.y) != 0u; }
 
-__device__ __forceinline__ void brick_alpha(const BrickMips& bm, int level, int x, int y, int z, const uint32_t* v,
+template <class T>
+__device__ __forceinline__ void brick_alpha(const BrickMips& bm, int level, int x, int y, int z, const T* v,
                                             int stride) {
-  surf3Dwrite(make_uchar4(v[0] >> 24, v[stride] >> 24, v[2 * stride] >> 24, v[3 * stride] >> 24),
-              bm.alpha[0][level], x * 4, y, z);
-  surf3Dwrite(make_uchar2(v[4 * stride] >> 24, v[5 * stride] >> 24), bm.alpha[1][level], x * 2, y, z);
+#pragma unroll
+  for (int c = 0; c < kMaxAlpha; ++c)
+    surf3Dwrite(alpha_texel(v, stride, c), bm.alpha[c][level], x * (int)sizeof(T), y, z);
 }
 
 __device__ __forceinline__ void brick_occ(const BrickMips& bm, int N, int level, int x, int y, int z, bool any) {
@@ -917,9 +918,8 @@ __device__ void brick_mips(const BrickMips& bm, int N, const int b3[3], BrickMip
   }
   __syncthreads();
   if (t < 64) {
-    if constexpr (STORAGE == VCT_STORAGE_RGBA8)
-      if (bm.has_alpha) brick_alpha(bm, 1, b3[0] * 4 + (t & 3), b3[1] * 4 + ((t >> 2) & 3), b3[2] * 4 + (t >> 4),
-                                    &scr.l1[0][t], 64);
+    if (bm.has_alpha) brick_alpha(bm, 1, b3[0] * 4 + (t & 3), b3[1] * 4 + ((t >> 2) & 3), b3[2] * 4 + (t >> 4),
+                                  &scr.l1[0][t], 64);
     return;
   }
   if (t >= 96) return;
@@ -940,10 +940,9 @@ __device__ void brick_mips(const BrickMips& bm, int N, const int b3[3], BrickMip
   }
   __syncwarp();
   if (lane < 8) {
-    if constexpr (STORAGE == VCT_STORAGE_RGBA8)
-      if (bm.has_alpha)
-        brick_alpha(bm, 2, b3[0] * 2 + (lane & 1), b3[1] * 2 + ((lane >> 1) & 1), b3[2] * 2 + (lane >> 2),
-                    &scr.l2[0][lane], 8);
+    if (bm.has_alpha)
+      brick_alpha(bm, 2, b3[0] * 2 + (lane & 1), b3[1] * 2 + ((lane >> 1) & 1), b3[2] * 2 + (lane >> 2),
+                  &scr.l2[0][lane], 8);
   } else if (lane < 14) {  // level 3: the brick's one texel of map d
     const int d = lane - 8;
     const T v = brick_mip_texel(scr.l2[d], 2, 0, 0, 0, d);
@@ -955,15 +954,14 @@ __device__ void brick_mips(const BrickMips& bm, int N, const int b3[3], BrickMip
     brick_occ(bm, N, 3, b3[0], b3[1], b3[2], any);
   }
   __syncwarp();
-  if constexpr (STORAGE == VCT_STORAGE_RGBA8)
-    if (lane == 0 && bm.has_alpha) brick_alpha(bm, 3, b3[0], b3[1], b3[2], scr.l3, 1);
+  if (lane == 0 && bm.has_alpha) brick_alpha(bm, 3, b3[0], b3[1], b3[2], scr.l3, 1);
 }
 
 // Levels 1-3 of an empty brick: zeros (the texels and the occupancy).
 template <int STORAGE>
 __device__ void brick_mips_zero(const BrickMips& bm, int N, const int b3[3]) {
   const int t = threadIdx.x;
-  const uint32_t zero[6] = {0u, 0u, 0u, 0u, 0u, 0u};
+  const typename BrickMipScratchT<STORAGE>::T zero[6] = {};
   int level = 0, x = 0, y = 0, z = 0;
   if (t < 64) {
     level = 1;
@@ -987,8 +985,7 @@ __device__ void brick_mips_zero(const BrickMips& bm, int N, const int b3[3]) {
     if constexpr (STORAGE == VCT_STORAGE_RGBA16F) surf3Dwrite(make_uint2(0u, 0u), bm.surf[d][level], x * 8, y, z);
     else surf3Dwrite(0u, bm.surf[d][level], x * 4, y, z);
   }
-  if constexpr (STORAGE == VCT_STORAGE_RGBA8)
-    if (bm.has_alpha) brick_alpha(bm, level, x, y, z, zero, 1);
+  if (bm.has_alpha) brick_alpha(bm, level, x, y, z, zero, 1);
   brick_occ(bm, N, level, x, y, z, false);
 }
 

@@ -220,8 +220,10 @@ struct HeavyStore {
 struct MapStore {
   cudaArray_t l0_arr = nullptr;
   cudaMipmappedArray_t dir_arr[kMaxMaps] = {};
-  cudaMipmappedArray_t alpha_arr[2] = {};
+  cudaMipmappedArray_t alpha_arr[kMaxAlpha] = {};
   void* occ_mem = nullptr;  // occupancy grids of empty-space skipping
+  ConeSchedules* sched_mem = nullptr;
+  ConeSchedules sched = {};  // host copy (launch_trace)
   MapSet ms = {};
 
   MapStore() = default;
@@ -239,7 +241,7 @@ struct MapStore {
       if (dir_arr[d]) cudaFreeMipmappedArray(dir_arr[d]);
       dir_arr[d] = nullptr;
     }
-    for (int k = 0; k < 2; ++k) {
+    for (int k = 0; k < kMaxAlpha; ++k) {
       if (ms.alpha_tex[k]) cudaDestroyTextureObject(ms.alpha_tex[k]);
       for (int l = 0; l < kMaxLevels; ++l)
         if (ms.alpha_surf[k][l]) cudaDestroySurfaceObject(ms.alpha_surf[k][l]);
@@ -250,6 +252,8 @@ struct MapStore {
     l0_arr = nullptr;
     if (occ_mem) cudaFree(occ_mem);
     occ_mem = nullptr;
+    if (sched_mem) cudaFree(sched_mem);
+    sched_mem = nullptr;
     std::memset(&ms, 0, sizeof(ms));
   }
 
@@ -301,12 +305,8 @@ struct MapStore {
     td.mipmapFilterMode = cudaFilterModeLinear;
     VCT_CUDA(cudaCreateTextureObject(&ms.l0_tex, &rd, &td, nullptr));
     for (int d = 0; d < nmaps && L > 1; ++d) VCT_CHECK(chain(r, L, desc, td, &dir_arr[d], ms.surf[d], &ms.tex[d]));
-    if (alpha_chains && nmaps >= 6 && storage == VCT_STORAGE_RGBA8 && L > 1) {
-      const cudaChannelFormatDesc d4 = cudaCreateChannelDesc(8, 8, 8, 8, cudaChannelFormatKindUnsigned);
-      const cudaChannelFormatDesc d2 = cudaCreateChannelDesc(8, 8, 0, 0, cudaChannelFormatKindUnsigned);
-      VCT_CHECK(chain(r, L, d4, td, &alpha_arr[0], ms.alpha_surf[0], &ms.alpha_tex[0]));
-      VCT_CHECK(chain(r, L, d2, td, &alpha_arr[1], ms.alpha_surf[1], &ms.alpha_tex[1]));
-    }
+    for (int k = 0; k < kMaxAlpha && alpha_chains && nmaps >= 6 && L > 1; ++k)
+      VCT_CHECK(chain(r, L, desc, td, &alpha_arr[k], ms.alpha_surf[k], &ms.alpha_tex[k]));
     ms.N = (int)r;
     ms.L = L;
     ms.nmaps = nmaps;
@@ -342,6 +342,12 @@ struct MapStore {
         ms.occ3[c] = reinterpret_cast<uint32_t*>(base + o);
         o += s * s * (size_t)ms.occ_wpr[c] * 4;
       }
+      // (before the owner's streams, which do not wait for this one, use it)
+      VCT_CUDA(cudaMalloc(&sched_mem, sizeof(ConeSchedules)));
+      VCT_CUDA(launch_cone_schedules(ms, sched_mem, cudaStreamLegacy));
+      VCT_CUDA(cudaMemcpyAsync(&sched, sched_mem, sizeof(ConeSchedules), cudaMemcpyDeviceToHost, cudaStreamLegacy));
+      VCT_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
+      ms.sched = sched_mem;
     }
     set_full_march(false);
     return VCT_OK;
@@ -415,6 +421,8 @@ struct vct_renderer {
   DevBuf<float4> gb_pos, gb_nrm;
   DevBuf<uchar4> frame;
   DevBuf<float4> frame_f32;
+  DevBuf<float4> trace_far, trace_px;  // TraceWork (trace_px: its three per-pixel arrays)
+  DevBuf<float> trace_shadow;
   bool frame_pending = false;
   bool have_frame = false;
   int launches = 0;  // engine kernels of the last encoded frame
@@ -582,6 +590,10 @@ struct vct_renderer {
     VCT_CHECK(gb_nrm.ensure(px));
     VCT_CHECK(frame.ensure(px));
     if (cfg.keep_float_frame) VCT_CHECK(frame_f32.ensure(px));
+    if (cfg.sampler == VCT_SAMPLER_HW) {
+      if (cfg.far_share) VCT_CHECK(trace_far.ensure(trace_far_slots(W, H)));
+      VCT_CHECK(trace_px.ensure(3 * px));
+    }
     VCT_CHECK(d_status.ensure(1));
     VCT_CHECK(h_status.ensure(1));
     std::memset(h_status.p, 0, sizeof(FrameStatus));
@@ -712,7 +724,7 @@ struct vct_renderer {
       for (int d = 0; d < 6; ++d)
         for (int l = 1; l <= 3; ++l) bm.surf[d][l] = ms.surf[d][l];
       bm.has_alpha = ms.alpha_tex[0] != 0;
-      for (int k = 0; k < 2 && bm.has_alpha; ++k)
+      for (int k = 0; k < kMaxAlpha && bm.has_alpha; ++k)
         for (int l = 1; l <= 3; ++l) bm.alpha[k][l] = ms.alpha_surf[k][l];
       for (int l = 1; l <= 3 && ms.skip_empty; ++l) bm.occ_raw[l] = ms.occ_raw[l];
       vb.mips = &bm;
@@ -805,8 +817,12 @@ struct vct_renderer {
       VCT_CUDA(cudaStreamWaitEvent(stream, ev_join, 0));
     }
     VCT_CUDA(cudaEventRecord(ev[3], stream));
+    if (cfg.sampler == VCT_SAMPLER_HW && tp.enable_direct && tp.enable_shadow)
+      VCT_CHECK(trace_shadow.ensure((size_t)W * H * std::max(sp.n_lights, 1)));
+    const size_t px = (size_t)W * H;
+    const TraceWork tw = {trace_far.p, trace_px.p, trace_px.p + px, trace_px.p + 2 * px, trace_shadow.p};
     VCT_CUDA(launch_trace(sp, cp, ms, tp, gb_pos.p, gb_nrm.p, frame.p, cfg.keep_float_frame ? frame_f32.p : nullptr,
-                          stream, &launches));
+                          maps.sched, tw, stream, &launches));
     judge_pending = tp.diffuse_in != nullptr && judge_stride > 0;
     if (judge_pending) {
       const int ox = (int)((judge_frame * 5u) % (uint32_t)judge_stride);
@@ -884,7 +900,6 @@ struct vct_renderer {
     tp.mip_mode = cfg.mip_mode;
     tp.diffuse_in = nullptr;
     tp.far_share = cfg.far_share;
-    tp.tile_rows = cfg.trace_tile_rows;
     return tp;
   }
 };

@@ -13,6 +13,7 @@ constexpr int kMaxLights = 10;   // MAX_POINT_LIGHTS, voxelize.frag:40,128
 constexpr int kMaxLevels = 7;    // create_tex_3d(res,res,res,7), renderer.cpp:186
 constexpr int kBrick = 8;        // voxelizer brick edge (voxels)
 constexpr int kMaxMaps = 7;  // six directional maps + the isotropic one (VCT_MIP_BOTH)
+constexpr int kMaxAlpha = 4;  // alpha chains: the x and y signs of a direction
 // Internal storage mode of the voxelizer: per-voxel attribute grids for
 // deferred light injection instead of shaded level-0 radiance.
 constexpr int kStorageAttr = 2;
@@ -108,11 +109,13 @@ struct MapSet {
   cudaTextureObject_t l0_tex;                    // linear, normalized coords, border 0
   cudaSurfaceObject_t surf[kMaxMaps][kMaxLevels];  // level l >= 1 of map d
   cudaTextureObject_t tex[kMaxMaps];             // mipmapped chain (base = level 1)
-  // Alpha-only copies of the six chains for shadow cones (anisotropic RGBA8;
-  // 0 when absent): levels 1..L-1 of (a-x, a+x, a-y, a+y) as RGBA8 in
-  // alpha_tex[0] and of (a-z, a+z) as RG8 in alpha_tex[1].
-  cudaSurfaceObject_t alpha_surf[2][kMaxLevels];
-  cudaTextureObject_t alpha_tex[2];
+  // Alpha-only copies of the six chains for shadow cones (anisotropic maps;
+  // 0 when absent): chain c holds levels 1..L-1 of (a-x or a+x, a-y or a+y,
+  // a-z, a+z) in the maps' own texel format, bit 0 of c choosing the x map
+  // and bit 1 the y map, so that one fetch serves the three maps of any
+  // direction.
+  cudaSurfaceObject_t alpha_surf[kMaxAlpha][kMaxLevels];
+  cudaTextureObject_t alpha_tex[kMaxAlpha];
   // A cone moving away from the grid stops once its sample position is more
   // than this far outside [0,1] along that axis (+inf: never).
   float exit_margin;
@@ -134,6 +137,58 @@ struct MapSet {
   uint32_t* occ[kMaxLevels];
   uint32_t* occ3[kMaxLevels];
   int occ_wpr[kMaxLevels];
+  // Step schedules of the cones of fixed aperture (ConeSchedules, built by
+  // launch_cone_schedules; null without occupancy grids).
+  const struct ConeSchedules* sched;
+};
+
+// Step schedules.  The march distances of a cone of fixed aperture (first
+// step at three voxels) do not depend on the pixel, so they, their lods and
+// the occupancy tests' constants are laid out once per map set.  A test at
+// distance d looks up one bit of an occupancy level, `base` being a word
+// offset from occ[1] with the common exponent bits of the cell numbers
+// (found as the low bits of 2^23 + cell) folded in.
+
+// Four steps of a shadow cone (aperture 0.1), tested against occ3: cell =
+// floor(saturate(origin + dir * d) * cells), word = z * zmul + y * ymul +
+// (x >> 5) + base.
+struct alignas(16) ShadowGroup {
+  float mid, cells;          // one test that covers all four steps (cells 0: none)
+  uint32_t base, zmul, ymul;
+  float next;                // first distance of the next group (+inf: the last one)
+  float cells1;              // the steps' own tests
+  uint32_t base1, zmul1, ymul1;
+  float pad[2];
+  alignas(16) float dist[4];
+  alignas(16) float lod[4];
+};
+constexpr int kShadowGroups = 40;
+struct ShadowSchedule {
+  ShadowGroup group[kShadowGroups];
+};
+
+// One step of a diffuse cone, tested against occ in 1/256 cells: t =
+// clamp(coordinate, lo, 1) * cells + offset, rounded down (cone_empty).
+struct alignas(16) ConeStep {
+  float dist, lod;
+  float cells;  // 256 * cells per unit (0: the step is not tested)
+  float lo;
+  uint32_t base, zmul, ymul;
+  float pad;
+};
+constexpr int kConeSteps = 40;
+struct ConeSchedule {
+  ConeStep step[kConeSteps];  // the last one's distance is +inf
+};
+
+// Directions of the five side cones of VCT_CONES_SIX60 around the normal.
+struct ConeRing {
+  float cphi[5], sphi[5];
+};
+struct ConeSchedules {
+  ShadowSchedule shadow;
+  ConeSchedule cone[2];  // by cone set
+  ConeRing ring;
 };
 
 // Levels 1-3 of the six RGBA8 directional chains written by the brick
@@ -145,7 +200,7 @@ struct MapSet {
 constexpr bool kFuseBrickMips = VCT_FUSE_BRICK_MIPS != 0;
 struct BrickMips {
   cudaSurfaceObject_t surf[6][4];   // [map][level 1..3]
-  cudaSurfaceObject_t alpha[2][4];  // [chain][level 1..3] (has_alpha)
+  cudaSurfaceObject_t alpha[kMaxAlpha][4];  // [chain][level 1..3] (has_alpha)
   uint8_t* occ_raw[4];              // [level 1..3] (null: no occupancy)
   uint8_t* dirty;  // (set by launch_voxelize from VoxBuffers::dirty)
   int has_alpha;
@@ -205,10 +260,18 @@ struct TraceParams {
   // Texture-unit sampler: pixel groups share the far fields of their diffuse
   // cones (vct_config::far_share).
   int far_share;
-  // Rows of a CTA's 16-pixel-wide tile of the shared-far-field tracer: 8,
-  // 16 (0 means 16) or 32.  The frame is the same for every value.
-  int tile_rows;
 };
+
+// Work arrays between the passes of one frame's trace (launch_trace).  Every
+// frame that may be in flight at the same time has its own.
+struct TraceWork {
+  float4* far;        // trace_far_slots(W, H): the groups' far fields
+  float4* diffuse;    // W * H: the diffuse term
+  float4* specular;   // W * H: the specular cone
+  float4* refracted;  // W * H: the refracted cone
+  float* shadow;      // W * H per light: occlusion of its shadow cone
+};
+inline size_t trace_far_slots(int W, int H) { return (size_t)((W + 3) / 4) * (size_t)((H + 1) / 2) * 9; }
 
 // ---- batched rendering (api_batch.cu) --------------------------------------
 // One scene of a batch, device-resident.  Scenes own their voxel maps; the
@@ -287,8 +350,8 @@ struct BatchShape {
   int bricks_ctas_per_sm;
   int trace_ctas_per_sm;
   int trace_dynamic;   // 1: tiles from an atomic queue; 0: static stride
-  int trace_per_scene; // 1: one launch of the one-scene trace kernel per scene
-  int trace_tile_rows; // 8, 16 or 32: CTA tile rows of the per-scene shared-far-field trace
+  int trace_per_scene; // 1: the one-scene trace (launch_trace) per scene
+  int trace_tile_rows; // 8, 16 or 32 (accepted; the per-scene trace has one tile shape)
 };
 
 // ---- learned diffuse term (k_mlp.cu) --------------------------------------
@@ -336,9 +399,18 @@ cudaError_t launch_mipmap(const MapSet& ms, int mip_mode, cudaStream_t st, int* 
                           FrameStatus* status = nullptr, int first_level = 0);
 cudaError_t launch_gbuffer(const SceneParams& sp, const CameraParams& cp, const RasterBuffers& rb,
                            cudaStream_t st, int* launches);
+// The step schedules of the cones of fixed aperture for ms (ms.N, ms.L and
+// its occupancy layout).  launch_trace takes them from the host: its kernels'
+// steps are warp-uniform, so they read them as kernel parameters.
+cudaError_t launch_cone_schedules(const MapSet& ms, ConeSchedules* out, cudaStream_t st);
 cudaError_t launch_trace(const SceneParams& sp, const CameraParams& cp, const MapSet& ms, const TraceParams& tp,
                          const float4* gb_pos, const float4* gb_nrm, uchar4* frame, float4* frame_f32,
-                         cudaStream_t st, int* launches);
+                         const ConeSchedules& sched, const TraceWork& tw, cudaStream_t st, int* launches);
+// A thread per pixel and everything in one kernel: the FP32 software sampler
+// and the voxel debug view.
+cudaError_t launch_trace_px(const SceneParams& sp, const CameraParams& cp, const MapSet& ms, const TraceParams& tp,
+                            const float4* gb_pos, const float4* gb_nrm, uchar4* frame, float4* frame_f32,
+                            cudaStream_t st, int* launches);
 // Exclusive scan of n u32 values into out[0..n] (out[n] = total); tmp must
 // hold scan_tmp_words(n) words.
 size_t scan_tmp_words(size_t n);

@@ -127,4 +127,17 @@ __device__ __forceinline__ uint2 aniso_rgba16f_dir(int d, Child child) {
   return finish16(acc);
 }
 
+// ---- alpha chains -----------------------------------------------------------
+// Texel of alpha chain c (x sign c & 1, y sign c >> 1) from the six maps'
+// texels v[0], v[stride], ..., v[5 * stride]: (a of -x or +x, a of -y or +y,
+// a-z, a+z), in the maps' own format.
+__device__ __forceinline__ uint32_t alpha_texel(const uint32_t* v, int stride, int c) {
+  return (v[(c & 1) * stride] >> 24) | (v[(2 + (c >> 1)) * stride] >> 24) << 8 | (v[4 * stride] >> 24) << 16 |
+         (v[5 * stride] & 0xff000000u);
+}
+__device__ __forceinline__ uint2 alpha_texel(const uint2* v, int stride, int c) {
+  return make_uint2(v[(c & 1) * stride].y >> 16 | (v[(2 + (c >> 1)) * stride].y & 0xffff0000u),
+                    v[4 * stride].y >> 16 | (v[5 * stride].y & 0xffff0000u));
+}
+
 }  // namespace vct
