@@ -85,10 +85,9 @@ vct_status adam_step(vct_renderer* r, float lr) {
   a.c1 = (float)(1.0 / (1.0 - std::pow(0.9, m.adam_t)));
   a.c2 = (float)(1.0 / (1.0 - std::pow(0.99, m.adam_t)));
   a.l2 = 1e-6f;
-  VCT_CUDA(launch_adam(m.w.p, m.w_grad.p, m.w_m.p, m.w_v.p, m.w_bf.p, kMlpWeights, a, r->stream));
-  a.l2 = 0.0f;
-  VCT_CUDA(launch_adam(m.table.p, m.table_grad.p, m.table_m.p, m.table_v.p, m.table_bf.p, m.table_floats(), a,
-                       r->stream));
+  const AdamArray table = {m.table.p, m.table_grad.p, m.table_m.p, m.table_v.p, m.table_bf.p, m.table_floats()};
+  const AdamArray w = {m.w.p, m.w_grad.p, m.w_m.p, m.w_v.p, m.w_bf.p, (size_t)kMlpWeights};
+  VCT_CUDA(launch_adam(table, w, a, r->stream));
   return VCT_OK;
 }
 
@@ -98,19 +97,23 @@ vct_status train_loop(vct_renderer* r, const vct_mlp_desc& d, vct_mlp_report* re
   const uint32_t steps = d.steps ? d.steps : 1;
   const uint32_t batch = std::max<uint32_t>(16, std::min(d.batch ? d.batch : (1u << 18), m.n_samples));
   VCT_CHECK(m.loss.ensure(steps));
+  VCT_CHECK(m.work.ensure(mlp_train_words((int)batch)));
   VCT_CUDA(cudaMemsetAsync(m.loss.p, 0, steps * sizeof(float), r->stream));
+  VCT_CHECK(m.pos.ensure(3 * (size_t)m.n_samples));
   const MlpParams p = m.params();
   cudaEvent_t e0, e1;
   VCT_CUDA(cudaEventCreate(&e0));
   VCT_CUDA(cudaEventCreate(&e1));
   VCT_CUDA(cudaEventRecord(e0, r->stream));
+  VCT_CUDA(launch_mlp_positions(m.samples.p, (int)m.n_samples, m.pos.p, r->stream));
   for (uint32_t s = 0; s < steps; ++s) {
     MlpBatch b;
     b.samples = m.samples.p;
+    b.pos = m.pos.p;
     b.total = (int)m.n_samples;
     b.first = (int)(((uint64_t)s * batch) % m.n_samples);
     b.n = (int)batch;
-    VCT_CUDA(launch_mlp_train(p, b, m.loss.p + s, r->stream));
+    VCT_CUDA(launch_mlp_train(p, b, m.work.p, m.loss.p + s, r->stream));
     // Constant for the first half of the steps, then decaying geometrically
     // to a tenth (the optimiser settles instead of ending on a noisy step).
     const double t = steps > 1 ? std::max(0.0, ((double)s - 0.5 * steps) / (0.5 * steps)) : 0.0;
@@ -324,16 +327,20 @@ extern "C" vct_status vct_mlp_gradients(vct_renderer* r, const float* samples, u
   DevBuf<float> in, l;
   VCT_CHECK(in.ensure((size_t)n * 12));
   VCT_CHECK(l.ensure(1));
+  VCT_CHECK(m.work.ensure(mlp_train_words((int)n)));
   VCT_CUDA(cudaMemcpyAsync(in.p, samples, (size_t)n * 12 * sizeof(float), cudaMemcpyHostToDevice, r->stream));
   VCT_CUDA(cudaMemsetAsync(l.p, 0, sizeof(float), r->stream));
   VCT_CUDA(cudaMemsetAsync(m.w_grad.p, 0, kMlpWeights * sizeof(float), r->stream));
   VCT_CUDA(cudaMemsetAsync(m.table_grad.p, 0, m.table_floats() * sizeof(float), r->stream));
+  VCT_CHECK(m.pos.ensure(3 * (size_t)n));
+  VCT_CUDA(launch_mlp_positions(in.p, (int)n, m.pos.p, r->stream));
   MlpBatch b;
   b.samples = in.p;
+  b.pos = m.pos.p;
   b.first = 0;
   b.n = (int)n;
   b.total = (int)n;
-  VCT_CUDA(launch_mlp_train(m.params(), b, l.p, r->stream));
+  VCT_CUDA(launch_mlp_train(m.params(), b, m.work.p, l.p, r->stream));
   if (loss) VCT_CUDA(cudaMemcpyAsync(loss, l.p, sizeof(float), cudaMemcpyDeviceToHost, r->stream));
   if (dweights)
     VCT_CUDA(cudaMemcpyAsync(dweights, m.w_grad.p, kMlpWeights * sizeof(float), cudaMemcpyDeviceToHost, r->stream));

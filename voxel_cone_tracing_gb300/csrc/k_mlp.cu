@@ -10,15 +10,9 @@
 // (samples / pixels); a layer's FP32 accumulator fragments are repacked in
 // registers into the next layer's BF16 A fragments (the D layout of
 // m16n8 tiles 2j, 2j+1 is the A layout of k-tile j), so activations never
-// leave registers.  Weights live in shared memory as [out][in] (forward B
-// operands) and [in][out] (backward B operands), rows padded to 72 bf16 so
-// that the fragment loads are bank-conflict free.
-// Training: per 16-row tile the warp runs forward, the MSE gradient, the
-// backward pass (activation gradients by mma, ReLU masks from the stored
-// forward fragments), the weight gradients dW_l = dH_l^T X_l by mma with
-// movmatrix-transposed fragments (accumulated in shared memory, flushed once
-// per CTA) and scatters the input gradient of the 32 hash features to the
-// table gradient (float2 atomics).  Adam runs as a separate elementwise pass.
+// leave registers.  Weights live in shared memory as [out][in], rows padded
+// to 72 bf16 so that the fragment loads are bank-conflict free.  (Training:
+// below, at its kernels.)  Adam runs as a separate elementwise pass.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -33,8 +27,6 @@ namespace {
 
 constexpr int kWS = 72;        // padded smem row stride of a 64-wide bf16 matrix
 constexpr int kWSw = kWS / 2;  // ... in 32-bit words
-constexpr int kW5TS = 24;      // padded row stride of W5^T ([64 in][16 out])
-constexpr int kDWS = 72;       // padded row stride of the fp32 dW accumulators
 
 __device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
   asm volatile(
@@ -42,12 +34,6 @@ __device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], 
       "{%0,%1,%2,%3};\n"
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-
-__device__ __forceinline__ uint32_t trans8x8(uint32_t x) {
-  uint32_t y;
-  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;\n" : "=r"(y) : "r"(x));
-  return y;
 }
 
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
@@ -73,6 +59,12 @@ __device__ __forceinline__ uint32_t grid_index(const MlpParams& p, int l, int cx
   return ((uint32_t)cx * 1u ^ (uint32_t)cy * 2654435761u ^ (uint32_t)cz * 805459861u) & ((1u << p.log2_table) - 1u);
 }
 
+// Entries of level l that grid_index can name.
+__host__ __device__ __forceinline__ uint32_t level_entries(const MlpParams& p, int l) {
+  const uint32_t r = (uint32_t)p.res[l] + 1u;
+  return ((p.dense_mask >> l) & 1) ? r * r * r : 1u << p.log2_table;
+}
+
 struct Corners {
   uint32_t idx[8];
   float w[8];
@@ -92,7 +84,20 @@ __device__ __forceinline__ void level_corners(const MlpParams& p, int l, V3 pos,
   }
 }
 
-// Hash features of one (row, level) pair.
+// Hash features of one (row, level) pair; `tab`: the level's entries (global
+// or shared memory).  (Loading a pair of corners along x as one 8-byte word
+// where they are neighbours, 6 loads instead of 8, was slower: 432 -> 465 us
+// for the bench frame's inference, whose encoders are bound by instructions.)
+__device__ __forceinline__ float2 corner_features(const Corners& c, const uint32_t* tab) {
+  float f0 = 0.f, f1 = 0.f;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const uint32_t v = tab[c.idx[k]];
+    f0 += c.w[k] * bf_lo(v);
+    f1 += c.w[k] * bf_hi(v);
+  }
+  return make_float2(f0, f1);
+}
 __device__ __forceinline__ float2 level_features(const MlpParams& p, int l, V3 pos) {
   Corners c;
   level_corners(p, l, pos, c);
@@ -112,13 +117,7 @@ struct SmemW {
   uint32_t w[4][64 * kWSw];  // W1..W4 [out][in]
   uint32_t w5[16 * kWSw];    // W5 [out 16][in 64]
 };
-// ... and their transposes for the backward pass.
-struct SmemWT {
-  uint32_t wt[4][64 * kWSw];     // W1^T..W4^T [in][out]
-  uint32_t w5t[64 * kW5TS / 2];  // W5^T [in 64][out 16]
-};
-
-__device__ void load_weights(const __nv_bfloat16* __restrict__ wg, SmemW& s, SmemWT* st) {
+__device__ void load_weights(const __nv_bfloat16* __restrict__ wg, SmemW& s) {
   const unsigned short* g = reinterpret_cast<const unsigned short*>(wg);
   unsigned short* w = reinterpret_cast<unsigned short*>(s.w);
   unsigned short* w5 = reinterpret_cast<unsigned short*>(s.w5);
@@ -127,15 +126,6 @@ __device__ void load_weights(const __nv_bfloat16* __restrict__ wg, SmemW& s, Sme
     w[l * 64 * kWS + o * kWS + k] = g[i];
   }
   for (int i = threadIdx.x; i < 16 * 64; i += blockDim.x) w5[(i >> 6) * kWS + (i & 63)] = g[4 * 4096 + i];
-  if (st) {
-    unsigned short* wt = reinterpret_cast<unsigned short*>(st->wt);
-    unsigned short* w5t = reinterpret_cast<unsigned short*>(st->w5t);
-    for (int i = threadIdx.x; i < 4 * 64 * 64; i += blockDim.x) {
-      const int l = i >> 12, o = (i >> 6) & 63, k = i & 63;
-      wt[l * 64 * kWS + k * kWS + o] = g[i];
-    }
-    for (int i = threadIdx.x; i < 16 * 64; i += blockDim.x) w5t[(i & 63) * kW5TS + (i >> 6)] = g[4 * 4096 + i];
-  }
 }
 
 // Fill the warp's 16 x 64 input tile E (bf16, stride kWS) for rows whose
@@ -268,52 +258,184 @@ __device__ __forceinline__ void layer_out(const uint32_t (&a)[4][4], const uint3
 }
 
 // ------------------------------------------------------------- training ----
-struct TrainSmem {
-  SmemW w;
-  SmemWT wt;
-  float dw[4][64 * kDWS];
-  float dw5[16 * kDWS];
-  unsigned short E[8][16 * kWS];
-  float pos[8][16][3];
-};
+// A step is three passes, so that the parts that wait for memory run with
+// every warp an SM holds, and the part that multiplies runs from shared
+// memory:
+//   k_mlp_encode  -- the rows' inputs: a thread per (row, level) gathers its
+//                    eight corners and packs two bf16 features;
+//   k_mlp_train   -- forward, loss, backward and weight gradients over
+//                    256-row tiles, on the tensor cores;
+//   k_mlp_scatter -- a thread per (row, level) adds the gradient of its
+//                    features to its eight corners.
+// Between them, word-major (a warp's lanes are neighbouring rows): kMlpInputs
+// words a row (16 of hash features, 4 of normal, albedo and the constant),
+// then 16 float2 of feature gradients.
+// In one kernel (8 warps an SM, the registers of the backward pass held
+// through the gathers, each warp adding its own 16 rows' weight gradients to
+// shared memory with atomics, 544 a lane and tile) a step of 2^18 rows took
+// 838 us at 2^15 entries a level and 1028 at 2^19 (GB300, with Adam); now 300
+// (encode 38, train 116, scatter 147: the atomics' rate in L2) and 430.  1000
+// rows: 80 -> 35.
+constexpr int kMlpInputs = 20;
+constexpr int kSmemRows = 1 << 15;         // batches at least this large use k_mlp_encode_smem
+constexpr uint32_t kSmemEntries = 48 << 10;  // for levels of at most this many entries
+__device__ __forceinline__ size_t batch_index(const MlpBatch& b, int j) {
+  uint32_t i = (uint32_t)b.first + (uint32_t)j;
+  if (i >= (uint32_t)b.total) i %= (uint32_t)b.total;
+  return i;
+}
+__device__ __forceinline__ V3 batch_pos(const MlpBatch& b, int j) {
+  const size_t i = batch_index(b, j), n = (size_t)b.total;
+  return v3(__ldg(b.pos + i), __ldg(b.pos + n + i), __ldg(b.pos + 2 * n + i));
+}
 
-// Weight gradient of one layer: dW[out][in] += dH^T (16 rows) * X.
-__device__ __forceinline__ void accum_dw(const uint32_t (&dh)[4][4], const uint32_t (&x)[4][4], int m_tiles,
-                                         float* dw) {
-  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  uint32_t bx[8][2];
-#pragma unroll
-  for (int nt = 0; nt < 8; ++nt) {
-    const int kk = nt >> 1;
-    bx[nt][0] = trans8x8(x[kk][(nt & 1) ? 2 : 0]);
-    bx[nt][1] = trans8x8(x[kk][(nt & 1) ? 3 : 1]);
+// The rows' positions, one array per coordinate (once per set of samples).
+__global__ void __launch_bounds__(256) k_mlp_positions(const float* __restrict__ samples, int n,
+                                                       float* __restrict__ pos) {
+  const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
+  if (i >= (size_t)n) return;
+  for (int d = 0; d < 3; ++d) pos[(size_t)d * n + i] = samples[i * 12 + d];
+}
+
+// The words of a row that are not hash features: blockIdx.y 16..19.
+__device__ __forceinline__ uint32_t plain_input(const float* q, int w) {
+  const V3 n = normalize(v3(q[3], q[4], q[5]));  // (n.x, n.y, n.z, alb.x, alb.y, alb.z, 1, 0)
+  return w == 0 ? pack_bf16(n.x, n.y) : w == 1 ? pack_bf16(n.z, q[6]) : w == 2 ? pack_bf16(q[7], q[8])
+                                                                                : pack_bf16(1.0f, 0.0f);
+}
+
+// Word blockIdx.y + first of every row: a level's features, gathered from
+// the table in L2, or (16 and up) the other inputs.
+__global__ void __launch_bounds__(256) k_mlp_encode(const __grid_constant__ MlpParams p, MlpBatch b, int first, uint32_t* __restrict__ inputs) {
+  const int row = blockIdx.x * 256 + threadIdx.x, l = first + (int)blockIdx.y;
+  if (row >= b.n) return;
+  uint32_t v;
+  if (l < kMlpLevels) {
+    const float2 f = level_features(p, l, batch_pos(b, row));
+    v = pack_bf16(f.x, f.y);
+  } else {
+    v = plain_input(b.samples + batch_index(b, row) * 12, l - kMlpLevels);
   }
-  for (int mt = 0; mt < m_tiles; ++mt) {
-    const uint32_t a[4] = {trans8x8(dh[mt][0]), trans8x8(dh[mt][2]), trans8x8(dh[mt][1]), trans8x8(dh[mt][3])};
+  inputs[(size_t)l * b.n + row] = v;
+}
+
+// The same for levels blockIdx.y whose entries fit in shared memory: the CTA
+// copies the level there once and its rows gather from it.
+__global__ void __launch_bounds__(1024) k_mlp_encode_smem(const __grid_constant__ MlpParams p, MlpBatch b, uint32_t* __restrict__ inputs) {
+  extern __shared__ __align__(16) uint32_t s_tab[];
+  const int l = (int)blockIdx.y;
+  const uint32_t entries = level_entries(p, l);
+  const uint32_t* tab = reinterpret_cast<const uint32_t*>(p.table_bf) + ((size_t)l << p.log2_table);
+  for (uint32_t i = threadIdx.x; i < (entries + 3) / 4; i += 1024)  // (a level's allocation is a multiple of 4)
+    reinterpret_cast<uint4*>(s_tab)[i] = __ldg(reinterpret_cast<const uint4*>(tab) + i);
+  __syncthreads();
+  for (int row = blockIdx.x * 1024 + threadIdx.x; row < b.n; row += gridDim.x * 1024) {
+    Corners c;
+    level_corners(p, l, batch_pos(b, row), c);
+    const float2 f = corner_features(c, s_tab);
+    inputs[(size_t)l * b.n + row] = pack_bf16(f.x, f.y);
+  }
+}
+
+// The loss's gradient in a level's features, added to its corners.  All
+// levels are in flight together (level by level, the rows meet in the coarse
+// levels' few entries: 189 against 148 us a step of 2^18 rows).  Two corners along x that share an aligned 16-byte word of the
+// table's gradient (half of them) take one atomic.
+__global__ void __launch_bounds__(256) k_mlp_scatter(const __grid_constant__ MlpParams p, MlpBatch b, const float2* __restrict__ d_features) {
+  const int l = (int)(blockIdx.x % kMlpLevels), row = (int)(blockIdx.x / kMlpLevels) * 256 + (int)threadIdx.x;
+  if (row >= b.n) return;
+  const float2 d = d_features[(size_t)l * b.n + row];
+  if (d.x == 0.f && d.y == 0.f) return;
+  Corners c;
+  level_corners(p, l, batch_pos(b, row), c);
+  float2* gl = p.table_grad + ((size_t)l << p.log2_table);
 #pragma unroll
-    for (int nt = 0; nt < 8; ++nt) {
-      float acc[4] = {0.f, 0.f, 0.f, 0.f};
-      mma16816(acc, a, bx[nt][0], bx[nt][1]);
-      float* r0 = dw + (16 * mt + g) * kDWS + 8 * nt + 2 * t;
-      float* r1 = r0 + 8 * kDWS;
-      atomicAdd(r0, acc[0]);
-      atomicAdd(r0 + 1, acc[1]);
-      atomicAdd(r1, acc[2]);
-      atomicAdd(r1 + 1, acc[3]);
+  for (int k = 0; k < 8; k += 2) {
+    const float2 a0 = make_float2(c.w[k] * d.x, c.w[k] * d.y), a1 = make_float2(c.w[k + 1] * d.x, c.w[k + 1] * d.y);
+    if (!(c.idx[k] & 1u) && c.idx[k + 1] == c.idx[k] + 1u) {
+      atomicAdd(reinterpret_cast<float4*>(gl + c.idx[k]), make_float4(a0.x, a0.y, a1.x, a1.y));
+    } else {
+      atomicAdd(gl + c.idx[k], a0);
+      atomicAdd(gl + c.idx[k + 1], a1);
     }
   }
 }
 
-// Backward through one 64x64 layer: dX = dH * W (W^T stored [in][out] as wt),
-// masked by (X > 0) when X is a ReLU output.
-__device__ __forceinline__ void back64(const uint32_t (&dh)[4][4], const uint32_t* wt, const uint32_t (&xmask)[4][4],
-                                       bool mask, float (&acc)[8][4]) {
-  layer64(dh, wt, acc);
-  if (!mask) return;
+constexpr int kTrainWarps = 16;
+constexpr int kTrainRows = 16 * kTrainWarps;  // rows of a tile: 16 a warp
+struct TrainSmem {
+  uint32_t w[4][64 * kWSw];            // W1..W4 [out][in]
+  uint32_t w5[16 * kWSw];              // W5 [out 16][in 64]
+  uint32_t x[4][kTrainRows * kWSw];    // h1..h4 of the tile, [row][column]
+  uint32_t g[kTrainRows * kWSw];       // the gradient in one layer's outputs
+};
+
+__device__ __forceinline__ void ldm4(uint32_t (&r)[4], const uint32_t* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(smem_u32(p))
+               : "memory");
+}
+__device__ __forceinline__ void ldm4t(uint32_t (&r)[4], const uint32_t* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(smem_u32(p))
+               : "memory");
+}
+
+// acc (16 x 64) = A (16 x 64) * W^T, W [out][in] in shared memory.
+__device__ __forceinline__ void forward64(const uint32_t (&a)[4][4], const uint32_t* W, float (&acc)[8][4]) {
+  const int lane = threadIdx.x & 31;
+  // matrices of one load: (n-tile, k 0-7), (n-tile, k 8-15), (next n-tile, ...)
+  const uint32_t* at = W + ((lane & 7) + (lane >> 4) * 8) * kWSw + ((lane >> 3) & 1) * 4;
+#pragma unroll
+  for (int nt = 0; nt < 8; ++nt) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
+#pragma unroll
+  for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+    for (int nt = 0; nt < 8; nt += 2) {
+      uint32_t r[4];
+      ldm4(r, at + 8 * nt * kWSw + 8 * kk);
+      mma16816(acc[nt], a[kk], r[0], r[1]);
+      mma16816(acc[nt + 1], a[kk], r[2], r[3]);
+    }
+}
+
+// acc (16 x 8 NT) = A (16 x 16 KT) * W, W [out][in] in shared memory.
+template <int KT, int NT>
+__device__ __forceinline__ void backward64(const uint32_t (&a)[4][4], const uint32_t* W, float (&acc)[8][4]) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t* at = W + ((lane & 7) + ((lane >> 3) & 1) * 8) * kWSw + (lane >> 4) * 4;
+#pragma unroll
+  for (int nt = 0; nt < NT; ++nt) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
+#pragma unroll
+  for (int kk = 0; kk < KT; ++kk)
+#pragma unroll
+    for (int nt = 0; nt < NT; nt += 2) {
+      uint32_t r[4];
+      ldm4t(r, at + 16 * kk * kWSw + 4 * nt);
+      mma16816(acc[nt], a[kk], r[0], r[1]);
+      mma16816(acc[nt + 1], a[kk], r[2], r[3]);
+    }
+}
+
+// A fragments <-> a warp's 16 rows of a tile in shared memory.
+__device__ __forceinline__ void put_a(uint32_t* rows, const uint32_t (&a)[4][4]) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+#pragma unroll
+  for (int kk = 0; kk < 4; ++kk) {
+    rows[g * kWSw + 8 * kk + t] = a[kk][0];
+    rows[(g + 8) * kWSw + 8 * kk + t] = a[kk][1];
+    rows[g * kWSw + 8 * kk + 4 + t] = a[kk][2];
+    rows[(g + 8) * kWSw + 8 * kk + 4 + t] = a[kk][3];
+  }
+}
+// Zeroes the accumulators where the ReLU outputs `rows` (a warp's 16) are 0.
+__device__ __forceinline__ void relu_mask(const uint32_t* rows, float (&acc)[8][4]) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
 #pragma unroll
   for (int nt = 0; nt < 8; ++nt) {
-    const int kk = nt >> 1;
-    const uint32_t m0 = xmask[kk][(nt & 1) ? 2 : 0], m1 = xmask[kk][(nt & 1) ? 3 : 1];
+    const uint32_t m0 = rows[g * kWSw + 4 * nt + t], m1 = rows[(g + 8) * kWSw + 4 * nt + t];
     if (!(bf_lo(m0) > 0.f)) acc[nt][0] = 0.f;
     if (!(bf_hi(m0) > 0.f)) acc[nt][1] = 0.f;
     if (!(bf_lo(m1) > 0.f)) acc[nt][2] = 0.f;
@@ -321,132 +443,172 @@ __device__ __forceinline__ void back64(const uint32_t (&dh)[4][4], const uint32_
   }
 }
 
-__global__ void __launch_bounds__(256, 1) k_mlp_train(MlpParams p, MlpBatch b, float* __restrict__ loss_out) {
+// dW[16 mt .. +15][16 nq .. +15] += G^T X over the tile's rows, G and X
+// [row][column] in shared memory.  The tensor core sums 64 rows at a time
+// (its own additions truncate); the running sum is kept by rounded additions.
+__device__ __forceinline__ void add_dw(const uint32_t* G, const uint32_t* X, int mt, int nq, float (&dw)[2][4]) {
+  const int lane = threadIdx.x & 31;
+  // A (out x row): (m 0-7, k 0-7), (m 8-15, k 0-7), (m 0-7, k 8-15), (m 8-15, k 8-15)
+  const uint32_t* ga = G + ((lane & 7) + (lane >> 4) * 8) * kWSw + 8 * mt + ((lane >> 3) & 1) * 4;
+  // B (row x in): (k 0-7, n-tile), (k 8-15, n-tile), then the next n-tile
+  const uint32_t* xa = X + ((lane & 7) + ((lane >> 3) & 1) * 8) * kWSw + 8 * nq + (lane >> 4) * 4;
+#pragma unroll 1
+  for (int k0 = 0; k0 < kTrainRows / 16; k0 += 4) {
+    float acc[2][4] = {};
+#pragma unroll
+    for (int kk = k0; kk < k0 + 4; ++kk) {
+      uint32_t a[4], x[4];
+      ldm4t(a, ga + 16 * kk * kWSw);
+      ldm4t(x, xa + 16 * kk * kWSw);
+      mma16816(acc[0], a, x[0], x[1]);
+      mma16816(acc[1], a, x[2], x[3]);
+    }
+#pragma unroll
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) dw[n][e] += acc[n][e];
+  }
+}
+
+__global__ void __launch_bounds__(kTrainWarps * 32, 1)
+    k_mlp_train(MlpParams p, MlpBatch b, const uint32_t* __restrict__ inputs, float2* __restrict__ d_features,
+                float* __restrict__ loss_out) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   TrainSmem& S = *reinterpret_cast<TrainSmem*>(smem_raw);
-  load_weights(p.w_bf, S.w, &S.wt);
-  for (int i = threadIdx.x; i < 4 * 64 * kDWS; i += blockDim.x) (&S.dw[0][0])[i] = 0.f;
-  for (int i = threadIdx.x; i < 16 * kDWS; i += blockDim.x) S.dw5[i] = 0.f;
+  {
+    const uint32_t* wg = reinterpret_cast<const uint32_t*>(p.w_bf);
+    for (int i = threadIdx.x; i < 4 * 64 * 32; i += kTrainWarps * 32)
+      S.w[i >> 11][((i >> 5) & 63) * kWSw + (i & 31)] = wg[i];
+    for (int i = threadIdx.x; i < 16 * 32; i += kTrainWarps * 32) S.w5[(i >> 5) * kWSw + (i & 31)] = wg[4 * 2048 + i];
+  }
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const int nwarps = blockDim.x >> 5;
-  unsigned short* E = S.E[warp];
+  const int mt = warp & 3, nq = warp >> 2;  // the warp's block of each 64 x 64 weight gradient
+  const int own = 16 * warp * kWSw;         // the warp's rows of a tile
+  float dw[4][2][4] = {}, dw5[2][4] = {};   // dw5: warps 0-3, 16 columns each
   float loss = 0.f;
   const float inv_n = 1.0f / (float)b.n;
-  for (int tile = blockIdx.x * nwarps + warp; tile * 16 < b.n; tile += gridDim.x * nwarps) {
-    const int row0 = tile * 16;
-    build_inputs(p, E, [&](int row, V3& pos, V3& nrm, V3& alb, bool& valid) {
-      const int s = row0 + row;
-      valid = s < b.n;
-      const int j = valid ? s : 0;
-      const float* q = b.samples + (size_t)(b.first + j) % b.total * 12;
-      pos = v3(q[0], q[1], q[2]);
-      nrm = v3(q[3], q[4], q[5]);
-      alb = v3(q[6], q[7], q[8]);
-      if ((lane >> 4) == 0) {
-        S.pos[warp][row][0] = pos.x; S.pos[warp][row][1] = pos.y; S.pos[warp][row][2] = pos.z;
+  for (int tile = blockIdx.x; tile * kTrainRows < b.n; tile += gridDim.x) {
+    const int row0 = tile * kTrainRows + 16 * warp;
+    const bool v0 = row0 + g < b.n, v1 = row0 + g + 8 < b.n;
+    auto load_x0 = [&](uint32_t(&a)[4][4]) {  // words 20..31 of a row are zeros
+      const uint32_t* q = inputs + (size_t)t * b.n + row0 + g;
+      const size_t w4 = 4 * (size_t)b.n;
+#pragma unroll
+      for (int i = 0; i < 5; ++i) {
+        a[i >> 1][(i & 1) * 2] = v0 ? __ldg(q + i * w4) : 0u;
+        a[i >> 1][(i & 1) * 2 + 1] = v1 ? __ldg(q + i * w4 + 8) : 0u;
       }
-    });
-    uint32_t x0[4][4], h1[4][4], h2[4][4], h3[4][4], h4[4][4];
+      a[2][2] = a[2][3] = a[3][0] = a[3][1] = a[3][2] = a[3][3] = 0u;
+    };
+    uint32_t a[4][4];
     float acc[8][4];
-    load_a(E, x0);
-    layer64(x0, S.w.w[0], acc); d_to_a(acc, h1, true);
-    layer64(h1, S.w.w[1], acc); d_to_a(acc, h2, true);
-    layer64(h2, S.w.w[2], acc); d_to_a(acc, h3, true);
-    layer64(h3, S.w.w[3], acc); d_to_a(acc, h4, true);
+    load_x0(a);
+#pragma unroll
+    for (int l = 0; l < 4; ++l) {
+      forward64(a, S.w[l], acc);
+      d_to_a(acc, a, true);
+      put_a(S.x[l] + own, a);
+    }
     float y[2][4];
-    layer_out(h4, S.w.w5, y);
+    layer_out(a, S.w5, y);
     // MSE gradient on the 3 valid outputs (cols 0..2 live in n-tile 0, t <= 1).
     float dy[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-      const int r = row0 + g + (e >= 2 ? 8 : 0);
-      const int c = 2 * t + (e & 1);
+      const int r = row0 + g + (e >= 2 ? 8 : 0), c = 2 * t + (e & 1);
       if (c < 3 && r < b.n) {
-        const float tg = b.samples[(size_t)(b.first + r) % b.total * 12 + 9 + c];
-        const float d = y[0][e] - tg;
+        const float d = y[0][e] - b.samples[batch_index(b, r) * 12 + 9 + c];
         loss += d * d * inv_n;
         dy[e] = 2.0f * d * inv_n;
       }
     }
-    uint32_t dya[4][4];
-    dya[0][0] = pack_bf16(dy[0], dy[1]);
-    dya[0][1] = pack_bf16(dy[2], dy[3]);
-    dya[0][2] = 0u;
-    dya[0][3] = 0u;
-    // dH4 = dY * W5 (masked by h4 > 0): one k-tile, B = W5^T [in][out].
-#pragma unroll
-    for (int nt = 0; nt < 8; ++nt) {
-      acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
-      const uint32_t* r = S.wt.w5t + (8 * nt + g) * (kW5TS / 2);
-      mma16816(acc[nt], dya[0], r[t], r[4 + t]);
-      const int kk = nt >> 1;
-      const uint32_t m0 = h4[kk][(nt & 1) ? 2 : 0], m1 = h4[kk][(nt & 1) ? 3 : 1];
-      if (!(bf_lo(m0) > 0.f)) acc[nt][0] = 0.f;
-      if (!(bf_hi(m0) > 0.f)) acc[nt][1] = 0.f;
-      if (!(bf_lo(m1) > 0.f)) acc[nt][2] = 0.f;
-      if (!(bf_hi(m1) > 0.f)) acc[nt][3] = 0.f;
+    a[0][0] = pack_bf16(dy[0], dy[1]);
+    a[0][1] = pack_bf16(dy[2], dy[3]);
+    a[0][2] = a[0][3] = 0u;
+    {
+      uint32_t* rows = S.g + own;
+      rows[g * kWSw + t] = a[0][0];
+      rows[(g + 8) * kWSw + t] = a[0][1];
+      rows[g * kWSw + 4 + t] = 0u;
+      rows[(g + 8) * kWSw + 4 + t] = 0u;
     }
-    accum_dw(dya, h4, 1, S.dw5);
-    uint32_t dh[4][4];
-    d_to_a(acc, dh, false);                  // dH4
-    accum_dw(dh, h3, 4, S.dw[3]);
-    back64(dh, S.wt.wt[3], h3, true, acc);    // dH3
-    d_to_a(acc, dh, false);
-    accum_dw(dh, h2, 4, S.dw[2]);
-    back64(dh, S.wt.wt[2], h2, true, acc);    // dH2
-    d_to_a(acc, dh, false);
-    accum_dw(dh, h1, 4, S.dw[1]);
-    back64(dh, S.wt.wt[1], h1, true, acc);    // dH1
-    d_to_a(acc, dh, false);
-    accum_dw(dh, x0, 4, S.dw[0]);
-    back64(dh, S.wt.wt[0], x0, false, acc);   // dE (cols 0..31 = hash features)
-    // Scatter: lane holds levels 4*nt + t (nt < 4) for rows g and g + 8.
-#pragma unroll 1
+    __syncthreads();  // the tile's h1..h4 and dY are there
+    if (warp < 4) add_dw(S.g, S.x[3], 0, warp, dw5);
+    backward64<1, 8>(a, S.w5, acc);  // dH4 = dY W5
+    relu_mask(S.x[3] + own, acc);
+    d_to_a(acc, a, false);
+    __syncthreads();  // dY has been read
+#pragma unroll
+    for (int l = 3; l > 0; --l) {
+      put_a(S.g + own, a);
+      __syncthreads();
+      add_dw(S.g, S.x[l - 1], mt, nq, dw[l]);
+      backward64<4, 8>(a, S.w[l], acc);
+      relu_mask(S.x[l - 1] + own, acc);
+      d_to_a(acc, a, false);
+      __syncthreads();
+    }
+    put_a(S.g + own, a);  // dH1
+    {
+      uint32_t x0[4][4];
+      load_x0(x0);
+      put_a(S.x[3] + own, x0);  // (h4 is done with)
+    }
+    __syncthreads();
+    add_dw(S.g, S.x[3], mt, nq, dw[0]);
+    backward64<4, 4>(a, S.w[0], acc);  // the hash features: columns 0..31
+    float2* d0 = d_features + (size_t)t * b.n + row0 + g;
+#pragma unroll
     for (int nt = 0; nt < 4; ++nt) {
-      const int l = 4 * nt + t;
-#pragma unroll 1
-      for (int h = 0; h < 2; ++h) {
-        const int row = g + 8 * h;
-        if (row0 + row >= b.n) continue;
-        const float d0 = acc[nt][2 * h], d1 = acc[nt][2 * h + 1];
-        if (d0 == 0.f && d1 == 0.f) continue;
-        Corners c;
-        level_corners(p, l, v3(S.pos[warp][row][0], S.pos[warp][row][1], S.pos[warp][row][2]), c);
-        float2* gl = p.table_grad + ((size_t)l << p.log2_table);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) atomicAdd(gl + c.idx[k], make_float2(c.w[k] * d0, c.w[k] * d1));
-      }
+      if (v0) d0[4 * nt * (size_t)b.n] = make_float2(acc[nt][0], acc[nt][1]);
+      if (v1) d0[4 * nt * (size_t)b.n + 8] = make_float2(acc[nt][2], acc[nt][3]);
     }
-    __syncwarp();
+    __syncthreads();  // the next tile writes over these
   }
-  __syncthreads();
-  for (int i = threadIdx.x; i < 4 * 4096; i += blockDim.x) {
-    const int l = i >> 12, o = (i >> 6) & 63, k = i & 63;
-    const float v = S.dw[l][o * kDWS + k];
-    if (v != 0.f) atomicAdd(p.w_grad + i, v);
-  }
-  for (int i = threadIdx.x; i < 16 * 64; i += blockDim.x) {
-    const float v = S.dw5[(i >> 6) * kDWS + (i & 63)];
-    if (v != 0.f) atomicAdd(p.w_grad + 4 * 4096 + i, v);
-  }
+  auto flush = [&](float* out, const float(&v)[2][4], int m, int n) {
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (v[j][e] != 0.f)
+          atomicAdd(out + (16 * m + g + (e >= 2 ? 8 : 0)) * 64 + 16 * n + 8 * j + 2 * t + (e & 1), v[j][e]);
+  };
+#pragma unroll
+  for (int l = 0; l < 4; ++l) flush(p.w_grad + l * 4096, dw[l], mt, nq);
+  if (warp < 4) flush(p.w_grad + 4 * 4096, dw5, 0, warp);
   for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
   if (lane == 0 && loss_out) atomicAdd(loss_out, loss);
 }
 
-// Adam on a flat parameter array; refreshes the bf16 copy and clears grads.
-__global__ void k_adam(float* __restrict__ prm, float* __restrict__ grad, float* __restrict__ m, float* __restrict__ v,
-                       __nv_bfloat16* __restrict__ prm_bf, size_t n, AdamStep a) {
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    const float gi = grad[i] + a.l2 * prm[i];
-    const float mi = a.beta1 * m[i] + (1.0f - a.beta1) * gi;
-    const float vi = a.beta2 * v[i] + (1.0f - a.beta2) * gi * gi;
-    m[i] = mi;
-    v[i] = vi;
-    const float pi = prm[i] - a.lr * (mi * a.c1) / (sqrtf(vi * a.c2) + a.eps);
-    prm[i] = pi;
-    grad[i] = 0.f;
-    prm_bf[i] = __float2bfloat16_rn(pi);
+// Adam on two flat parameter arrays (the table, then the weights; lengths a
+// multiple of 4), four values a thread; refreshes the bf16 copies and clears
+// the gradients.  Bound by memory: 34 bytes a parameter.
+__device__ __forceinline__ float adam_one(const AdamStep& a, float l2, float prm, float grad, float& m, float& v) {
+  const float gi = grad + l2 * prm;
+  m = a.beta1 * m + (1.0f - a.beta1) * gi;
+  v = a.beta2 * v + (1.0f - a.beta2) * gi * gi;
+  return prm - a.lr * (m * a.c1) / (sqrtf(v * a.c2) + a.eps);
+}
+__global__ void __launch_bounds__(256) k_adam(AdamArray table, AdamArray w, AdamStep a) {
+  const size_t nt = table.n / 4, n = nt + w.n / 4;
+  for (size_t q = (size_t)blockIdx.x * 256 + threadIdx.x; q < n; q += (size_t)gridDim.x * 256) {
+    const bool in_table = q < nt;
+    const AdamArray& arr = in_table ? table : w;
+    const size_t i = in_table ? q : q - nt;
+    const float l2 = in_table ? 0.0f : a.l2;
+    const float4 g = reinterpret_cast<const float4*>(arr.grad)[i];
+    float4 p = reinterpret_cast<const float4*>(arr.prm)[i], m = reinterpret_cast<const float4*>(arr.m)[i],
+           v = reinterpret_cast<const float4*>(arr.v)[i];
+    p.x = adam_one(a, l2, p.x, g.x, m.x, v.x);
+    p.y = adam_one(a, l2, p.y, g.y, m.y, v.y);
+    p.z = adam_one(a, l2, p.z, g.z, m.z, v.z);
+    p.w = adam_one(a, l2, p.w, g.w, m.w, v.w);
+    reinterpret_cast<float4*>(arr.m)[i] = m;
+    reinterpret_cast<float4*>(arr.v)[i] = v;
+    reinterpret_cast<float4*>(arr.prm)[i] = p;
+    reinterpret_cast<float4*>(arr.grad)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    reinterpret_cast<uint2*>(arr.prm_bf)[i] = make_uint2(pack_bf16(p.x, p.y), pack_bf16(p.z, p.w));
   }
 }
 
@@ -471,12 +633,12 @@ struct InferSmem {
   unsigned short E[8][16 * kWS];
 };
 
-__global__ void __launch_bounds__(256, 4) k_mlp_infer(MlpParams p, SceneParams sp, const float4* __restrict__ gb_pos,
+__global__ void __launch_bounds__(256, 4) k_mlp_infer(const __grid_constant__ MlpParams p, SceneParams sp, const float4* __restrict__ gb_pos,
                                                    const float4* __restrict__ gb_nrm, int n_px,
                                                    float4* __restrict__ out) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   SmemW& W = *reinterpret_cast<SmemW*>(smem_raw);
-  load_weights(p.w_bf, W, nullptr);
+  load_weights(p.w_bf, W);
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int nwarps = blockDim.x >> 5;
@@ -520,11 +682,11 @@ __global__ void __launch_bounds__(256, 4) k_mlp_infer(MlpParams p, SceneParams s
 
 // Forward of explicit samples (tests, evaluation): rows of 12 floats
 // (pos, normal, albedo, ignored target).
-__global__ void __launch_bounds__(256) k_mlp_eval(MlpParams p, const float* __restrict__ samples, int n,
+__global__ void __launch_bounds__(256) k_mlp_eval(const __grid_constant__ MlpParams p, const float* __restrict__ samples, int n,
                                                   float* __restrict__ out) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   InferSmem& S = *reinterpret_cast<InferSmem*>(smem_raw);
-  load_weights(p.w_bf, S.w, nullptr);
+  load_weights(p.w_bf, S.w);
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int nwarps = blockDim.x >> 5;
@@ -655,7 +817,7 @@ __device__ __forceinline__ void tc_input(const SceneParams& sp, const float4* __
 
 template <bool FROM_GBUF>
 __global__ void __launch_bounds__(kWsThreads, 1)
-    k_mlp_fwd_tc(MlpParams p, SceneParams sp, const float4* __restrict__ gb_pos, const float4* __restrict__ gb_nrm,
+    k_mlp_fwd_tc(const __grid_constant__ MlpParams p, SceneParams sp, const float4* __restrict__ gb_pos, const float4* __restrict__ gb_nrm,
                  const float* __restrict__ samples, int n, float4* __restrict__ out4, float* __restrict__ out3,
                  FrameStatus* status) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -840,29 +1002,53 @@ int sm_count() {
 
 }  // namespace
 
-size_t mlp_train_smem() { return sizeof(TrainSmem); }
-size_t mlp_infer_smem() { return sizeof(InferSmem); }
 
 cudaError_t launch_mlp_init(float* prm, __nv_bfloat16* prm_bf, size_t n, float scale, uint64_t seed, cudaStream_t st) {
   k_mlp_init<<<sm_count() * 4, 256, 0, st>>>(prm, prm_bf, n, scale, seed);
   return cudaGetLastError();
 }
 
-cudaError_t launch_mlp_train(const MlpParams& p, const MlpBatch& b, float* loss, cudaStream_t st) {
-  const size_t smem = sizeof(TrainSmem);
-  cudaError_t e = cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  const int tiles = (b.n + 15) / 16;
-  int grid = sm_count();
-  if (grid * 8 > tiles) grid = (tiles + 7) / 8;
-  if (grid < 1) grid = 1;
-  k_mlp_train<<<grid, 256, smem, st>>>(p, b, loss);
+size_t mlp_train_words(int n) { return ((size_t)n * kMlpInputs + 1) / 2 * 2 + (size_t)n * 2 * kMlpLevels; }
+
+cudaError_t launch_mlp_positions(const float* samples, int n, float* pos, cudaStream_t st) {
+  if (n <= 0) return cudaSuccess;
+  k_mlp_positions<<<(unsigned)(((size_t)n + 255) / 256), 256, 0, st>>>(samples, n, pos);
   return cudaGetLastError();
 }
 
-cudaError_t launch_adam(float* prm, float* grad, float* m, float* v, __nv_bfloat16* prm_bf, size_t n,
-                        const AdamStep& a, cudaStream_t st) {
-  k_adam<<<sm_count() * 8, 256, 0, st>>>(prm, grad, m, v, prm_bf, n, a);
+cudaError_t launch_mlp_train(const MlpParams& p, const MlpBatch& b, uint32_t* work, float* loss, cudaStream_t st) {
+  if (b.n <= 0) return cudaSuccess;
+  const size_t smem = sizeof(TrainSmem);
+  cudaError_t e = cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  uint32_t* inputs = work;
+  float2* d_features = reinterpret_cast<float2*>(work + ((size_t)b.n * kMlpInputs + 1) / 2 * 2);
+  // The levels (the first ones: their sizes do not decrease) whose entries fit
+  // in shared memory, when there are rows enough to pay for copying them: at
+  // 2^15 entries a level 2^18 rows encode in 38 us instead of 81; a small
+  // batch gathers less than the copies.
+  int in_smem = 0;
+  size_t tab = 0;
+  while (b.n >= kSmemRows && in_smem < kMlpLevels && level_entries(p, in_smem) <= kSmemEntries)
+    tab = std::max(tab, (size_t)((level_entries(p, in_smem++) + 3) / 4 * 16));
+  if (in_smem) {
+    e = cudaFuncSetAttribute(k_mlp_encode_smem, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tab);
+    if (e != cudaSuccess) return e;
+    const int per_sm = std::max(1, std::min(2, (int)(220 * 1024 / (tab + 1024))));
+    const dim3 grid((unsigned)std::max(1, sm_count() * per_sm / in_smem), (unsigned)in_smem);
+    k_mlp_encode_smem<<<grid, 1024, tab, st>>>(p, b, inputs);
+  }
+  const unsigned blocks = (unsigned)((b.n + 255) / 256);
+  k_mlp_encode<<<dim3(blocks, (unsigned)(kMlpInputs - in_smem)), 256, 0, st>>>(p, b, in_smem, inputs);
+  const int tiles = (b.n + kTrainRows - 1) / kTrainRows;
+  k_mlp_train<<<std::min(tiles, sm_count()), kTrainWarps * 32, smem, st>>>(p, b, inputs, d_features, loss);
+  k_mlp_scatter<<<blocks * kMlpLevels, 256, 0, st>>>(p, b, d_features);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_adam(const AdamArray& table, const AdamArray& w, const AdamStep& a, cudaStream_t st) {
+  const size_t blocks = (table.n / 4 + w.n / 4 + 255) / 256;
+  k_adam<<<(unsigned)std::min<size_t>(blocks, (size_t)sm_count() * 8), 256, 0, st>>>(table, w, a);
   return cudaGetLastError();
 }
 

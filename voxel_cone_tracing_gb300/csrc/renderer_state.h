@@ -138,6 +138,8 @@ struct MlpState {
   DevBuf<float> samples;  // rows of 12 floats
   uint32_t n_samples = 0;
   DevBuf<float> loss;     // one slot per optimiser step
+  DevBuf<float> pos;      // the samples' positions, one array per coordinate
+  DevBuf<uint32_t> work;  // a step's inputs and feature gradients (launch_mlp_train)
 
   size_t table_floats() const { return (size_t)levels * ((size_t)1 << log2_table) * 2; }
 

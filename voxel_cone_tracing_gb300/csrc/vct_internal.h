@@ -372,11 +372,18 @@ struct MlpParams {
 // albedo, target RGB), `n` rows starting at row `first` (mod `total`).
 struct MlpBatch {
   const float* samples;
+  const float* pos;  // their positions, `total` x, then y, then z (launch_mlp_positions)
   int first, n, total;
 };
 
 struct AdamStep {
-  float lr, beta1, beta2, eps, c1, c2, l2;  // c1 = 1/(1-beta1^t), c2 = 1/(1-beta2^t)
+  float lr, beta1, beta2, eps, c1, c2;  // c1 = 1/(1-beta1^t), c2 = 1/(1-beta2^t)
+  float l2;                             // of the weights (the table has none)
+};
+struct AdamArray {  // n a multiple of 4, every array 16-byte aligned
+  float *prm, *grad, *m, *v;
+  __nv_bfloat16* prm_bf;
+  size_t n;
 };
 
 // ---- launchers (stream-ordered, no host synchronisation) ----------------
@@ -482,9 +489,12 @@ cudaError_t launch_trace_batch(const BatchWork& tiles, const BatchBuffers& bb, c
 
 // Learned diffuse term.
 cudaError_t launch_mlp_init(float* prm, __nv_bfloat16* prm_bf, size_t n, float scale, uint64_t seed, cudaStream_t st);
-cudaError_t launch_mlp_train(const MlpParams& p, const MlpBatch& b, float* loss, cudaStream_t st);
-cudaError_t launch_adam(float* prm, float* grad, float* m, float* v, __nv_bfloat16* prm_bf, size_t n,
-                        const AdamStep& a, cudaStream_t st);
+// The positions of n rows, one array per coordinate (3 n floats).
+cudaError_t launch_mlp_positions(const float* samples, int n, float* pos, cudaStream_t st);
+// `work`: mlp_train_words(b.n) words.
+size_t mlp_train_words(int n);
+cudaError_t launch_mlp_train(const MlpParams& p, const MlpBatch& b, uint32_t* work, float* loss, cudaStream_t st);
+cudaError_t launch_adam(const AdamArray& table, const AdamArray& w, const AdamStep& a, cudaStream_t st);
 // Inference / evaluation of the network: on the 5th-generation tensor cores
 // (tcgen05.mma, TMEM accumulators) when `tc`, else in mma.sync warp tiles.
 cudaError_t launch_mlp_infer(const MlpParams& p, const SceneParams& sp, const float4* gb_pos, const float4* gb_nrm,
