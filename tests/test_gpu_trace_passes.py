@@ -37,7 +37,8 @@ def _frame(vct, s, w, h, **cfg):
     (1, 1, 32, 1, dict()), (3, 2, 8, 1, dict()), (15, 17, 64, 0, dict()), (33, 31, 128, 4, dict()),
     (50, 37, 256, 2, dict(far_share=0)), (41, 20, 64, 3, dict(cone_set=1)), (41, 20, 64, 3, dict(mip_mode=1)),
     (47, 33, 64, 2, dict(storage=1, radiance_max=4.0)), (47, 33, 32, 2, dict(storage=1, mip_mode=2, cone_set=1)),
-    (29, 18, 512, 1, dict())],
+    (29, 18, 512, 1, dict()), (23, 9, 32, 4, dict(sampler=1)), (9, 5, 64, 0, dict(sampler=1, mip_mode=1, cone_set=1)),
+    (13, 6, 32, 1, dict(sampler=1, storage=1))],
     ids=lambda v: "-".join(f"{k}{x}" for k, x in v.items()) or "default" if isinstance(v, dict) else str(v))
 def test_passes_match_the_full_march(vct, w, h, grid, lights, cfg):
     s = _scene(w, h, lights)

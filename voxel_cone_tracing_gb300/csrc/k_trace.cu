@@ -14,29 +14,6 @@
 namespace vct {
 namespace {
 
-#ifndef VCT_TRACE_ROWS
-#define VCT_TRACE_ROWS 8
-#endif
-#ifndef VCT_TRACE_MIN_BLOCKS
-#define VCT_TRACE_MIN_BLOCKS 12
-#endif
-// A k_trace CTA shades a 16 x kTraceRows pixel tile (each warp a
-// kTraceWarpW x (32 / kTraceWarpW) block); the texture-unit variant is compiled for kTraceMinBlocks resident
-// CTAs per SM (register budget 65536 / (16 * rows * blocks) per thread).
-// Measured on the 1080p bench frame (trace ms): 128 threads x 12 CTAs (40
-// registers, 48 warps per SM) 2.59; x 9 (56 registers) 2.64; 256 threads
-// x 4 (64 registers) 2.71, x 6 (40) 2.62; 32 registers 3.77 (spills);
-// 64-thread CTAs x 22 2.98. Warps of 8x4 pixels instead of 16x2 strips:
-// 2.536 vs 2.543 alternating on one GPU, within noise across GPUs (same frame).
-constexpr int kTraceRows = VCT_TRACE_ROWS;
-constexpr int kTraceThreads = 16 * kTraceRows;
-constexpr int kTraceMinBlocks = VCT_TRACE_MIN_BLOCKS;
-#ifndef VCT_TRACE_WARP_W
-#define VCT_TRACE_WARP_W 8
-#endif
-constexpr int kTraceWarpW = VCT_TRACE_WARP_W;
-static_assert((kTraceWarpW == 8 || kTraceWarpW == 16) && kTraceRows % (32 / kTraceWarpW) == 0,
-              "a k_trace tile holds whole warp blocks");
 #ifndef VCT_TRACE_BATCH_MIN_BLOCKS
 #define VCT_TRACE_BATCH_MIN_BLOCKS 3
 #endif
@@ -355,46 +332,62 @@ __device__ __forceinline__ void trace_px(const SceneParams& sp, const CameraPara
     // within_cube(pos, 0) (:61-64, 250): a fragment outside returns without
     // writing; the pixel keeps the clear colour.
     if (fabsf(pos.x) < 1.0f && fabsf(pos.y) < 1.0f && fabsf(pos.z) < 1.0f) {
-      if (tp.view_voxel_dir < 7) {  // voxel debug view, :253-257
-        // (map 6: the isotropic chain of VCT_MIP_BOTH; no such map otherwise)
-        if (tp.view_voxel_dir >= 0 && (tp.view_voxel_dir <= 5 || (tp.view_voxel_dir == 6 && m.nmaps == 7))) {
-          const float lod = fmaxf(tp.view_voxel_lod, 0.0f);
-          const V3 one = v3(1.f, 0.f, 0.f);
-          const int d = ISO ? 0 : tp.view_voxel_dir;
-          out = sample_voxel<SAMPLER, ISO, STORAGE>(m, pos, d, d, d, one, lod);
+      const V3 cam = v3(cp.cam_pos[0], cp.cam_pos[1], cp.cam_pos[2]);
+      const V3 view_dir = normalize(world - cam);
+      V3 fd = v3(0.f, 0.f, 0.f), fdir = v3(0.f, 0.f, 0.f), fs = v3(0.f, 0.f, 0.f);
+      if (tp.enable_diffuse) {
+        if (tp.diffuse_in) {
+          const float4 d = tp.diffuse_in[p];
+          fd = mulv(mat3v(mat.diffuse), v3(d.x, d.y, d.z));
+        } else if (SHARE && far) {
+          fd = mulv(mat3v(mat.diffuse), trace_diffuse_shared<ISO>(m, tp.cone_set, pos, nrm, far));
         } else {
-          out = f4(0.f, 0.f, 0.f, 0.f);
+          fd = mulv(mat3v(mat.diffuse), trace_diffuse<SAMPLER, ISO, STORAGE>(m, tp.cone_set, pos, nrm));
         }
-      } else {
-        const V3 cam = v3(cp.cam_pos[0], cp.cam_pos[1], cp.cam_pos[2]);
-        const V3 view_dir = normalize(world - cam);
-        V3 fd = v3(0.f, 0.f, 0.f), fdir = v3(0.f, 0.f, 0.f), fs = v3(0.f, 0.f, 0.f);
-        if (tp.enable_diffuse) {
-          if (tp.diffuse_in) {
-            const float4 d = tp.diffuse_in[p];
-            fd = mulv(mat3v(mat.diffuse), v3(d.x, d.y, d.z));
-          } else if (SHARE && far) {
-            fd = mulv(mat3v(mat.diffuse), trace_diffuse_shared<ISO>(m, tp.cone_set, pos, nrm, far));
-          } else {
-            fd = mulv(mat3v(mat.diffuse), trace_diffuse<SAMPLER, ISO, STORAGE>(m, tp.cone_set, pos, nrm));
-          }
-        }
-        if (tp.enable_direct)
-          fdir = direct_light<SAMPLER, ISO, STORAGE, false>(sp, m, tp.enable_shadow, mat, pos, nrm, view_dir, nullptr, 0);
-        const float sap = specular_aperture(mat.shininess);
-        if (tp.enable_specular) {
-          const V3 sd = normalize(reflect(-view_dir, nrm));
-          const float4 c = trace_cone<SAMPLER, ISO, STORAGE>(m, pos, sd, sap, kMaxDistance);
-          fs = mulv(mat3v(mat.specular), v3(c.x, c.y, c.z));
-        }
-        V3 f = fs + fd + fdir;
-        if (refracts(mat) && tp.enable_specular) {
-          const V3 rd = refract(view_dir, nrm, 1.0f / mat.ior);
-          const float4 c = trace_cone<SAMPLER, ISO, STORAGE>(m, pos, rd, sap, kMaxDistance);
-          const V3 tr = mulv(mat3v(mat.transmittance), v3(c.x, c.y, c.z));
-          f = tr * (1.0f - mat.dissolve) + f * mat.dissolve;
-        }
-        out = f4(f.x, f.y, f.z, 1.0f);
+      }
+      if (tp.enable_direct)
+        fdir = direct_light<SAMPLER, ISO, STORAGE, false>(sp, m, tp.enable_shadow, mat, pos, nrm, view_dir, nullptr, 0);
+      const float sap = specular_aperture(mat.shininess);
+      if (tp.enable_specular) {
+        const V3 sd = normalize(reflect(-view_dir, nrm));
+        const float4 c = trace_cone<SAMPLER, ISO, STORAGE>(m, pos, sd, sap, kMaxDistance);
+        fs = mulv(mat3v(mat.specular), v3(c.x, c.y, c.z));
+      }
+      V3 f = fs + fd + fdir;
+      if (refracts(mat) && tp.enable_specular) {
+        const V3 rd = refract(view_dir, nrm, 1.0f / mat.ior);
+        const float4 c = trace_cone<SAMPLER, ISO, STORAGE>(m, pos, rd, sap, kMaxDistance);
+        const V3 tr = mulv(mat3v(mat.transmittance), v3(c.x, c.y, c.z));
+        f = tr * (1.0f - mat.dissolve) + f * mat.dissolve;
+      }
+      out = f4(f.x, f.y, f.z, 1.0f);
+    }
+  }
+  frame[p] = make_uchar4(unorm8(out.x), unorm8(out.y), unorm8(out.z), unorm8(out.w));
+  if (frame_f32) frame_f32[p] = out;
+}
+
+// The voxel debug view (:253-257): one lookup a pixel.
+template <int SAMPLER, bool ISO, int STORAGE>
+__global__ void __launch_bounds__(256) k_view(SceneParams sp, CameraParams cp, const __grid_constant__ MapSet m,
+                                              TraceParams tp, const float4* __restrict__ gb_pos,
+                                              const float4* __restrict__ gb_nrm, uchar4* __restrict__ frame,
+                                              float4* __restrict__ frame_f32) {
+  const int px = blockIdx.x * 16 + (threadIdx.x & 15), py = blockIdx.y * 16 + (threadIdx.x >> 4);
+  if (px >= cp.W || py >= cp.H) return;
+  const size_t p = (size_t)py * cp.W + px;
+  float4 out = f4(0.15f, 0.25f, 0.25f, 1.0f);  // glClearColor, renderer.cpp:398
+  if (__float_as_uint(gb_nrm[p].w) != 0xffffffffu) {
+    const float4 g0 = gb_pos[p];
+    const V3 pos = v3(g0.x / sp.cube_size, g0.y / sp.cube_size, g0.z / sp.cube_size) * 0.5f + v3(0.5f, 0.5f, 0.5f);
+    // within_cube(pos, 0) (:61-64, 250): a fragment outside returns without
+    // writing; the pixel keeps the clear colour.
+    if (fabsf(pos.x) < 1.0f && fabsf(pos.y) < 1.0f && fabsf(pos.z) < 1.0f) {
+      // (map 6: the isotropic chain of VCT_MIP_BOTH; no such map otherwise)
+      out = f4(0.f, 0.f, 0.f, 0.f);
+      if (tp.view_voxel_dir >= 0 && (tp.view_voxel_dir <= 5 || (tp.view_voxel_dir == 6 && m.nmaps == 7))) {
+        const int d = ISO ? 0 : tp.view_voxel_dir;
+        out = sample_voxel<SAMPLER, ISO, STORAGE>(m, pos, d, d, d, v3(1.f, 0.f, 0.f), fmaxf(tp.view_voxel_lod, 0.0f));
       }
     }
   }
@@ -402,15 +395,113 @@ __device__ __forceinline__ void trace_px(const SceneParams& sp, const CameraPara
   if (frame_f32) frame_f32[p] = out;
 }
 
-template <int SAMPLER, bool ISO, int STORAGE>
-__global__ void __launch_bounds__(kTraceThreads, SAMPLER == VCT_SAMPLER_HW ? kTraceMinBlocks : 1)
-    k_trace(SceneParams sp, CameraParams cp, MapSet m, TraceParams tp, const float4* __restrict__ gb_pos,
-            const float4* __restrict__ gb_nrm, uchar4* __restrict__ frame, float4* __restrict__ frame_f32) {
+// A frame with the FP32 software sampler (main, :246-275).  A step of a cone
+// is 48 texel loads and their arithmetic, so a pixel's cones one after the
+// other are a long serial chain and a small frame leaves most of the chip
+// idle: a CTA takes an 8x4-pixel block with a warp per cone -- the diffuse
+// cones, the specular (and refracted) one, the lights' shadow cones shared by
+// up to kExactLights warps -- and its first warp puts them together.
+// 320x180, 64^3, one light (GB300, trace): 1741 us with a thread per pixel
+// (255 registers, 8 warps an SM), 958 as here at 128 registers, 700 at 48,
+// 647 at 40 (it spills 0.8 KB; more resident warps are worth it).  Bound by
+// instructions (unpacking and weighting texels: ALU pipe 56%).
+constexpr int kExactLights = 2;
+template <bool ISO, int STORAGE>
+__global__ void __launch_bounds__((9 + 1 + kExactLights) * 32, 4)
+    k_trace_exact(SceneParams sp, CameraParams cp, const __grid_constant__ MapSet m, TraceParams tp, int diffuse_warps,
+                  int light_warps, const float4* __restrict__ gb_pos, const float4* __restrict__ gb_nrm,
+                  uchar4* __restrict__ frame, float4* __restrict__ frame_f32) {
+  __shared__ float s_cone[11][3][32];  // 0-8: the diffuse cones, 9: specular, 10: refracted
+  __shared__ float s_occ[kMaxLights][32];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  trace_px<SAMPLER, ISO, STORAGE>(
-      sp, cp, m, tp, gb_pos, gb_nrm, frame, frame_f32,
-      blockIdx.x * 16 + (w % (16 / kTraceWarpW)) * kTraceWarpW + lane % kTraceWarpW,
-      blockIdx.y * kTraceRows + (w / (16 / kTraceWarpW)) * (32 / kTraceWarpW) + lane / kTraceWarpW);
+  const int px = blockIdx.x * 8 + (lane & 7), py = blockIdx.y * 4 + (lane >> 3);
+  const size_t p = (size_t)py * cp.W + px;
+  const bool inside = px < cp.W && py < cp.H;
+  bool valid = false;
+  float4 g0 = f4(0.f, 0.f, 0.f, 0.f);
+  V3 pos = v3(0.f, 0.f, 0.f), nrm = v3(0.f, 0.f, 1.f);
+  if (inside) {
+    const float4 g1 = gb_nrm[p];
+    if (__float_as_uint(g1.w) != 0xffffffffu) {
+      g0 = gb_pos[p];
+      pos = v3(g0.x / sp.cube_size, g0.y / sp.cube_size, g0.z / sp.cube_size) * 0.5f + v3(0.5f, 0.5f, 0.5f);
+      nrm = v3(g1.x, g1.y, g1.z);
+      valid = fabsf(pos.x) < 1.0f && fabsf(pos.y) < 1.0f && fabsf(pos.z) < 1.0f;  // within_cube, :250
+    }
+  }
+  const int nl = min(max(sp.n_lights, 0), kMaxLights);
+  const vct_material_data& mat = sp.materials[valid ? __float_as_uint(g0.w) : 0u];
+  const V3 view_dir = normalize(v3(g0.x, g0.y, g0.z) - v3(cp.cam_pos[0], cp.cam_pos[1], cp.cam_pos[2]));
+  auto keep = [&](int slot, float4 c) {
+    s_cone[slot][0][lane] = c.x;
+    s_cone[slot][1][lane] = c.y;
+    s_cone[slot][2][lane] = c.z;
+  };
+  if (valid) {
+    const int r = w - diffuse_warps;
+    if (r > 0) {
+      for (int i = r - 1; i < nl; i += light_warps) {
+        V3 ld;
+        float d;
+        light_dir(sp, i, pos, ld, d);
+        s_occ[i][lane] = m.skip_empty ? trace_shadow<VCT_SAMPLER_EXACT, ISO, STORAGE, false, true>(
+                                            m, m.sched->shadow.group, pos, ld, d)
+                                      : trace_shadow<VCT_SAMPLER_EXACT, ISO, STORAGE, false, false>(
+                                            m, m.sched->shadow.group, pos, ld, d);
+      }
+    } else {
+      // a diffuse cone, or the specular one and, of transparent materials, the refracted one
+      int slot = w;
+      V3 dir;
+      float ap;
+      if (r < 0) {
+        const V3 o1 = normalize(tangent(nrm));
+        const V3 o2 = normalize(cross(o1, nrm));
+        dir = diffuse_dir(tp.cone_set, m.sched->ring, nrm, o1, o2, w, ap);
+      } else {
+        slot = 9;
+        dir = normalize(reflect(-view_dir, nrm));
+        ap = specular_aperture(mat.shininess);
+      }
+      const int passes = r < 0 ? 1 : (!tp.enable_specular ? 0 : (refracts(mat) ? 2 : 1));
+#pragma unroll 1
+      for (int pass = 0; pass < passes; ++pass) {
+        if (pass) dir = refract(view_dir, nrm, 1.0f / mat.ior);
+        keep(slot + pass, trace_cone<VCT_SAMPLER_EXACT, ISO, STORAGE>(m, pos, dir, ap, kMaxDistance));
+      }
+    }
+  }
+  __syncthreads();
+  if (w != 0 || !inside) return;
+  float4 out = f4(0.15f, 0.25f, 0.25f, 1.0f);  // glClearColor, renderer.cpp:398
+  if (valid) {
+    auto cone = [&](int slot) { return v3(s_cone[slot][0][lane], s_cone[slot][1][lane], s_cone[slot][2][lane]); };
+    V3 fd = v3(0.f, 0.f, 0.f), fdir = v3(0.f, 0.f, 0.f), fs = v3(0.f, 0.f, 0.f);
+    if (tp.enable_diffuse) {
+      V3 d;
+      if (tp.diffuse_in) {
+        const float4 q = tp.diffuse_in[p];
+        d = v3(q.x, q.y, q.z);
+      } else {
+        d = cone(0);
+        for (int k = 1; k < diffuse_warps; ++k) d = d + cone(k);
+        d = d * (1.0f / (float)diffuse_warps);
+      }
+      fd = mulv(mat3v(mat.diffuse), d);
+    }
+    if (tp.enable_direct)
+      fdir = direct_light<VCT_SAMPLER_EXACT, ISO, STORAGE, true>(sp, m, tp.enable_shadow, mat, pos, nrm, view_dir,
+                                                                 &s_occ[0][lane], 32);
+    if (tp.enable_specular) fs = mulv(mat3v(mat.specular), cone(9));
+    V3 f = fs + fd + fdir;
+    if (refracts(mat) && tp.enable_specular) {
+      const V3 tr = mulv(mat3v(mat.transmittance), cone(10));
+      f = tr * (1.0f - mat.dissolve) + f * mat.dissolve;
+    }
+    out = f4(f.x, f.y, f.z, 1.0f);
+  }
+  frame[p] = make_uchar4(unorm8(out.x), unorm8(out.y), unorm8(out.z), unorm8(out.w));
+  if (frame_f32) frame_f32[p] = out;
 }
 
 // One pixel of the one-launch batch tracers: the warp (a block of kShareW x 2 groups, its
@@ -627,10 +718,24 @@ __global__ void __launch_bounds__(256, SHARE ? kTraceBatchShareMinBlocks : kTrac
 }
 
 template <int SAMPLER, bool ISO, int STORAGE>
-cudaError_t run(const SceneParams& sp, const CameraParams& cp, const MapSet& ms, const TraceParams& tp,
-                const float4* gb_pos, const float4* gb_nrm, uchar4* frame, float4* frame_f32, cudaStream_t st) {
-  dim3 grid((cp.W + 15) / 16, (cp.H + kTraceRows - 1) / kTraceRows);
-  k_trace<SAMPLER, ISO, STORAGE><<<grid, kTraceThreads, 0, st>>>(sp, cp, ms, tp, gb_pos, gb_nrm, frame, frame_f32);
+cudaError_t run_view(const SceneParams& sp, const CameraParams& cp, const MapSet& ms, const TraceParams& tp,
+                     const float4* gb_pos, const float4* gb_nrm, uchar4* frame, float4* frame_f32, cudaStream_t st) {
+  const dim3 grid((cp.W + 15) / 16, (cp.H + 15) / 16);
+  k_view<SAMPLER, ISO, STORAGE><<<grid, 256, 0, st>>>(sp, cp, ms, tp, gb_pos, gb_nrm, frame, frame_f32);
+  return cudaGetLastError();
+}
+
+template <bool ISO, int STORAGE>
+cudaError_t run_exact(const SceneParams& sp, const CameraParams& cp, const MapSet& ms, const TraceParams& tp,
+                      const float4* gb_pos, const float4* gb_nrm, uchar4* frame, float4* frame_f32, cudaStream_t st) {
+  if (tp.view_voxel_dir < 7)
+    return run_view<VCT_SAMPLER_EXACT, ISO, STORAGE>(sp, cp, ms, tp, gb_pos, gb_nrm, frame, frame_f32, st);
+  const int nl = std::min(std::max(sp.n_lights, 0), kMaxLights);
+  const int diffuse = tp.enable_diffuse && !tp.diffuse_in ? (tp.cone_set == VCT_CONES_SIX60 ? 6 : 9) : 0;
+  const int lights = tp.enable_direct && tp.enable_shadow ? std::min(nl, kExactLights) : 0;
+  const dim3 grid((cp.W + 7) / 8, (cp.H + 3) / 4);
+  k_trace_exact<ISO, STORAGE><<<grid, (diffuse + 1 + lights) * 32, 0, st>>>(sp, cp, ms, tp, diffuse, lights, gb_pos,
+                                                                            gb_nrm, frame, frame_f32);
   return cudaGetLastError();
 }
 
@@ -772,16 +877,14 @@ cudaError_t launch_trace_px(const SceneParams& sp, const CameraParams& cp, const
                             const float4* gb_pos, const float4* gb_nrm, uchar4* frame, float4* frame_f32,
                             cudaStream_t st, int* launches) {
   if (launches) ++*launches;
-  const bool iso = tp.mip_mode == VCT_MIP_ISO;
+  const bool iso = tp.mip_mode == VCT_MIP_ISO, rgba8 = ms.storage == VCT_STORAGE_RGBA8;
   if (tp.sampler == VCT_SAMPLER_EXACT) {
-    if (ms.storage == VCT_STORAGE_RGBA8)
-      return iso ? run<VCT_SAMPLER_EXACT, true, VCT_STORAGE_RGBA8>(sp, cp, ms, tp, gb_pos, gb_nrm, frame, frame_f32, st)
-                 : run<VCT_SAMPLER_EXACT, false, VCT_STORAGE_RGBA8>(sp, cp, ms, tp, gb_pos, gb_nrm, frame, frame_f32, st);
-    return iso ? run<VCT_SAMPLER_EXACT, true, VCT_STORAGE_RGBA16F>(sp, cp, ms, tp, gb_pos, gb_nrm, frame, frame_f32, st)
-               : run<VCT_SAMPLER_EXACT, false, VCT_STORAGE_RGBA16F>(sp, cp, ms, tp, gb_pos, gb_nrm, frame, frame_f32, st);
+    auto run = iso ? (rgba8 ? run_exact<true, VCT_STORAGE_RGBA8> : run_exact<true, VCT_STORAGE_RGBA16F>)
+                   : (rgba8 ? run_exact<false, VCT_STORAGE_RGBA8> : run_exact<false, VCT_STORAGE_RGBA16F>);
+    return run(sp, cp, ms, tp, gb_pos, gb_nrm, frame, frame_f32, st);
   }
-  return iso ? run<VCT_SAMPLER_HW, true, VCT_STORAGE_RGBA8>(sp, cp, ms, tp, gb_pos, gb_nrm, frame, frame_f32, st)
-             : run<VCT_SAMPLER_HW, false, VCT_STORAGE_RGBA8>(sp, cp, ms, tp, gb_pos, gb_nrm, frame, frame_f32, st);
+  auto run = iso ? run_view<VCT_SAMPLER_HW, true, VCT_STORAGE_RGBA8> : run_view<VCT_SAMPLER_HW, false, VCT_STORAGE_RGBA8>;
+  return run(sp, cp, ms, tp, gb_pos, gb_nrm, frame, frame_f32, st);
 }
 
 }  // namespace vct

@@ -413,8 +413,7 @@ cudaError_t launch_cone_schedules(const MapSet& ms, ConeSchedules* out, cudaStre
 cudaError_t launch_trace(const SceneParams& sp, const CameraParams& cp, const MapSet& ms, const TraceParams& tp,
                          const float4* gb_pos, const float4* gb_nrm, uchar4* frame, float4* frame_f32,
                          const ConeSchedules& sched, const TraceWork& tw, cudaStream_t st, int* launches);
-// A thread per pixel and everything in one kernel: the FP32 software sampler
-// and the voxel debug view.
+// A frame in one kernel: the FP32 software sampler and the voxel debug view.
 cudaError_t launch_trace_px(const SceneParams& sp, const CameraParams& cp, const MapSet& ms, const TraceParams& tp,
                             const float4* gb_pos, const float4* gb_nrm, uchar4* frame, float4* frame_f32,
                             cudaStream_t st, int* launches);
