@@ -80,7 +80,8 @@ struct vct_batch {
   uint32_t bin_big_cap = 0;
   HeavyStore heavy;
   DevBuf<unsigned char> rbig;
-  DevBuf<uint32_t> rbig_count, rbig_offset;
+  DevBuf<unsigned long long> rbig_count;
+  DevBuf<uint32_t> rbig_first;
   uint32_t rbig_cap = 0;
   DevBuf<unsigned long long> vis;
   DevBuf<float4> gb_pos, gb_nrm;
@@ -136,8 +137,7 @@ struct vct_batch {
     bb.rb.big = rbig.p;
     bb.rb.big_cap = rbig_cap;
     bb.rb.big_count = rbig_count.p;
-    bb.rb.big_offset = rbig_offset.p;
-    bb.rb.scan_tmp = nullptr;
+    bb.rb.big_first = rbig_first.p;
     bb.rb.gb_pos = gb_pos.p;
     bb.rb.gb_nrm = gb_nrm.p;
     bb.rb.status = d_status.p;
@@ -167,7 +167,7 @@ struct vct_batch {
   }
   vct_status grow_rbig(uint32_t cap) {
     VCT_CHECK(rbig.ensure((size_t)cap * big_record_bytes()));
-    VCT_CHECK(rbig_offset.ensure((size_t)cap + 1));
+    VCT_CHECK(rbig_first.ensure(cap));
     rbig_cap = cap;
     return VCT_OK;
   }
@@ -508,7 +508,7 @@ vct_status build_batch(vct_batch* b, const vct_batch_scene* descs, uint32_t n) {
   VCT_CHECK(b->bin_rec.ensure(std::max<size_t>(b->tris.total(), 1)));
   VCT_CHECK(b->bin_big_count.ensure(1));
   VCT_CHECK(b->grow_bin_big(1 << 12));
-  VCT_CHECK(b->rbig_count.ensure(2));
+  VCT_CHECK(b->rbig_count.ensure(1));
   VCT_CHECK(b->grow_rbig(1 << 16));
   VCT_CHECK(b->queue.ensure(2));
   VCT_CHECK(b->vis.ensure(px));

@@ -9,10 +9,9 @@
 //                  order); triangles crossing the near plane or a guard band
 //                  of |x|,|y| <= 16w are clipped (Sutherland-Hodgman) and
 //                  fanned; vertices snapped to 1/256 pixel; triangles whose
-//                  pixel box holds <= 32 pixels are rasterised right here,
-//                  larger ones become records for the tiled pass.
-//   k_gb_big_*  -- 16x16-pixel tiles of the large triangles, one pixel per
-//                  thread.
+//                  pixel box holds <= 64 pixels are rasterised right here,
+//                  larger ones become records.
+//   k_gb_big    -- a warp per 32x32-pixel tile of a record's box.
 //   coverage    -- integer edge functions at pixel centres, top-left rule;
 //                  depth = FP32 z_window interpolated in screen space; the
 //                  visibility buffer keeps min((depth bits << 32) | triangle
@@ -24,23 +23,31 @@
 
 #include "vct_internal.h"
 #include "vct_math.cuh"
+#include "vct_snap.h"
 
 namespace vct {
 namespace {
 
-constexpr int kSmallPixels = 32;
-constexpr int kTile = 16;
+// The box a setup thread rasters itself: its loop is serial, a record costs an
+// atomic and a warp of k_gb_big.  G-buffer of 500,000 triangles at 1920x1080 and
+// 120,000 at 1367x771: 8 pixels 172 and 174 us, 16 129 and 96, 32 110 and 89,
+// 64 106 and 84.
+constexpr int kSmallPixels = 64;
+constexpr int kTileBits = 5;  // a large triangle's tile: 32x32 pixels of its box
+constexpr int kTile = 1 << kTileBits;
+constexpr int kAcross = 2;    // blocks of a row in flight
+constexpr int kSetup = 128;   // threads of a setup block
 constexpr float kGuard = 16.0f;
 
+// A screen triangle: counter-clockwise, snapped vertices, window depths.
 struct BigRec {
-  long long area;
   int X[3], Y[3];
   float z[3];
   float farea;
   uint32_t tri;
-  int tl;
+  int tl;              // bit k: edge k keeps the samples on it
   int x0, y0, x1, y1;  // pixel bbox (inclusive)
-  int tw;              // tiles across
+  uint32_t tw;         // tiles across
   uint32_t scene;      // scene of a batch (0 for one renderer)
 };
 
@@ -80,94 +87,146 @@ __device__ __forceinline__ float plane_eval(int pl, const CV& v) {
   }
 }
 
-__device__ __forceinline__ void plot(unsigned long long* vis, int W, int px, int py, float zz, uint32_t tri) {
-  if (!(zz < 1.0f)) return;
+// The visibility key of depth zz: ~0 (never stored) past the far plane.
+__device__ __forceinline__ unsigned long long depth_key(float zz, uint32_t tri) {
+  if (!(zz < 1.0f)) return ~0ull;
   if (!(zz > 0.0f)) zz = 0.0f;
-  const unsigned long long key = ((unsigned long long)__float_as_uint(zz) << 32) | tri;
-  unsigned long long* slot = vis + (size_t)py * W + px;
-  if (key < *reinterpret_cast<volatile unsigned long long*>(slot)) atomicMin(slot, key);
+  return ((unsigned long long)__float_as_uint(zz) << 32) | tri;
 }
 
-__device__ __forceinline__ void pixel_test(const BigRec& r, unsigned long long* vis, int W, int px, int py) {
-  const long long sx = 256LL * px + 128, sy = 256LL * py + 128;
-  const long long w0 = edge_fn(r.X[1], r.Y[1], r.X[2], r.Y[2], sx, sy);
-  const long long w1 = edge_fn(r.X[2], r.Y[2], r.X[0], r.Y[0], sx, sy);
-  const long long w2 = edge_fn(r.X[0], r.Y[0], r.X[1], r.Y[1], sx, sy);
-  if (!(w0 > 0 || (w0 == 0 && (r.tl & 1)))) return;
-  if (!(w1 > 0 || (w1 == 0 && (r.tl & 2)))) return;
-  if (!(w2 > 0 || (w2 == 0 && (r.tl & 4)))) return;
-  const float b1 = rdiv(__ll2float_rn(w1), r.farea), b2 = rdiv(__ll2float_rn(w2), r.farea);
+// The edge functions of a triangle at a pixel centre, each lowered by one
+// where the edge does not keep the samples on it: inside = none negative.
+template <class T>
+struct Edges {
+  T w[3];
+  T dx[3], dy[3];  // per pixel across, per pixel up
+  int on[3];       // what w was lowered by
+  __device__ __forceinline__ void at(const BigRec& r, int px, int py) {
+    const T sx = (T)(256 * px + 128), sy = (T)(256 * py + 128);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const int a = (k + 1) % 3, b = (k + 2) % 3;  // edge k: vertex k + 1 -> vertex k + 2
+      const T ex = (T)r.X[b] - r.X[a], ey = (T)r.Y[b] - r.Y[a];
+      on[k] = (r.tl >> k) & 1 ? 0 : 1;
+      w[k] = ex * (sy - r.Y[a]) - ey * (sx - r.X[a]) - on[k];
+      dx[k] = -ey * 256;
+      dy[k] = ex * 256;
+    }
+  }
+  __device__ __forceinline__ bool inside() const { return (w[0] | w[1] | w[2]) >= 0; }
+};
+__device__ __forceinline__ float to_float(int v) { return __int2float_rn(v); }
+__device__ __forceinline__ float to_float(long long v) { return __ll2float_rn(v); }
+
+template <class T>
+__device__ __forceinline__ unsigned long long pixel_key(const BigRec& r, const Edges<T>& e) {
+  const float b1 = rdiv(to_float(e.w[1] + e.on[1]), r.farea), b2 = rdiv(to_float(e.w[2] + e.on[2]), r.farea);
   float zz = radd(r.z[0], rmul(b1, rsub(r.z[1], r.z[0])));
   zz = radd(zz, rmul(b2, rsub(r.z[2], r.z[0])));
-  plot(vis, W, px, py, zz, r.tri);
+  return depth_key(zz, r.tri);
+}
+
+// Rasterises the record's whole box, one thread.
+template <class T>
+__device__ __forceinline__ void raster_box(const BigRec& r, unsigned long long* vis, int W) {
+  Edges<T> e;
+  e.at(r, r.x0, r.y0);
+  for (int py = r.y0; py <= r.y1; ++py) {
+    Edges<T> q = e;
+    for (int px = r.x0; px <= r.x1; ++px) {
+      if (q.inside()) {
+        const unsigned long long key = pixel_key(r, q);
+        if (key != ~0ull) atomicMin(vis + (size_t)py * W + px, key);
+      }
+#pragma unroll
+      for (int k = 0; k < 3; ++k) q.w[k] += q.dx[k];
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) e.w[k] += e.dy[k];
+  }
+}
+
+// 1/256-pixel coordinate of normalised device coordinate n on K / 128 pixels.
+__device__ __forceinline__ int snap_ndc(float n, int K) {
+  bool close;
+  const int v = snap_scaled(n, (uint32_t)K, close);
+  if (!close) return v;
+  return (int)__double2ll_rn(__dmul_rn(__dadd_rn((double)n, 1.0), (double)K));
 }
 
 // Set up one (possibly clipped) screen triangle; raster it here if small.
-__device__ void raster_subtri(const CV v[3], const CameraParams& cp, uint32_t tri, const RasterBuffers& rb,
-                              uint32_t scene) {
+__device__ __forceinline__ void raster_subtri(const CV v[3], int W, int H, uint32_t tri, const RasterBuffers& rb,
+                                              uint32_t scene) {
   BigRec r;
-  long long X[3], Y[3];
   for (int k = 0; k < 3; ++k) {
     if (!(v[k].c[3] > 0.0f)) return;
     const float nx = rdiv(v[k].c[0], v[k].c[3]), ny = rdiv(v[k].c[1], v[k].c[3]), nz = rdiv(v[k].c[2], v[k].c[3]);
     if (!(fabsf(nx) <= 64.0f) || !(fabsf(ny) <= 64.0f) || !(nz == nz)) return;
-    X[k] = __double2ll_rn(__dmul_rn(__dadd_rn((double)nx, 1.0), (double)cp.W * 128.0));
-    Y[k] = __double2ll_rn(__dmul_rn(__dadd_rn((double)ny, 1.0), (double)cp.H * 128.0));
+    r.X[k] = snap_ndc(nx, W * 128);
+    r.Y[k] = snap_ndc(ny, H * 128);
     r.z[k] = radd(rmul(0.5f, nz), 0.5f);
   }
-  long long area = (X[1] - X[0]) * (Y[2] - Y[0]) - (Y[1] - Y[0]) * (X[2] - X[0]);
+  const long long ax = r.X[1] - r.X[0], ay = r.Y[1] - r.Y[0], bx = r.X[2] - r.X[0], by = r.Y[2] - r.Y[0];
+  long long area = ax * by - ay * bx;
   if (area == 0) return;
   if (area < 0) {
-    long long t = X[1]; X[1] = X[2]; X[2] = t;
-    t = Y[1]; Y[1] = Y[2]; Y[2] = t;
+    int t = r.X[1]; r.X[1] = r.X[2]; r.X[2] = t;
+    t = r.Y[1]; r.Y[1] = r.Y[2]; r.Y[2] = t;
     float tz = r.z[1]; r.z[1] = r.z[2]; r.z[2] = tz;
     area = -area;
   }
-  const long long x0 = max(0LL, ceil_div(min(X[0], min(X[1], X[2])) - 128, 256));
-  const long long x1 = min((long long)cp.W - 1, floor_div(max(X[0], max(X[1], X[2])) - 128, 256));
-  const long long y0 = max(0LL, ceil_div(min(Y[0], min(Y[1], Y[2])) - 128, 256));
-  const long long y1 = min((long long)cp.H - 1, floor_div(max(Y[0], max(Y[1], Y[2])) - 128, 256));
-  if (x1 < x0 || y1 < y0) return;
-  r.area = area;
+  // the pixels whose centres (256 p + 128) lie in the box
+  const int minx = min(r.X[0], min(r.X[1], r.X[2])), maxx = max(r.X[0], max(r.X[1], r.X[2]));
+  const int miny = min(r.Y[0], min(r.Y[1], r.Y[2])), maxy = max(r.Y[0], max(r.Y[1], r.Y[2]));
+  r.x0 = max(0, (minx + 127) >> 8);
+  r.x1 = min(W - 1, (maxx - 128) >> 8);
+  r.y0 = max(0, (miny + 127) >> 8);
+  r.y1 = min(H - 1, (maxy - 128) >> 8);
+  if (r.x1 < r.x0 || r.y1 < r.y0) return;
   r.farea = __ll2float_rn(area);
-  for (int k = 0; k < 3; ++k) { r.X[k] = (int)X[k]; r.Y[k] = (int)Y[k]; }
-  r.tl = (top_left(X[1], Y[1], X[2], Y[2]) ? 1 : 0) | (top_left(X[2], Y[2], X[0], Y[0]) ? 2 : 0) |
-         (top_left(X[0], Y[0], X[1], Y[1]) ? 4 : 0);
+  r.tl = (top_left(r.X[1], r.Y[1], r.X[2], r.Y[2]) ? 1 : 0) | (top_left(r.X[2], r.Y[2], r.X[0], r.Y[0]) ? 2 : 0) |
+         (top_left(r.X[0], r.Y[0], r.X[1], r.Y[1]) ? 4 : 0);
   r.tri = tri;
-  r.x0 = (int)x0; r.x1 = (int)x1; r.y0 = (int)y0; r.y1 = (int)y1;
-  const long long npx = (x1 - x0 + 1) * (y1 - y0 + 1);
-  if (npx <= kSmallPixels) {
-    for (int py = r.y0; py <= r.y1; ++py)
-      for (int px = r.x0; px <= r.x1; ++px) pixel_test(r, rb.vis, cp.W, px, py);
+  const int nx = r.x1 - r.x0 + 1, ny = r.y1 - r.y0 + 1;
+  if (nx * ny <= kSmallPixels) {
+    // (within 2^14 the products of two differences stay below 2^29)
+    if (maxx - minx <= (1 << 14) && maxy - miny <= (1 << 14)) raster_box<int>(r, rb.vis, W);
+    else raster_box<long long>(r, rb.vis, W);
     return;
   }
-  r.tw = (r.x1 - r.x0 + kTile) / kTile;
   r.scene = scene;
-  const uint32_t slot = atomicAdd(&rb.big_count[0], 1u);
-  if (slot < rb.big_cap) reinterpret_cast<BigRec*>(rb.big)[slot] = r;
+  // Records and tiles are counted in one word, so the first tiles ascend with
+  // the records and need no scan.  The lanes with a single tile, most of them,
+  // share one atomic.
+  r.tw = (uint32_t)(nx + kTile - 1) >> kTileBits;
+  const uint32_t tiles = r.tw * ((uint32_t)(ny + kTile - 1) >> kTileBits);
+  unsigned long long at;
+  if (tiles == 1) {
+    const unsigned m = __activemask();
+    const int lane = threadIdx.x & 31, lead = __ffs((int)m) - 1;
+    unsigned long long base = 0;
+    if (lane == lead) base = atomicAdd(rb.big_count, (1ull << 32 | 1ull) * (unsigned)__popc(m));
+    at = __shfl_sync(m, base, lead) + (1ull << 32 | 1ull) * (unsigned)__popc(m & ((1u << lane) - 1u));
+  } else {
+    at = atomicAdd(rb.big_count, 1ull << 32 | tiles);
+  }
+  const uint32_t slot = (uint32_t)(at >> 32);
+  if (slot >= rb.big_cap) return;  // (reported; the frame is encoded again)
+  reinterpret_cast<BigRec*>(rb.big)[slot] = r;
+  rb.big_first[slot] = (uint32_t)at;
 }
 
-__device__ __forceinline__ void setup_tri(const SceneParams& sp, const CameraParams& cp, const RasterBuffers& rb,
-                                          uint32_t t, uint32_t scene) {
-  if (t >= sp.total_tris) return;
-  const DevInstance& in = sp.inst[find_instance(sp, t)];
-  const uint32_t lt = t - in.tri_base;
-  CV cv[3];
-  float w[3];
-  for (int k = 0; k < 3; ++k) vertex_clip(in, cp.PV, __ldg(in.indices + 3 * (size_t)lt + k), w, cv[k]);
-  bool all_in = true;
-  for (int pl = 0; pl < 5; ++pl)
-    for (int k = 0; k < 3; ++k)
-      if (!(plane_eval(pl, cv[k]) >= 0.0f)) all_in = false;
-  if (all_in) {
-    raster_subtri(cv, cp, t, rb, scene);
-    return;
-  }
+// The clipped triangle's fan, called, not inlined: its polygons live in local
+// memory, and few triangles need it.
+__device__ __noinline__ void raster_clipped(const CV cv[3], int W, int H, uint32_t t, const RasterBuffers& rb,
+                                            uint32_t scene) {
   CV a[10], b[10];
   int n = 3;
   for (int k = 0; k < 3; ++k) a[k] = cv[k];
+#pragma unroll 1
   for (int pl = 0; pl < 5; ++pl) {
     int m = 0;
+#pragma unroll 1
     for (int i = 0; i < n; ++i) {
       const CV p0 = a[i], p1 = a[(i + 1) % n];
       const float d0 = plane_eval(pl, p0), d1 = plane_eval(pl, p1);
@@ -184,13 +243,36 @@ __device__ __forceinline__ void setup_tri(const SceneParams& sp, const CameraPar
     for (int i = 0; i < n; ++i) a[i] = b[i];
     if (n < 3) return;
   }
+#pragma unroll 1
   for (int k = 1; k + 1 < n; ++k) {
     const CV tri3[3] = {a[0], a[k], a[k + 1]};
-    raster_subtri(tri3, cp, t, rb, scene);
+    raster_subtri(tri3, W, H, t, rb, scene);
   }
 }
 
-__global__ void __launch_bounds__(256) k_gb_setup(SceneParams sp, CameraParams cp, RasterBuffers rb) {
+__device__ __forceinline__ void setup_tri(const SceneParams& sp, const CameraParams& cp, const RasterBuffers& rb,
+                                          uint32_t t, uint32_t scene) {
+  if (t >= sp.total_tris) return;
+  const DevInstance& in = sp.inst[find_instance(sp, t)];
+  const uint32_t lt = t - in.tri_base;
+  CV cv[3];
+  float w[3];
+  for (int k = 0; k < 3; ++k) vertex_clip(in, cp.PV, __ldg(in.indices + 3 * (size_t)lt + k), w, cv[k]);
+  bool all_in = true;
+  for (int pl = 0; pl < 5; ++pl)
+    for (int k = 0; k < 3; ++k)
+      if (!(plane_eval(pl, cv[k]) >= 0.0f)) all_in = false;
+  if (all_in) raster_subtri(cv, cp.W, cp.H, t, rb, scene);
+  else raster_clipped(cv, cp.W, cp.H, t, rb, scene);
+}
+
+// Latency of the instance, index and vertex loads, so registers decide (64: 32
+// warps an SM): vertices are snapped without FP64, a rate-limited unit here;
+// small boxes take 32-bit stepped edge functions and fire-and-forget atomics
+// (reading the visibility word first, to skip the atomic, stalled on every
+// pixel); the clipper is a call.  500,000 triangles, 1920x1080: 86 us with
+// FP64 and the clipper inline (98 registers), 38 now.
+__global__ void __launch_bounds__(kSetup, 8) k_gb_setup(SceneParams sp, CameraParams cp, RasterBuffers rb) {
   setup_tri(sp, cp, rb, blockIdx.x * blockDim.x + threadIdx.x, 0u);
 }
 
@@ -203,7 +285,7 @@ __device__ __forceinline__ RasterBuffers scene_rb(const RasterBuffers& rb, const
   return r;
 }
 
-__global__ void __launch_bounds__(256) k_gb_setup_batch(BatchWork w, RasterBuffers rb) {
+__global__ void __launch_bounds__(kSetup, 8) k_gb_setup_batch(BatchWork w, RasterBuffers rb) {
   for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < w.total; g += gridDim.x * blockDim.x) {
     const int s = batch_scene_of(w, g);
     const BatchScene& S = w.scenes[s];
@@ -211,70 +293,90 @@ __global__ void __launch_bounds__(256) k_gb_setup_batch(BatchWork w, RasterBuffe
   }
 }
 
-// Tile counts of the large-triangle records -> exclusive prefix (one CTA).
-__global__ void __launch_bounds__(1024) k_gb_big_scan(RasterBuffers rb) {
-  __shared__ uint32_t warp_tot[32];
-  __shared__ uint32_t s_carry;
-  const uint32_t n = min(rb.big_count[0], rb.big_cap);
-  const BigRec* rec = reinterpret_cast<const BigRec*>(rb.big);
-  if (threadIdx.x == 0) s_carry = 0;
-  __syncthreads();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (uint32_t base = 0; base < n; base += 1024) {
-    const uint32_t i = base + threadIdx.x;
-    uint32_t v = 0;
-    if (i < n) v = (uint32_t)rec[i].tw * (uint32_t)((rec[i].y1 - rec[i].y0 + kTile) / kTile);
-    uint32_t incl = v;
-    for (int o = 1; o < 32; o <<= 1) {
-      uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += t;
-    }
-    if (lane == 31) warp_tot[warp] = incl;
-    __syncthreads();
-    if (warp == 0) {
-      uint32_t wv = warp_tot[lane], wi = wv;
-      for (int o = 1; o < 32; o <<= 1) {
-        uint32_t t = __shfl_up_sync(0xffffffffu, wi, o);
-        if (lane >= o) wi += t;
-      }
-      warp_tot[lane] = wi - wv;
-    }
-    __syncthreads();
-    const uint32_t carry = s_carry;
-    if (i < n) rb.big_offset[i] = carry + warp_tot[warp] + incl - v;
-    __syncthreads();
-    if (threadIdx.x == 1023) s_carry = carry + warp_tot[warp] + incl;
-    __syncthreads();
+// The last of n ascending values that is not above x (the first one is not),
+// found by a warp.
+__device__ __forceinline__ uint32_t warp_last_not_above(const uint32_t* __restrict__ v, uint32_t n, uint32_t x) {
+  const uint32_t lane = threadIdx.x & 31;
+  uint32_t lo = 0, hi = n;
+  while (hi - lo > 1) {
+    const uint32_t step = (hi - lo + 31) / 32, i = lo + lane * step;
+    const unsigned below = __ballot_sync(0xffffffffu, i < hi && __ldg(v + i) <= x);
+    lo += (31 - __clz((int)below)) * step;
+    hi = min(hi, lo + step);
   }
-  if (threadIdx.x == 0) {
-    rb.big_offset[n] = s_carry;
-    rb.big_count[1] = s_carry;
-    rb.status->big_total = rb.big_count[0];
-    rb.status->big_tiles = s_carry;
-  }
+  return lo;
 }
 
-__global__ void __launch_bounds__(kTile * kTile) k_gb_big(RasterBuffers rb, int W, const BatchScene* scenes) {
-  const uint32_t n = min(rb.big_count[0], rb.big_cap);
-  const uint32_t total = rb.big_count[1];
-  const BigRec* rec = reinterpret_cast<const BigRec*>(rb.big);
-  for (uint32_t t = blockIdx.x; t < total; t += gridDim.x) {
-    int lo = 0, hi = (int)n - 1;
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (rb.big_offset[mid] <= t) lo = mid; else hi = mid - 1;
-    }
-    const BigRec& r = rec[lo];
-    const uint32_t lt = t - rb.big_offset[lo];
-    const int tx = (int)(lt % (uint32_t)r.tw), ty = (int)(lt / (uint32_t)r.tw);
-    const int px = r.x0 + tx * kTile + (threadIdx.x % kTile), py = r.y0 + ty * kTile + (threadIdx.x / kTile);
+// The large triangles' tiles, a warp each, 8x4 pixels at a time with the edge
+// functions stepped from block to block.  A warp finds its tile's record in
+// the ascending first tiles by a 32-way search (three or four probes); a tile
+// wholly outside an edge stops there.  Bound by the chain of loads to the
+// record and by the atomics' issue, which is why they return nothing.  16x16
+// tiles with a thread to a pixel, a scan kernel for their offsets and a binary
+// search in every thread took 75 + 5 us (1920x1080, 500,000 triangles), this
+// takes 20; 16 scenes in a batch 752 + 102 -> 95.  Lists of tiles written by
+// the setup thread were no alternative: one thread writes a whole screen's
+// (64x64 tiles 155 us for all of the G-buffer, 32x32 210).
+__global__ void __launch_bounds__(256) k_gb_big(RasterBuffers rb, int W, const BatchScene* scenes) {
+  const uint32_t total = (uint32_t)*rb.big_count, records = (uint32_t)(*rb.big_count >> 32);
+  const int lane = threadIdx.x & 31;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    rb.status->big_total = records;
+    rb.status->big_tiles = total;
+  }
+  // few tiles: up to 8 warps on one, each taking every so many-th row of blocks
+  const uint32_t warps = gridDim.x * 8;
+  int sh = 0;
+  while (sh < 3 && total <= warps >> (sh + 1)) ++sh;
+  for (uint32_t j = blockIdx.x * 8 + (threadIdx.x >> 5); j >> sh < total; j += warps) {
+    const uint32_t t = j >> sh;
+    const int strip = (int)(j & ((1u << sh) - 1)) * 4, step = 4 << sh;
+    const uint32_t n = warp_last_not_above(rb.big_first, min(records, rb.big_cap), t);
+    // (past a full list's last record t lies below its box: no rows)
+    const BigRec r = reinterpret_cast<const BigRec*>(rb.big)[n];
+    const uint32_t lt = t - rb.big_first[n];
     unsigned long long* vis = rb.vis;
     int w = W;
     if (scenes) {  // a batch: the record's scene
       vis += scenes[r.scene].px_base;
       w = scenes[r.scene].W;
     }
-    if (px <= r.x1 && py <= r.y1) pixel_test(r, vis, w, px, py);
+    const int x0 = r.x0 + (int)(lt % r.tw) * kTile, y0 = r.y0 + (int)(lt / r.tw) * kTile;
+    const int x1 = min(r.x1, x0 + kTile - 1), y1 = min(r.y1, y0 + kTile - 1);
+    Edges<long long> e;
+    e.at(r, x0, y0);
+    bool out = false;  // an edge with the whole tile outside
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+      out |= e.w[k] + max(e.dx[k] * (x1 - x0), 0ll) + max(e.dy[k] * (y1 - y0), 0ll) < 0;
+    if (out) continue;
+    const int lx = lane & 7, ly = lane >> 3;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      e.w[k] += e.dx[k] * lx + e.dy[k] * (ly + strip);
+      e.dx[k] *= 8;
+      e.dy[k] *= step;
+    }
+#pragma unroll 1
+    for (int py = y0 + strip + ly; py - ly <= y1; py += step) {
+      Edges<long long> q = e;
+#pragma unroll 1
+      for (int px = x0 + lx; px - lx <= x1; px += 8 * kAcross) {
+        unsigned long long key[kAcross], *slot = vis + (size_t)py * w + px;
+#pragma unroll
+        for (int u = 0; u < kAcross; ++u) {
+          key[u] = ~0ull;
+          if (q.inside() && px + 8 * u <= x1 && py <= y1) key[u] = pixel_key(r, q);
+#pragma unroll
+          for (int k = 0; k < 3; ++k) q.w[k] += q.dx[k];
+        }
+#pragma unroll
+        for (int u = 0; u < kAcross; ++u)
+          if (key[u] != ~0ull) atomicMin(slot + 8 * u, key[u]);
+      }
+#pragma unroll
+      for (int k = 0; k < 3; ++k) e.w[k] += e.dy[k];
+    }
   }
 }
 
@@ -347,17 +449,16 @@ cudaError_t launch_gbuffer(const SceneParams& sp, const CameraParams& cp, const 
                            int* launches) {
   cudaError_t e = cudaMemsetAsync(rb.vis, 0xff, (size_t)cp.W * cp.H * sizeof(unsigned long long), st);
   if (e != cudaSuccess) return e;
-  e = cudaMemsetAsync(rb.big_count, 0, 2 * sizeof(uint32_t), st);
+  e = cudaMemsetAsync(rb.big_count, 0, sizeof(*rb.big_count), st);
   if (e != cudaSuccess) return e;
-  if (sp.total_tris) k_gb_setup<<<(sp.total_tris + 255) / 256, 256, 0, st>>>(sp, cp, rb);
-  k_gb_big_scan<<<1, 1024, 0, st>>>(rb);
+  if (sp.total_tris) k_gb_setup<<<(sp.total_tris + kSetup - 1) / kSetup, kSetup, 0, st>>>(sp, cp, rb);
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  k_gb_big<<<sms * 8, kTile * kTile, 0, st>>>(rb, cp.W, nullptr);
+  k_gb_big<<<sms * 6, 256, 0, st>>>(rb, cp.W, nullptr);
   dim3 grid((cp.W + 15) / 16, (cp.H + 15) / 16);
   k_gb_resolve<<<grid, 256, 0, st>>>(sp, cp, rb);
-  if (launches) *launches += (sp.total_tris ? 1 : 0) + 3;
+  if (launches) *launches += (sp.total_tris ? 1 : 0) + 2;
   return cudaGetLastError();
 }
 
@@ -366,19 +467,18 @@ cudaError_t launch_gbuffer_batch(const BatchWork& tris, const BatchWork& tiles, 
   const RasterBuffers& rb = bb.rb;
   cudaError_t e = cudaMemsetAsync(rb.vis, 0xff, total_px * sizeof(unsigned long long), st);
   if (e != cudaSuccess) return e;
-  e = cudaMemsetAsync(rb.big_count, 0, 2 * sizeof(uint32_t), st);
+  e = cudaMemsetAsync(rb.big_count, 0, sizeof(*rb.big_count), st);
   if (e != cudaSuccess) return e;
   int nl = 0;
   if (tris.total) {
-    const unsigned grid = (unsigned)std::max(1, std::min<int>(sms * 4, (int)((tris.total + 255) / 256)));
-    k_gb_setup_batch<<<grid, 256, 0, st>>>(tris, rb);
+    const unsigned grid = (unsigned)std::max(1, std::min<int>(sms * 32, (int)((tris.total + kSetup - 1) / kSetup)));
+    k_gb_setup_batch<<<grid, kSetup, 0, st>>>(tris, rb);
     ++nl;
   }
-  k_gb_big_scan<<<1, 1024, 0, st>>>(rb);
-  k_gb_big<<<sms * 8, kTile * kTile, 0, st>>>(rb, 0, tris.scenes);
+  k_gb_big<<<sms * 6, 256, 0, st>>>(rb, 0, tris.scenes);
   const unsigned rgrid = (unsigned)std::max(1, std::min<int>(sms * 8, (int)tiles.total));
   k_gb_resolve_batch<<<rgrid, 256, 0, st>>>(tiles, rb);
-  nl += 3;
+  nl += 2;
   if (launches) *launches += nl;
   return cudaGetLastError();
 }

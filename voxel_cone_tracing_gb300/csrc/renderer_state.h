@@ -418,7 +418,8 @@ struct vct_renderer {
   HostBuf<FrameStatus> h_status;
   DevBuf<unsigned long long> vis;
   DevBuf<unsigned char> big;
-  DevBuf<uint32_t> big_count, big_offset;
+  DevBuf<unsigned long long> big_count;
+  DevBuf<uint32_t> big_first;
   uint32_t big_cap = 0;
   DevBuf<float4> gb_pos, gb_nrm;
   DevBuf<uchar4> frame;
@@ -599,7 +600,7 @@ struct vct_renderer {
     VCT_CHECK(d_status.ensure(1));
     VCT_CHECK(h_status.ensure(1));
     std::memset(h_status.p, 0, sizeof(FrameStatus));
-    VCT_CHECK(big_count.ensure(2));
+    VCT_CHECK(big_count.ensure(1));
     VCT_CHECK(grow_big(1 << 16));
     VCT_CHECK(grow_bin_big(1 << 12));
     return alloc_maps((uint32_t)cfg.grid_res);
@@ -614,7 +615,7 @@ struct vct_renderer {
 
   vct_status grow_big(uint32_t cap) {
     VCT_CHECK(big.ensure((size_t)cap * big_record_bytes()));
-    VCT_CHECK(big_offset.ensure((size_t)cap + 1));
+    VCT_CHECK(big_first.ensure(cap));
     big_cap = cap;
     return VCT_OK;
   }
@@ -751,8 +752,7 @@ struct vct_renderer {
     rb.big = big.p;
     rb.big_cap = big_cap;
     rb.big_count = big_count.p;
-    rb.big_offset = big_offset.p;
-    rb.scan_tmp = nullptr;
+    rb.big_first = big_first.p;
     rb.gb_pos = gb_pos.p;
     rb.gb_nrm = gb_nrm.p;
     rb.status = d_status.p;

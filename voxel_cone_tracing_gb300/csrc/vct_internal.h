@@ -234,9 +234,8 @@ struct RasterBuffers {
   unsigned long long* vis;  // W*H (depth bits << 32 | triangle id)
   void* big;                // raster work records
   uint32_t big_cap;
-  uint32_t* big_count;      // [0] records, [1] tiles
-  uint32_t* big_offset;     // tile prefix per record (big_cap + 1)
-  uint32_t* scan_tmp;
+  unsigned long long* big_count;  // records << 32 | tiles
+  uint32_t* big_first;      // a record's first tile (big_cap)
   float4* gb_pos;           // world position, material id bits in .w
   float4* gb_nrm;           // world normal, triangle id bits in .w
   FrameStatus* status;

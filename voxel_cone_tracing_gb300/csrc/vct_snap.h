@@ -53,4 +53,31 @@ VCT_SNAP_HD inline long long snap_fixed(float g, int k) {
   return (bits >> 31) ? base - q : base + q;
 }
 
+// round-half-even((g + 1) * K) as FP64 computes it -- the sum and the product
+// each rounded once -- for |g| <= 64 and 1 <= K <= 2^21 (K need not be a power
+// of two: 128 times a frame's width or height).  With g = m * 2^-s the exact
+// value is K + m K / 2^s, m K below 2^45; FP64's own rounding moves it by less
+// than 2^-24, so an integer shift rounds alike unless the fraction is that near
+// one half.  `close` reports such a value (and returns nothing of use): the
+// caller then rounds in FP64.
+VCT_SNAP_HD inline int snap_scaled(float g, uint32_t K, bool& close) {
+#ifdef __CUDA_ARCH__
+  const uint32_t bits = __float_as_uint(g);
+#else
+  uint32_t bits;
+  std::memcpy(&bits, &g, sizeof(bits));
+#endif
+  close = false;
+  const int exp = (int)((bits >> 23) & 0xffu);
+  if (exp < 127 - 31) return (int)K;  // |g K| < 2^-10
+  const long long m = (long long)((bits & 0x7fffffu) | 0x800000u) * K;
+  const long long p = (bits >> 31) ? -m : m;
+  const int s = 150 - exp;  // in [17, 54]
+  const long long half = 1LL << (s - 1);
+  const long long off = (p & ((1LL << s) - 1)) - half;  // the fraction's distance from one half
+  const long long band = s > 24 ? 1LL << (s - 24) : 0;
+  close = off <= band && off >= -band;
+  return (int)K + (int)((p + half) >> s);
+}
+
 }  // namespace vct
