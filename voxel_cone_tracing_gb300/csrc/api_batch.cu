@@ -73,10 +73,11 @@ struct vct_batch {
   std::vector<size_t> px_base;
   size_t total_px = 0;
   // batch-wide work arrays
-  DevBuf<uint32_t> brick_count, brick_offset, brick_cursor, pair_list, scan_tmp, bin_big_count, queue;
+  DevBuf<uint32_t> brick_count, brick_offset, brick_cursor, brick_units, pair_list, scan_tmp, bin_big_count, queue;
   DevBuf<uint8_t> brick_dirty;  // BatchBuffers::dirty
   DevBuf<BinRec> bin_big;
   DevBuf<uint2> bin_rec;  // per padded batch triangle (counting -> filling pass)
+  DevBuf<TriRec> tri_rec;  // per padded batch triangle (counting pass -> bricks)
   uint32_t bin_big_cap = 0;
   HeavyStore heavy;
   DevBuf<unsigned char> rbig;
@@ -142,8 +143,11 @@ struct vct_batch {
     bb.rb.gb_nrm = gb_nrm.p;
     bb.rb.status = d_status.p;
     bb.frame = frame.p;
+    bb.units = brick_units.p;
     bb.heavy = kHeavySplit ? heavy.view() : HeavyBricks{};
     bb.bin_rec = bin_rec.p;
+    bb.tri_rec = tri_rec.p;
+    bb.tri_prefix = work(tris).prefix;
     bb.dirty = brick_dirty.p;
     bb.mips = fused ? d_mips.p : nullptr;
     return bb;
@@ -199,9 +203,7 @@ struct vct_batch {
                              stream));
     VCT_CUDA(cudaMemsetAsync(d_status.p, 0, sizeof(FrameStatus), stream));
     VCT_CUDA(record(0));
-    BatchWork wb = work(bricks);
-    wb.queue = queue.p + 1;  // the brick queue (queue[0] schedules the trace)
-    VCT_CUDA(launch_voxelize_batch(work(tris), wb, bricks.total(), cfg.vox_mode, VCT_STORAGE_RGBA8, bb,
+    VCT_CUDA(launch_voxelize_batch(work(tris), work(bricks), bricks.total(), cfg.vox_mode, VCT_STORAGE_RGBA8, bb,
                                    scan_tmp.p, shape, sms, stream, &launches));
     VCT_CUDA(record(1));
     if (fused) {
@@ -500,17 +502,19 @@ vct_status build_batch(vct_batch* b, const vct_batch_scene* descs, uint32_t n) {
   VCT_CHECK(b->brick_count.ensure(nbk));
   VCT_CHECK(b->brick_offset.ensure(nbk + 1));
   VCT_CHECK(b->brick_cursor.ensure(nbk));
+  VCT_CHECK(b->brick_units.ensure(nbk + 4));
   VCT_CHECK(b->brick_dirty.ensure(nbk));
   VCT_CUDA(cudaMemsetAsync(b->brick_dirty.p, 1, nbk, b->stream));  // the new maps: every brick writes once
   VCT_CHECK(b->heavy.reserve(nbk, 1024, 65536, b->stream));
   VCT_CHECK(b->scan_tmp.ensure(scan_tmp_words(nbk)));
   VCT_CHECK(b->pair_list.ensure((size_t)std::min<uint64_t>(0xffffff00ull, 4ull * total_tris + 65536ull)));
   VCT_CHECK(b->bin_rec.ensure(std::max<size_t>(b->tris.total(), 1)));
+  VCT_CHECK(b->tri_rec.ensure(std::max<size_t>(b->tris.total(), 1)));
   VCT_CHECK(b->bin_big_count.ensure(1));
   VCT_CHECK(b->grow_bin_big(1 << 12));
   VCT_CHECK(b->rbig_count.ensure(1));
   VCT_CHECK(b->grow_rbig(1 << 16));
-  VCT_CHECK(b->queue.ensure(2));
+  VCT_CHECK(b->queue.ensure(1));
   VCT_CHECK(b->vis.ensure(px));
   VCT_CHECK(b->gb_pos.ensure(px));
   VCT_CHECK(b->gb_nrm.ensure(px));

@@ -10,7 +10,8 @@
 // point allocates nothing.  The caller passes its inputs (meshes, materials,
 // lights) and its output buffer; every intermediate the voxelizer needs (the
 // per-brick triangle counts, offsets and cursors, the triangle-brick pair
-// list, the instance records and the status word) lives in one file-scope
+// list, the large triangles' records, the split bricks' sums, the instance
+// records and the status word) lives in one file-scope
 // device array below, which exists once per GPU for as long as the library
 // is loaded.
 //
@@ -45,7 +46,11 @@ constexpr int kNaMaxBricks = (kNaMaxGrid / kBrick) * (kNaMaxGrid / kBrick) * (kN
 constexpr uint32_t kNaMaxPairs = 1u << 21;
 constexpr uint32_t kNaMaxMeshes = 64;
 constexpr uint32_t kNaMaxMaterials = 4096;
+constexpr uint32_t kNaBig = 4096;      // large-triangle records; further ones are binned by their warps
+constexpr uint32_t kNaSlots = 256, kNaItems = 4096;  // split bricks and their extra chunks; further ones run whole
 constexpr int kNaScanTmp = kNaMaxBricks / 4096 + 8;
+
+constexpr size_t kNaSlotBytes = 5 * sizeof(uint32_t) * kBrick * kBrick * kBrick;  // four channels and a count
 
 struct NoAllocScratch {
   uint32_t brick_count[kNaMaxBricks];
@@ -56,6 +61,16 @@ struct NoAllocScratch {
   uint32_t material_of_id[kNaMaxMaterials];  // identity: triangle material id -> material
   DevInstance inst[kNaMaxMeshes];
   FrameStatus status;
+  uint32_t units[kNaMaxBricks + 4];
+  BinRec big[kNaBig];
+  uint32_t big_count;
+  uint2 bin_rec[kNaMaxPairs];  // (a call has at most that many triangles)
+  int32_t heavy_slot[kNaMaxBricks];
+  uint32_t heavy_brick[kNaSlots];
+  uint2 heavy_items[kNaItems];
+  uint32_t heavy_counters[2];
+  alignas(16) uint32_t heavy_done[kNaSlots];  // cleared with the sums by each call
+  alignas(16) unsigned char heavy_acc[kNaSlots * kNaSlotBytes];
 };
 
 static __device__ __align__(256) unsigned char g_scratch[sizeof(NoAllocScratch)];
@@ -175,6 +190,15 @@ extern "C" vct_status vct_voxelize_noalloc(const vct_device_mesh* meshes, uint32
   vb.scan_tmp = s->scan_tmp;
   vb.counts = nullptr;
   vb.status = &s->status;
+  vb.units = s->units;
+  vb.big = s->big;
+  vb.big_cap = kNaBig;
+  vb.big_count = &s->big_count;
+  vb.bin_rec = s->bin_rec;
+  if (heavy_slot_bytes(VCT_STORAGE_RGBA8) > kNaSlotBytes) return set_error(VCT_ERR_CUDA, "voxelizer scratch too small");
+  vb.heavy = {s->heavy_slot, s->heavy_brick, s->heavy_done, s->heavy_acc, s->heavy_items, s->heavy_counters, kNaSlots,
+              kNaItems};
+  VCT_CUDA(cudaMemsetAsync(s->heavy_done, 0, sizeof(s->heavy_done) + sizeof(s->heavy_acc), st));
   VCT_CUDA(launch_voxelize_linear(sp, grid_res, vox_mode, vb, static_cast<uchar4*>(level0_rgba8), st));
 
   FrameStatus hs;

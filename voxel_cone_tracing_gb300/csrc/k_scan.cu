@@ -77,20 +77,36 @@ __global__ void __launch_bounds__(kT) k_scan_top(uint32_t* __restrict__ tile_tot
     *out_total = carry;
     if (fuse.total_copy) *fuse.total_copy = carry;
   }
-  if (fuse.hb.slot && threadIdx.x < 3) fuse.hb.counters[threadIdx.x] = 0u;  // the plan's counters, before k_scan_add
+  // the counters of the plan and of the list, before k_scan_add
+  if (fuse.hb.slot && threadIdx.x < 2) fuse.hb.counters[threadIdx.x] = 0u;
+  if (fuse.units.list && threadIdx.x < 3) fuse.units.count[threadIdx.x] = 0u;
 }
 
 __global__ void __launch_bounds__(256) k_scan_add(const uint32_t* __restrict__ in, uint32_t* __restrict__ out,
                                                   uint32_t* __restrict__ copy_out,
                                                   const uint32_t* __restrict__ tile_tot, size_t n, ScanFuse fuse) {
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const uint32_t v = out[i] + tile_tot[i / kTile];
-  out[i] = v;
-  if (copy_out) copy_out[i] = v;
-  if (fuse.hb.slot) {
-    const uint32_t c = fuse.cap;
-    heavy_plan_brick((uint32_t)i, min(v, c), min(v + in[i], c), min(out[n], c), fuse.slots, fuse.hb);
+  const uint32_t c = fuse.cap;
+  uint32_t pairs = 0;
+  if (i < n) {
+    const uint32_t v = out[i] + tile_tot[i / kTile];
+    out[i] = v;
+    if (copy_out) copy_out[i] = v;
+    if (fuse.hb.slot) heavy_plan_brick((uint32_t)i, min(v, c), min(v + in[i], c), min(out[n], c), fuse.slots, fuse.hb);
+    pairs = min(v + in[i], c) - min(v, c);
+  }
+  if (!fuse.units.list) return;
+  const BrickUnits& u = fuse.units;
+  const int kind = i >= n ? 2 : pairs > kLongBrick ? 0 : pairs || !u.dirty || u.dirty[i] ? 1 : 2;
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const unsigned m = __ballot_sync(0xffffffffu, kind == k);
+    if (!m) continue;
+    uint32_t at = 0;
+    if (lane == 0) at = atomicAdd(&u.count[k], (uint32_t)__popc(m));
+    at = __shfl_sync(0xffffffffu, at, 0) + (uint32_t)__popc(m & ((1u << lane) - 1u));
+    if (kind == k) u.list[k ? u.cap - 1u - at : at] = (uint32_t)i;
   }
 }
 
@@ -107,7 +123,8 @@ cudaError_t launch_exclusive_scan(const uint32_t* in, uint32_t* out, uint32_t* c
     // No bricks: nothing to plan (the counters still start at zero).
     cudaError_t e = cudaMemsetAsync(out, 0, sizeof(uint32_t), st);
     if (e == cudaSuccess && f.total_copy) e = cudaMemsetAsync(f.total_copy, 0, sizeof(uint32_t), st);
-    if (e == cudaSuccess && f.hb.slot) e = cudaMemsetAsync(f.hb.counters, 0, 3 * sizeof(uint32_t), st);
+    if (e == cudaSuccess && f.hb.slot) e = cudaMemsetAsync(f.hb.counters, 0, 2 * sizeof(uint32_t), st);
+    if (e == cudaSuccess && f.units.list) e = cudaMemsetAsync(f.units.count, 0, 3 * sizeof(uint32_t), st);
     return e;
   }
   const size_t ntiles = (n + kTile - 1) / kTile;

@@ -6,13 +6,13 @@
 //      (margin-expanded) box test says it may touch; per-brick counts.
 //   2. exclusive scan of the counts -> per-brick list offsets.
 //   3. k_bin<true>: scatter triangle ids into the per-brick lists.
-//   4. k_bricks: one CTA per brick.  Warps take 32 triangles at a time, set
-//      them up in shared memory, expand (triangle, sample|voxel) work items
-//      across lanes, decide coverage with the exact rule of the selected mode,
-//      shade in FP32 (voxelize.frag:124-153) and add fixed-point colour sums
-//      and counts into shared-memory accumulators.  The CTA then writes its
-//      whole brick of level 0 (empty voxels = 0, which is the clear) as RGBA8
-//      or RGBA16F through a surface -- level 0 is written exactly once.
+//   4. k_bricks: resident CTAs take the bricks that have pairs (and the empty
+//      ones that must be cleared) from a list the scan makes.  A CTA sets up
+//      128 pairs in shared memory, decides coverage with the exact rule of the
+//      selected mode, shades what is covered in FP32 (voxelize.frag:124-153),
+//      adds fixed-point colour sums and counts into shared-memory
+//      accumulators, and writes its whole brick of level 0 as RGBA8 or RGBA16F
+//      through a surface -- level 0 is written exactly once.
 //
 // Coverage rules (the CPU oracle implements the same ones):
 //   REF_RASTER2X -- the reference's method: dominant-axis projection
@@ -22,8 +22,8 @@
 //     barycentric interpolation, voxel = int(N*(0.5*c+0.5)) (voxelize.frag
 //     :156-157, truncation).
 //   CONSERVATIVE -- exact separating-axis triangle/box test on vertices
-//     snapped to 1/256 voxel (int64, the plane test in int128), colour at
-//     the triangle point closest to the voxel centre.
+//     snapped to 1/256 voxel (vct_cover.h), colour at the triangle point
+//     closest to the voxel centre.
 #include <cuda_fp16.h>
 
 #include <algorithm>
@@ -31,6 +31,7 @@
 #include <climits>
 #include <type_traits>
 
+#include "vct_cover.h"
 #include "vct_internal.h"
 #include "vct_math.cuh"
 #include "vct_mip.cuh"
@@ -44,33 +45,21 @@ namespace {
 #endif
 constexpr int kThreads = VCT_BRICK_THREADS;  // threads of a brick CTA
 constexpr int kWarps = kThreads / 32;
-#ifndef VCT_BRICK_BALANCE
-#define VCT_BRICK_BALANCE 1
-#endif
-// 1: a brick CTA spreads each round's samples over all its threads (a scan
-// over the round's pairs); 0: each warp expands the samples of its own pairs.
-constexpr bool kBrickBalance = VCT_BRICK_BALANCE != 0;
 #ifndef VCT_BRICK_ROUND
 #define VCT_BRICK_ROUND 0
 #endif
-// Pairs per round of the balanced expansion (0: one per thread); their
-// triangle setups are the larger part of a brick CTA's shared memory.
+// Pairs per round of a brick CTA (0: one per thread); their triangle setups
+// are the larger part of its shared memory.
 constexpr int kRound = VCT_BRICK_ROUND > 0 ? VCT_BRICK_ROUND : kThreads;
 static_assert(kRound % 32 == 0 && kRound <= kThreads, "round of whole warps, at most one pair per thread");
-constexpr int kSetupSlots = kBrickBalance ? kRound : kThreads;
-constexpr int kExclSlots = kBrickBalance ? kRound : kWarps * 33;
-#ifndef VCT_BRICK_MIN_BLOCKS
-#define VCT_BRICK_MIN_BLOCKS 0
-#endif
-// Resident brick CTAs per SM the kernels are compiled for (0: the default
-// per coverage rule).  Both rules keep 7 per SM (30 KB of shared memory
-// each); the conservative rule's kernel is held to the 72 registers that 7
-// allow (unbounded it takes 98 and fits 5: 512^3 voxelize 1.47 -> 1.75 ms).
-// Measured with 64-pair rounds (20 KB) at 8-10 per SM: the 512^3 raster
-// rule gains 5%, the bench frame and the batch lose 4-8%.
-template <int MODE>
+// Resident brick CTAs per SM the kernels are compiled for: 7 (72 registers,
+// 26 to 28 KB of shared memory each with RGBA8), 5 where the attribute sums
+// take 40 KB.  96-pair rounds at 8 per SM (64 registers) and 96-thread CTAs at
+// 9 took the same or longer (512^3: 985 us of voxelization against 1006 and
+// 1112), 64-pair rounds longer still.
+template <int STORAGE>
 constexpr int brick_min_blocks() {
-  return VCT_BRICK_MIN_BLOCKS > 0 ? VCT_BRICK_MIN_BLOCKS : (MODE == VCT_VOX_CONSERVATIVE ? 7 : 1);
+  return STORAGE == kStorageAttr ? 5 : 7;
 }
 constexpr int kBrickVox = kBrick * kBrick * kBrick;
 constexpr float kBinMargin = 0.25f;   // voxels; >> snapping and FP32 error
@@ -114,6 +103,32 @@ __device__ __forceinline__ void load_tri(const SceneParams& sp, uint32_t t, TriL
     if (NORMALS) tl.n[k] = normalize(nm_mul(in.NM, a.w, b.x, b.y));
   }
   if (NORMALS) tl.mat = __ldg(sp.obj_material + min(__ldg(in.tri_obj + lt), sp.n_obj - 1u));
+}
+
+__device__ __forceinline__ void store_rec(TriRec& r, const TriLoad& tl) {
+  r.q[0] = make_float4(tl.g[0][0], tl.g[0][1], tl.g[0][2], tl.g[1][0]);
+  r.q[1] = make_float4(tl.g[1][1], tl.g[1][2], tl.g[2][0], tl.g[2][1]);
+  r.q[2] = make_float4(tl.g[2][2], tl.n[0].x, tl.n[0].y, tl.n[0].z);
+  r.q[3] = make_float4(tl.n[1].x, tl.n[1].y, tl.n[1].z, tl.n[2].x);
+  r.q[4] = make_float4(tl.n[2].y, tl.n[2].z, __uint_as_float(tl.mat), 0.0f);
+}
+__device__ __forceinline__ void load_rec(const TriRec& r, TriLoad& tl) {
+  const float4 a = r.q[0], b = r.q[1], c = r.q[2], d = r.q[3], e = r.q[4];
+  tl.g[0][0] = a.x; tl.g[0][1] = a.y; tl.g[0][2] = a.z;
+  tl.g[1][0] = a.w; tl.g[1][1] = b.x; tl.g[1][2] = b.y;
+  tl.g[2][0] = b.z; tl.g[2][1] = b.w; tl.g[2][2] = c.x;
+  tl.n[0] = v3(c.y, c.z, c.w);
+  tl.n[1] = v3(d.x, d.y, d.z);
+  tl.n[2] = v3(d.w, e.x, e.y);
+  tl.mat = __float_as_uint(e.z);
+  tl.ok = true;
+}
+// A listed triangle: from its record, or without records from the meshes.
+template <bool REC>
+__device__ __forceinline__ void fetch_tri(const SceneParams& sp, const TriRec* __restrict__ recs, uint32_t t,
+                                          TriLoad& tl) {
+  if constexpr (REC) load_rec(recs[t], tl);
+  else load_tri<true>(sp, t, tl);
 }
 
 // ------------------------------------------------ conservative brick test --
@@ -196,22 +211,23 @@ constexpr uint32_t kRecAgain = 1u << 31;
 // triangle when it has few candidate bricks.  A triangle with more
 // candidates (room walls span 1024 bricks at 256^3) is recorded by the
 // counting pass in `big` and binned by k_bin_big, which spreads each record
-// over several CTAs; without a record list (or when it is full) the warp
-// bins it, the lanes splitting the candidate range.
+// over several CTAs; when the record list is full the warp bins it, the lanes
+// splitting the candidate range.
 // All 32 lanes of a warp call it together (each with its own triangle t of
 // the same scene; t >= total_tris is an idle lane).
 template <bool FILL>
 __device__ __forceinline__ void bin_tri(const SceneParams& sp, int N, uint32_t t, uint32_t* __restrict__ count,
                                         uint32_t* __restrict__ cursor, uint32_t* __restrict__ list, uint32_t cap,
                                         FrameStatus* st, BinRec* __restrict__ big, uint32_t big_cap,
-                                        uint32_t* __restrict__ big_count, uint32_t scene, uint2* __restrict__ rec) {
+                                        uint32_t* __restrict__ big_count, uint32_t scene, uint2* __restrict__ rec,
+                                        TriRec* __restrict__ recs) {
   const int lane = threadIdx.x & 31;
   const int nb = N / kBrick;
   float v[3][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
   int blo[3] = {0, 0, 0}, bhi[3] = {-1, -1, -1};
   int vol = 0;
   bool again = true;  // (filling pass) this lane's triangle is binned from scratch
-  if (FILL && rec && t < sp.total_tris) {
+  if (FILL && t < sp.total_tris) {
     // Replay the counting pass's bricks (same pairs, no triangle reload).
     const uint2 r = rec[t];
     again = (r.y & kRecAgain) != 0u;
@@ -229,7 +245,12 @@ __device__ __forceinline__ void bin_tri(const SceneParams& sp, int N, uint32_t t
   }
   if (again && t < sp.total_tris) {
     TriLoad tl;
-    load_tri<false>(sp, t, tl);
+    if (!FILL && recs) {
+      load_tri<true>(sp, t, tl);
+      if (tl.ok) store_rec(recs[t], tl);
+    } else {
+      load_tri<false>(sp, t, tl);
+    }
     if (!tl.ok) {
       if (!FILL) atomicAdd(&st->rejected_tris, 1u);
     } else {
@@ -256,23 +277,20 @@ __device__ __forceinline__ void bin_tri(const SceneParams& sp, int N, uint32_t t
       for (int by = blo[1]; by <= bhi[1]; ++by)
         for (int bx = blo[0]; bx <= bhi[0]; ++bx, ++i)
           if (bin_one<FILL>(v, bx, by, bz, nb, vol > 1, t, count, cursor, list, cap)) mask |= 1u << i;
-    if (!FILL && rec)
+    if (!FILL)
       rec[t] = make_uint2((uint32_t)blo[0] | (uint32_t)blo[1] << 10 | (uint32_t)blo[2] << 20,
                           mask | (uint32_t)(bhi[0] - blo[0]) << 8 | (uint32_t)(bhi[1] - blo[1]) << 11 |
                               (uint32_t)(bhi[2] - blo[2]) << 14);
-  } else if (!FILL && rec && t < sp.total_tris) {
-    // no bricks, or a large triangle: binned by its record (k_bin_big) or by the warp
-    rec[t] = make_uint2(0u, vol > kSoloBricks && !big ? kRecAgain : 0u);
   }
   bool in_warp = vol > kSoloBricks;
-  if (in_warp && big) {
-    // Counting pass records it; the filling pass leaves it to k_bin_big.
-    // A full record list is reported (big_total > big_cap) and the frame is
-    // encoded again with a larger one.
-    in_warp = false;
-    if (!FILL) {
+  if (!FILL && t < sp.total_tris && (in_warp || vol <= 0)) {
+    // No bricks, or a large triangle: binned by its record (k_bin_big), or
+    // where the record list is full by the warp, in both passes.  (The caller
+    // is told, and may enlarge the list.)
+    if (in_warp) {
       const uint32_t slot = atomicAdd(big_count, 1u);
       if (slot < big_cap) {
+        in_warp = false;
         BinRec r;
         for (int k = 0; k < 3; ++k)
           for (int d = 0; d < 3; ++d) r.v[k][d] = v[k][d];
@@ -284,6 +302,7 @@ __device__ __forceinline__ void bin_tri(const SceneParams& sp, int N, uint32_t t
         big[slot] = r;
       }
     }
+    rec[t] = make_uint2(0u, in_warp ? kRecAgain : 0u);
   }
   unsigned warp_big = __ballot_sync(0xffffffffu, in_warp);
   while (warp_big) {
@@ -308,9 +327,9 @@ __global__ void __launch_bounds__(256) k_bin(SceneParams sp, int N, uint32_t* __
                                              uint32_t* __restrict__ cursor, uint32_t* __restrict__ list,
                                              uint32_t cap, FrameStatus* st, BinRec* __restrict__ big,
                                              uint32_t big_cap, uint32_t* __restrict__ big_count,
-                                             uint2* __restrict__ rec) {
+                                             uint2* __restrict__ rec, TriRec* __restrict__ recs) {
   bin_tri<FILL>(sp, N, blockIdx.x * blockDim.x + threadIdx.x, count, cursor, list, cap, st, big, big_cap, big_count,
-                0u, rec);
+                0u, rec, recs);
 }
 
 // Every scene's triangles in one persistent launch; scene triangle ranges
@@ -324,7 +343,7 @@ __global__ void __launch_bounds__(256) k_bin_batch(BatchWork w, BatchBuffers bb)
     bin_tri<FILL>(S.sp, S.N, t, FILL ? nullptr : bb.brick_count + S.brick_base,
                   FILL ? bb.brick_cursor + S.brick_base : nullptr, bb.pair_list, bb.pair_cap, bb.status, bb.big,
                   bb.big_cap, bb.big_count, (uint32_t)s,
-                  bb.bin_rec ? bb.bin_rec + (g - t) : nullptr);
+                  bb.bin_rec + (g - t), bb.tri_rec + (g - t));
   }
 }
 
@@ -400,6 +419,14 @@ __device__ __forceinline__ T take_cg(T& g) {
   g = 0;
   return v;
 }
+// v added to a 64-bit sum in shared memory, as two 32-bit atomics and a carry:
+// 985 us of voxelization at 512^3, 1050 with 64-bit atomics.
+__device__ __forceinline__ void add64(unsigned long long* sum, unsigned long long v) {
+  uint32_t* w = reinterpret_cast<uint32_t*>(sum);
+  const uint32_t lo = (uint32_t)v, old = atomicAdd(w, lo);
+  const uint32_t hi = (uint32_t)(v >> 32) + (old + lo < old ? 1u : 0u);
+  if (hi) atomicAdd(w + 1, hi);
+}
 // atomic_add_to: voxel i of these sums added into a global copy (the
 // accumulator slot of a split brick); take_from: voxel i of the global copy
 // read from L2 into these sums and zeroed there.
@@ -443,10 +470,10 @@ template <> struct AccT<VCT_STORAGE_RGBA16F> {
   __device__ __forceinline__ void add(const SceneParams& sp, int v, const vct_material_data& m, V3 p, V3 nrm) {
     const float4 col = voxel_color(sp, m, p, nrm);
     const float k = 4294967296.0f / sp.radiance_max;
-    atomicAdd(&c[0][v], __float2ull_rn(col.x * k));
-    atomicAdd(&c[1][v], __float2ull_rn(col.y * k));
-    atomicAdd(&c[2][v], __float2ull_rn(col.z * k));
-    atomicAdd(&c[3][v], __float2ull_rn(col.w * 4294967296.0f));
+    add64(&c[0][v], __float2ull_rn(col.x * k));
+    add64(&c[1][v], __float2ull_rn(col.y * k));
+    add64(&c[2][v], __float2ull_rn(col.z * k));
+    add64(&c[3][v], __float2ull_rn(col.w * 4294967296.0f));
     atomicAdd(&n[v], 1u);
   }
 };
@@ -497,30 +524,31 @@ template <> struct AccT<kStorageAttr> {
 };
 
 // Mean of n 16-bit fixed-point contributions summing to c, as unorm8
-// rounded to nearest (ties up).
+// rounded to nearest (ties up): floor((510 c + 65535 n) / (2 n 65535)), both
+// sides over 255; in 32 bits while n 65535 * 2 + 257 n fits.
 __device__ __forceinline__ unsigned char unorm8_mean(uint32_t c, uint32_t n) {
-  const unsigned long long v = ((unsigned long long)c * 510ull + (unsigned long long)n * 65535ull) /
-                               (2ull * n * 65535ull);
+  if (n <= 32700u && c <= n * 65535u) return (unsigned char)((2u * c + 257u * n) / (514u * n));
+  const unsigned long long v = (2ull * c + 257ull * n) / (514ull * n);
   return (unsigned char)(v > 255ull ? 255ull : v);
 }
 typedef AccT<VCT_STORAGE_RGBA8> Acc;
 
 // -------------------------------------------------- reference raster mode --
 struct SetupRef {
-  long long area;
   int A[3], B[3];
   float c[3];
   float farea;
   V3 gp[3], gn[3];
   uint32_t mat;
-  int axis, tl;
-  int i0, ni, j0, nj;
+  int e[3];         // the edges at the window's first sample (row_edge)
+  uint32_t window;  // first sample in the brick's columns (4 + 4 bits), samples a row - 1 (4), axis (2), fill rule (3)
 };
 
-// Returns the number of samples of this triangle inside the brick's columns.
-__device__ int setup_ref(const SceneParams& sp, int N, uint32_t t, const int b3[3], SetupRef& s) {
+// Returns the number of sample rows of this triangle inside the brick's columns.
+template <bool REC>
+__device__ int setup_ref(const SceneParams& sp, const TriRec* __restrict__ recs, int N, uint32_t t, const int b3[3], SetupRef& s) {
   TriLoad tl;
-  load_tri<true>(sp, t, tl);
+  fetch_tri<REC>(sp, recs, t, tl);
   if (!tl.ok) return 0;
   // Dominant axis, voxelize.geom:27-51 (FP32, fixed order).
   float e1[3], e2[3];
@@ -563,7 +591,6 @@ __device__ int setup_ref(const SceneParams& sp, int N, uint32_t t, const int b3[
   const long long j0 = max((long long)sb0, ceil_div(minB - 128, 256));
   const long long j1 = min((long long)sb0 + 2 * kBrick - 1, floor_div(maxB - 128, 256));
   if (i1 < i0 || j1 < j0) return 0;
-  s.area = area;
   s.farea = __ll2float_rn(area);
   for (int k = 0; k < 3; ++k) {
     s.A[k] = (int)A[k];
@@ -573,26 +600,41 @@ __device__ int setup_ref(const SceneParams& sp, int N, uint32_t t, const int b3[
     s.gp[k] = v3(tl.g[o][0], tl.g[o][1], tl.g[o][2]);
     s.gn[k] = tl.n[o];
   }
-  s.tl = (top_left(A[1], B[1], A[2], B[2]) ? 1 : 0) | (top_left(A[2], B[2], A[0], B[0]) ? 2 : 0) |
-         (top_left(A[0], B[0], A[1], B[1]) ? 4 : 0);
+  for (int k = 0; k < 3; ++k) {
+    const int a = (k + 1) % 3, b = (k + 2) % 3;
+    s.e[k] = row_edge(A[a], B[a], A[b], B[b], top_left(A[a], B[a], A[b], B[b]), (int)i0, (int)j0);
+  }
   s.mat = tl.mat;
-  s.axis = axis;
-  s.i0 = (int)i0; s.ni = (int)(i1 - i0 + 1);
-  s.j0 = (int)j0; s.nj = (int)(j1 - j0 + 1);
-  return s.ni * s.nj;
+  s.window = (uint32_t)(i0 - sa0) | (uint32_t)(j0 - sb0) << 4 | (uint32_t)(i1 - i0) << 8 | (uint32_t)axis << 12;
+  return (int)(j1 - j0 + 1);
 }
 
+// The covered samples of row `row` of the setup's window, as bits; `code` +
+// their index: the sample in the brick's columns, i in the low 4 bits.
+__device__ __forceinline__ uint32_t cover(const SetupRef& s, int row, uint32_t& code) {
+  const uint32_t w = s.window;
+  code = (w & 15u) | ((w >> 4 & 15u) + (uint32_t)row) << 4;
+  int e[3], ey[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const int a = (k + 1) % 3, b = (k + 2) % 3;
+    e[k] = s.e[k] + (s.A[b] - s.A[a]) * row;
+    ey[k] = s.B[b] - s.B[a];
+  }
+  return row_mask(e[0], e[1], e[2], ey[0], ey[1], ey[2], (int)(w >> 8 & 15u) + 1);
+}
+
+// One covered sample.
 template <class A>
-__device__ __forceinline__ void item_ref(const SceneParams& sp, int N, const int b3[3], const SetupRef& s, int local,
-                                         A& acc) {
-  const int i = s.i0 + local % s.ni, j = s.j0 + local / s.ni;
+__device__ __forceinline__ void hit(const SceneParams& sp, int N, const int b3[3], const SetupRef& s, uint32_t code,
+                                    A& acc) {
+  const int axis = (int)(s.window >> 12 & 3u);
+  const int i = 2 * kBrick * (axis == 0 ? b3[1] : b3[0]) + (int)(code & 15u);
+  const int j = 2 * kBrick * (axis == 2 ? b3[1] : b3[2]) + (int)(code >> 4 & 15u);
   const long long sx = 256LL * i + 128, sy = 256LL * j + 128;
   const long long w0 = edge_fn(s.A[1], s.B[1], s.A[2], s.B[2], sx, sy);
   const long long w1 = edge_fn(s.A[2], s.B[2], s.A[0], s.B[0], sx, sy);
   const long long w2 = edge_fn(s.A[0], s.B[0], s.A[1], s.B[1], sx, sy);
-  if (!(w0 > 0 || (w0 == 0 && (s.tl & 1)))) return;
-  if (!(w1 > 0 || (w1 == 0 && (s.tl & 2)))) return;
-  if (!(w2 > 0 || (w2 == 0 && (s.tl & 4)))) return;
   const float b1 = rdiv(__ll2float_rn(w1), s.farea), b2 = rdiv(__ll2float_rn(w2), s.farea);
   float cz = radd(s.c[0], rmul(b1, rsub(s.c[1], s.c[0])));
   cz = radd(cz, rmul(b2, rsub(s.c[2], s.c[0])));
@@ -601,8 +643,8 @@ __device__ __forceinline__ void item_ref(const SceneParams& sp, int N, const int
   if (!(t > -1.0f && t < Nf)) return;
   const int kd = __float2int_rz(t);
   int vx, vy, vz;
-  if (s.axis == 2) { vx = i >> 1; vy = j >> 1; vz = kd; }
-  else if (s.axis == 0) { vx = kd; vy = i >> 1; vz = j >> 1; }
+  if (axis == 2) { vx = i >> 1; vy = j >> 1; vz = kd; }
+  else if (axis == 0) { vx = kd; vy = i >> 1; vz = j >> 1; }
   else { vx = i >> 1; vy = kd; vz = j >> 1; }
   const int lx = vx - b3[0] * kBrick, ly = vy - b3[1] * kBrick, lz = vz - b3[2] * kBrick;
   if ((unsigned)lx >= (unsigned)kBrick || (unsigned)ly >= (unsigned)kBrick || (unsigned)lz >= (unsigned)kBrick) return;
@@ -614,30 +656,38 @@ __device__ __forceinline__ void item_ref(const SceneParams& sp, int N, const int
 
 // ---------------------------------------------------- conservative mode ----
 struct SetupSat {
-  int V[3][3];
+  int V[3][3];  // relative to the brick
   V3 gp[3], gn[3];
   uint32_t mat;
-  int x0, nx, y0, ny, z0, nz;
+  // The triangle's box in the brick: first voxel (3 x 3 bits), voxels - 1
+  // across x (3) and down z (3), ceil(512 / voxels across x) (10), the form
+  // of the test (2).
+  uint32_t box;
 };
 
-__device__ int setup_sat(const SceneParams& sp, int N, uint32_t t, const int b3[3], SetupSat& s) {
+// Returns the number of columns (along z) of the triangle's box in the brick.
+template <bool REC>
+__device__ int setup_sat(const SceneParams& sp, const TriRec* __restrict__ recs, int N, uint32_t t, const int b3[3], SetupSat& s) {
   TriLoad tl;
-  load_tri<true>(sp, t, tl);
+  fetch_tri<REC>(sp, recs, t, tl);
   if (!tl.ok) return 0;
   // Vertices snapped to 1/256 voxel: round((g + 1) * N * 128), exactly, in
   // integer arithmetic (N is a power of two; vct_snap.h).
   const int shift = __ffs(N) - 1 + 7;
   int lo[3], hi[3];
+  long long extent = 0;
   for (int d = 0; d < 3; ++d) {
-    long long mn = LLONG_MAX, mx = LLONG_MIN;
+    const int origin = b3[d] * kBrick * 256;
+    int mn = INT_MAX, mx = INT_MIN;
     for (int k = 0; k < 3; ++k) {
-      long long q = snap_fixed(tl.g[k][d], shift);
-      s.V[k][d] = (int)q;
+      const int q = (int)snap_fixed(tl.g[k][d], shift) - origin;
+      s.V[k][d] = q;
       mn = min(mn, q);
       mx = max(mx, q);
     }
-    lo[d] = (int)max((long long)b3[d] * kBrick, ceil_div(mn, 256) - 1);
-    hi[d] = (int)min((long long)b3[d] * kBrick + kBrick - 1, floor_div(mx, 256));
+    extent = max(extent, (long long)mx - mn);
+    lo[d] = max(0, ((mn + 255) >> 8) - 1);
+    hi[d] = min(kBrick - 1, mx >> 8);
     if (hi[d] < lo[d]) return 0;
   }
   for (int k = 0; k < 3; ++k) {
@@ -645,51 +695,33 @@ __device__ int setup_sat(const SceneParams& sp, int N, uint32_t t, const int b3[
     s.gn[k] = tl.n[k];
   }
   s.mat = tl.mat;
-  s.x0 = lo[0]; s.nx = hi[0] - lo[0] + 1;
-  s.y0 = lo[1]; s.ny = hi[1] - lo[1] + 1;
-  s.z0 = lo[2]; s.nz = hi[2] - lo[2] + 1;
-  return s.nx * s.ny * s.nz;
+  const uint32_t nx = (uint32_t)(hi[0] - lo[0] + 1), form = extent <= kSatInt ? 0u : extent <= kSatLong ? 1u : 2u;
+  s.box = (uint32_t)lo[0] | (uint32_t)lo[1] << 3 | (uint32_t)lo[2] << 6 | (nx - 1) << 9 |
+          (uint32_t)(hi[2] - lo[2]) << 12 | ((511u + nx) / nx) << 15 | form << 25;
+  return (int)nx * (hi[1] - lo[1] + 1);
 }
 
-__device__ __forceinline__ bool axis_sep(long long p0, long long p1, long long p2, long long r) {
-  return min(p0, min(p1, p2)) > r || max(p0, max(p1, p2)) < -r;
+// The column test's forms for triangles that are large beside a brick, called
+// so that the kernel's body holds the 32-bit form alone.
+__device__ __noinline__ uint32_t cover_large(const SetupSat& s, bool wide, int x, int y, int z0, int nz) {
+  if (wide) return sat_column<long long>(s.V, x, y, z0, nz);
+  uint32_t mask = 0;
+#pragma unroll 1
+  for (int k = 0; k < nz; ++k) mask |= (sat_exact(s.V, x, y, z0 + k) ? 1u : 0u) << k;
+  return mask;
 }
 
-// Exact closed-box SAT on integer coordinates (1/256 voxel units).
-__device__ bool sat_exact(const int V[3][3], long long cx, long long cy, long long cz, long long h) {
-  long long u[3][3];
-  const long long c[3] = {cx, cy, cz};
-  for (int k = 0; k < 3; ++k)
-    for (int d = 0; d < 3; ++d) u[k][d] = (long long)V[k][d] - c[d];
-  for (int d = 0; d < 3; ++d) {
-    long long mn = min(u[0][d], min(u[1][d], u[2][d])), mx = max(u[0][d], max(u[1][d], u[2][d]));
-    if (mn > h || mx < -h) return false;
-  }
-  long long f[3][3];
-  for (int d = 0; d < 3; ++d) {
-    f[0][d] = u[1][d] - u[0][d];
-    f[1][d] = u[2][d] - u[1][d];
-    f[2][d] = u[0][d] - u[2][d];
-  }
-  const long long n0 = f[0][1] * f[1][2] - f[0][2] * f[1][1];
-  const long long n1 = f[0][2] * f[1][0] - f[0][0] * f[1][2];
-  const long long n2 = f[0][0] * f[1][1] - f[0][1] * f[1][0];
-  const __int128 dd = (__int128)n0 * u[0][0] + (__int128)n1 * u[0][1] + (__int128)n2 * u[0][2];
-  const __int128 rr = (__int128)h * ((__int128)llabs(n0) + (__int128)llabs(n1) + (__int128)llabs(n2));
-  if (dd > rr || dd < -rr) return false;
-  for (int e = 0; e < 3; ++e) {
-    const long long fx = f[e][0], fy = f[e][1], fz = f[e][2];
-    if (axis_sep(-fz * u[0][1] + fy * u[0][2], -fz * u[1][1] + fy * u[1][2], -fz * u[2][1] + fy * u[2][2],
-                 h * (llabs(fz) + llabs(fy))))
-      return false;
-    if (axis_sep(fz * u[0][0] - fx * u[0][2], fz * u[1][0] - fx * u[1][2], fz * u[2][0] - fx * u[2][2],
-                 h * (llabs(fz) + llabs(fx))))
-      return false;
-    if (axis_sep(-fy * u[0][0] + fx * u[0][1], -fy * u[1][0] + fx * u[1][1], -fy * u[2][0] + fx * u[2][1],
-                 h * (llabs(fy) + llabs(fx))))
-      return false;
-  }
-  return true;
+// The touched voxels of column `col` of the setup's box, as bits; `code` +
+// their index: the voxel in the brick, z in the low 3 bits.
+__device__ __forceinline__ uint32_t cover(const SetupSat& s, int col, uint32_t& code) {
+  const uint32_t w = s.box;
+  const int nx = (int)(w >> 9 & 7u) + 1, nz = (int)(w >> 12 & 7u) + 1;
+  const int row = (int)((uint32_t)col * (w >> 15 & 1023u) >> 9);  // col / nx: col < 64, so exact
+  const int x = (int)(w & 7u) + col - row * nx, y = (int)(w >> 3 & 7u) + row, z0 = (int)(w >> 6 & 7u);
+  code = (uint32_t)(z0 | y << 3 | x << 6);
+  const uint32_t form = w >> 25;
+  if (form == 0u) return sat_column<int>(s.V, x, y, z0, nz);
+  return cover_large(s, form == 1u, x, y, z0, nz);
 }
 
 // Barycentric weights of the closest triangle point to p (Voronoi-region
@@ -725,20 +757,18 @@ __device__ void closest_bary(V3 p, V3 a, V3 b, V3 c, float w[3]) {
   w[0] = 1.f - v - t; w[1] = v; w[2] = t;
 }
 
+// One touched voxel.
 template <class A>
-__device__ __forceinline__ void item_sat(const SceneParams& sp, int N, const int b3[3], const SetupSat& s, int local,
-                                         A& acc) {
-  const int x = s.x0 + local % s.nx;
-  const int y = s.y0 + (local / s.nx) % s.ny;
-  const int z = s.z0 + local / (s.nx * s.ny);
-  if (!sat_exact(s.V, 256LL * x + 128, 256LL * y + 128, 256LL * z + 128, 128)) return;
+__device__ __forceinline__ void hit(const SceneParams& sp, int N, const int b3[3], const SetupSat& s, uint32_t code,
+                                    A& acc) {
+  const int lx = (int)(code >> 6 & 7u), ly = (int)(code >> 3 & 7u), lz = (int)(code & 7u);
+  const int x = b3[0] * kBrick + lx, y = b3[1] * kBrick + ly, z = b3[2] * kBrick + lz;
   const float inv = 2.0f / (float)N;
   const V3 vc = v3(((float)x + 0.5f) * inv - 1.0f, ((float)y + 0.5f) * inv - 1.0f, ((float)z + 0.5f) * inv - 1.0f);
   float w[3];
   closest_bary(vc, s.gp[0], s.gp[1], s.gp[2], w);
   const V3 p = s.gp[0] * w[0] + s.gp[1] * w[1] + s.gp[2] * w[2];
   const V3 n = s.gn[0] * w[0] + s.gn[1] * w[1] + s.gn[2] * w[2];
-  const int lx = x - b3[0] * kBrick, ly = y - b3[1] * kBrick, lz = z - b3[2] * kBrick;
   acc.add(sp, (lz * kBrick + ly) * kBrick + lx, sp.materials[s.mat], p, n);
 }
 
@@ -746,101 +776,95 @@ __device__ __forceinline__ void item_sat(const SceneParams& sp, int N, const int
 template <int MODE>
 using SetupOf = typename std::conditional<MODE == VCT_VOX_CONSERVATIVE, SetupSat, SetupRef>::type;
 
+// Shared memory of a round of pairs.
+template <int MODE>
+struct RoundOf {
+  SetupOf<MODE> setup[kRound];
+  int first[kRound];           // a pair's first row (column) among the round's
+  uint16_t queue[kWarps][64];  // covered samples not yet shaded: pair << 9 | code
+  int sum[kWarps];
+};
+static_assert(kRound <= 128, "a queue entry holds the pair in 7 bits");
+
 // Accumulates the (triangle, brick) pairs list[beg, end) of the brick at b3
 // into acc (all threads of the CTA; cleared first, barrier at the end).
-template <int MODE, int STORAGE>
-__device__ __forceinline__ void brick_accumulate(const SceneParams& sp, int N, const int b3[3],
+// Rounds of up to kRound pairs: a setup per thread, a scan of the pairs' rows
+// (columns), then every warp tests rows in turn, a lane each, and queues what
+// is covered; it shades a full warp's worth from the queue at a time: of the
+// samples tested a third to a half are covered, and shading one costs ten
+// times the test.  (64-bit tests, each followed at once by its shading, and a
+// CTA per brick of the grid, 512^3 and two million triangles, conservative:
+// 1423 us, 256^3 and 500,000, raster: 215; now 737 and 150.  Half of that is
+// the pairs' loads and setup, a quarter shading.)
+template <int MODE, int STORAGE, bool REC>
+__device__ __forceinline__ void brick_accumulate(const SceneParams& sp, const TriRec* __restrict__ recs, int N, const int b3[3],
                                                  const uint32_t* __restrict__ list, uint32_t beg, uint32_t end,
-                                                 AccT<STORAGE>& acc, SetupOf<MODE> (&setup)[kSetupSlots],
-                                                 int (&excl)[kExclSlots]) {
+                                                 AccT<STORAGE>& acc, RoundOf<MODE>& rd) {
   for (int i = threadIdx.x; i < kBrickVox; i += kThreads) acc.clear(i);
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if constexpr (kBrickBalance) {
-    // Rounds of up to kRound pairs: one setup per thread, an exclusive
-    // scan of the pairs' sample counts, then every thread expands samples
-    // it, it + kThreads, ... of the round (a triangle covering the whole
-    // brick does not hold up one warp while the others wait).
-    __shared__ int s_wsum[kWarps];
-    SetupOf<MODE>* su = setup;
-    int* ex = excl;
-    for (uint32_t b0 = beg; b0 < end; b0 += kRound) {
-      const uint32_t n = min((uint32_t)kRound, end - b0);
-      int cnt = 0;
-      if ((uint32_t)threadIdx.x < n) {
-        if (MODE == VCT_VOX_CONSERVATIVE)
-          cnt = setup_sat(sp, N, __ldg(list + b0 + threadIdx.x), b3, reinterpret_cast<SetupSat&>(su[threadIdx.x]));
-        else
-          cnt = setup_ref(sp, N, __ldg(list + b0 + threadIdx.x), b3, reinterpret_cast<SetupRef&>(su[threadIdx.x]));
-      }
-      int incl = cnt;
-      for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += v;
-      }
-      if (lane == 31) s_wsum[warp] = incl;
-      __syncthreads();
-      int off = 0, total = 0;
-#pragma unroll
-      for (int w = 0; w < kWarps; ++w) {
-        const int v = s_wsum[w];
-        off += w < warp ? v : 0;
-        total += v;
-      }
-      if (threadIdx.x < kRound) ex[threadIdx.x] = off + incl - cnt;
-      __syncthreads();
-      for (int it = threadIdx.x; it < total; it += kThreads) {
-        int lo = 0, hi = (int)n - 1;  // owner = last pair with ex <= it
-        while (lo < hi) {
-          const int mid = (lo + hi + 1) >> 1;
-          if (ex[mid] <= it) lo = mid; else hi = mid - 1;
-        }
-        const int local = it - ex[lo];
-        if (MODE == VCT_VOX_CONSERVATIVE)
-          item_sat(sp, N, b3, reinterpret_cast<const SetupSat&>(su[lo]), local, acc);
-        else
-          item_ref(sp, N, b3, reinterpret_cast<const SetupRef&>(su[lo]), local, acc);
-      }
-      __syncthreads();  // the round's setups and offsets are free again
+  uint16_t* queue = rd.queue[warp];
+  for (uint32_t b0 = beg; b0 < end; b0 += kRound) {
+    const uint32_t n = min((uint32_t)kRound, end - b0);
+    int cnt = 0;
+    if ((uint32_t)threadIdx.x < n) {
+      const uint32_t t = __ldg(list + b0 + threadIdx.x);
+      if constexpr (MODE == VCT_VOX_CONSERVATIVE) cnt = setup_sat<REC>(sp, recs, N, t, b3, rd.setup[threadIdx.x]);
+      else cnt = setup_ref<REC>(sp, recs, N, t, b3, rd.setup[threadIdx.x]);
     }
-  } else {
-    // Rounds of up to kWarps * 32 pairs, split evenly between the warps (a
-    // brick with a few dozen pairs keeps every warp busy expanding samples).
-    for (uint32_t b0 = beg; b0 < end; b0 += kWarps * 32) {
-      const uint32_t n = min((uint32_t)(kWarps * 32), end - b0);
-      const uint32_t q = (n + kWarps - 1) / kWarps;
-      const uint32_t k = warp * q + lane;
-      const uint32_t e = b0 + k;
-      int cnt = 0;
-      if (lane < q && k < n) {
-        if (MODE == VCT_VOX_CONSERVATIVE)
-          cnt = setup_sat(sp, N, __ldg(list + e), b3, reinterpret_cast<SetupSat&>(setup[warp * 32 + lane]));
-        else
-          cnt = setup_ref(sp, N, __ldg(list + e), b3, reinterpret_cast<SetupRef&>(setup[warp * 32 + lane]));
-      }
-      int incl = cnt;
-      for (int o = 1; o < 32; o <<= 1) {
-        int v = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += v;
-      }
-      excl[warp * 33 + lane] = incl - cnt;
-      const int total = __shfl_sync(0xffffffffu, incl, 31);
-      __syncwarp();
-      for (int it = lane; it < total; it += 32) {
-        int lo = 0, hi = 31;  // owner = last lane with excl <= it
-        while (lo < hi) {
-          int mid = (lo + hi + 1) >> 1;
-          if (excl[warp * 33 + mid] <= it) lo = mid; else hi = mid - 1;
-        }
-        const int local = it - excl[warp * 33 + lo];
-        if (MODE == VCT_VOX_CONSERVATIVE)
-          item_sat(sp, N, b3, reinterpret_cast<const SetupSat&>(setup[warp * 32 + lo]), local, acc);
-        else
-          item_ref(sp, N, b3, reinterpret_cast<const SetupRef&>(setup[warp * 32 + lo]), local, acc);
-      }
-      __syncwarp();
+    int incl = cnt;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += v;
     }
+    if (lane == 31) rd.sum[warp] = incl;
     __syncthreads();
+    int off = 0, total = 0;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) {
+      const int v = rd.sum[w];
+      off += w < warp ? v : 0;
+      total += v;
+    }
+    if (threadIdx.x < kRound) rd.first[threadIdx.x] = off + incl - cnt;
+    __syncthreads();
+    int at = 0, queued = 0;
+    uint32_t mask = 0, code = 0;
+    for (;;) {
+      while (queued < 32) {
+        const unsigned some = __ballot_sync(0xffffffffu, mask != 0u);
+        if (some) {  // one covered sample of every lane that has any
+          if (mask) {
+            queue[queued + __popc(some & ((1u << lane) - 1u))] = (uint16_t)(code + (uint32_t)__ffs((int)mask) - 1u);
+            mask &= mask - 1u;
+          }
+          queued += __popc(some);
+          continue;
+        }
+        if (at >= total) break;
+        const int it = at + lane * kWarps + warp;  // (a few rows reach every warp)
+        at += kThreads;
+        if (it < total) {
+          int lo = 0, hi = (int)n - 1;  // owner = last pair with first <= it
+          while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (rd.first[mid] <= it) lo = mid; else hi = mid - 1;
+          }
+          mask = cover(rd.setup[lo], it - rd.first[lo], code);
+          code |= (uint32_t)lo << 9;
+        }
+      }
+      const int m = min(queued, 32);
+      if (m == 0) break;
+      __syncwarp();
+      queued -= m;
+      if (lane < m) {
+        const uint32_t q = queue[queued + lane];
+        hit(sp, N, b3, rd.setup[q >> 9], q & 511u, acc);
+      }
+      __syncwarp();  // the entries are read before their place is written again
+    }
+    __syncthreads();  // the round's setups and offsets are free again
   }
 }
 
@@ -992,7 +1016,8 @@ __device__ void brick_mips_zero(const BrickMips& bm, int N, const int b3[3]) {
 // Writes the brick at b3 from its sums: order-independent mean, round to
 // nearest (ties up); empty voxels = 0.  `acc` may be in shared or global
 // memory.
-template <int STORAGE>
+// SURF: level 0 through the surface (else into l0_lin alone).
+template <int STORAGE, bool SURF = true>
 __device__ __forceinline__ void brick_finalize(const SceneParams& sp, int N, const int b3[3], const AccT<STORAGE>& acc,
                                                cudaSurfaceObject_t l0, uint32_t* __restrict__ counts,
                                                FrameStatus* st, const InjGrids& inj, void* l0_lin,
@@ -1019,7 +1044,7 @@ __device__ __forceinline__ void brick_finalize(const SceneParams& sp, int N, con
       uchar4 o = make_uchar4(0, 0, 0, 0);
       if (n) o = make_uchar4(unorm8_mean(acc.c[0][i], n), unorm8_mean(acc.c[1][i], n), unorm8_mean(acc.c[2][i], n),
                              unorm8_mean(acc.c[3][i], n));
-      surf3Dwrite(o, l0, x * 4, y, z);
+      if constexpr (SURF) surf3Dwrite(o, l0, x * 4, y, z);
       if (l0_lin) static_cast<uchar4*>(l0_lin)[((size_t)z * N + y) * N + x] = o;
       if (bm) scr->l0[i] = (uint32_t)o.x | (uint32_t)o.y << 8 | (uint32_t)o.z << 16 | (uint32_t)o.w << 24;
     } else {
@@ -1055,22 +1080,21 @@ __device__ __forceinline__ void brick_coords(int N, uint32_t brick, int b3[3]) {
 // One unit of brick work, all threads of the CTA (the shared-memory arrays
 // come from the caller, so that a persistent CTA reuses them unit after
 // unit): the whole brick, or -- for a dense brick with an accumulator slot
-// (hb->slot[slot_index] >= 0) -- its chunk `chunk` of kHeavyChunk pairs.
+// (hb->slot[slot_index] >= 0) -- its chunk `chunk`.
 // A chunk adds its sums into the slot; the CTA that completes the brick's
 // last chunk takes the sums back (zeroing the slot and its counter for the
 // next frame) and writes the brick.  `item`: the unit is an extra chunk
 // (>= 1) of a split brick.  Every kernel calls this from one place only,
 // so that its code exists once per kernel (instruction-cache footprint).
-template <int MODE, int STORAGE>
-__device__ __forceinline__ void brick_unit(const SceneParams& sp, int N, uint32_t brick,
+template <int MODE, int STORAGE, bool SURF = true, bool REC = true>
+__device__ __forceinline__ void brick_unit(const SceneParams& sp, const TriRec* __restrict__ recs, int N, uint32_t brick,
                                            const uint32_t* __restrict__ offset, const uint32_t* __restrict__ list,
                                            uint32_t cap, cudaSurfaceObject_t l0, uint32_t* __restrict__ counts,
-                                           FrameStatus* st, AccT<STORAGE>& acc, SetupOf<MODE> (&setup)[kSetupSlots],
-                                           int (&excl)[kExclSlots], const InjGrids& inj, void* l0_lin,
+                                           FrameStatus* st, AccT<STORAGE>& acc, RoundOf<MODE>& rd, const InjGrids& inj, void* l0_lin,
                                            const HeavyBricks* hb, uint32_t slot_index, uint32_t chunk, bool item,
                                            const BrickMips* bm = nullptr, uint8_t* dirty = nullptr) {
-  static_assert(sizeof(BrickMipScratchT<VCT_STORAGE_RGBA16F>) <= sizeof(setup),
-                "fused mips fit in the triangle setups' memory");
+  static_assert(sizeof(BrickMipScratchT<VCT_STORAGE_RGBA16F>) <= sizeof(rd),
+                "fused mips fit in the round's memory");
   __shared__ uint32_t s_last;
   int b3[3];
   brick_coords(N, brick, b3);
@@ -1093,7 +1117,7 @@ __device__ __forceinline__ void brick_unit(const SceneParams& sp, int N, uint32_
         surf3Dwrite(make_uchar4(0, 0, 0, 0), inj.normal, x * 4, y, z);
         surf3Dwrite(make_uchar4(0, 0, 0, 0), inj.emission, x * 4, y, z);
       } else if (STORAGE == VCT_STORAGE_RGBA8) {
-        surf3Dwrite(make_uchar4(0, 0, 0, 0), l0, x * 4, y, z);
+        if constexpr (SURF) surf3Dwrite(make_uchar4(0, 0, 0, 0), l0, x * 4, y, z);
         if (l0_lin) static_cast<uchar4*>(l0_lin)[((size_t)z * N + y) * N + x] = make_uchar4(0, 0, 0, 0);
       } else {
         surf3Dwrite(make_ushort4(0, 0, 0, 0), l0, x * 8, y, z);
@@ -1109,17 +1133,18 @@ __device__ __forceinline__ void brick_unit(const SceneParams& sp, int N, uint32_
   const int slot = (hb && hb->slot && (item || end - beg0 > kHeavyChunk)) ? hb->slot[slot_index] : -1;
   uint32_t beg = beg0, stop = end;
   if (slot >= 0) {
-    beg = min(beg0 + chunk * kHeavyChunk, end);
-    stop = min(beg + kHeavyChunk, end);
+    const uint32_t span = heavy_span(end - beg0);
+    beg = min(beg0 + chunk * span, end);
+    stop = min(beg + span, end);
   }
-  brick_accumulate<MODE, STORAGE>(sp, N, b3, list, beg, stop, acc, setup, excl);
+  brick_accumulate<MODE, STORAGE, REC>(sp, recs, N, b3, list, beg, stop, acc, rd);
   if (slot >= 0) {
     AccT<STORAGE>& g = static_cast<AccT<STORAGE>*>(hb->acc)[slot];
     for (int i = threadIdx.x; i < kBrickVox; i += kThreads) acc.atomic_add_to(g, i);
     __threadfence();  // this CTA's sums are in L2 before its chunk counts as done
     __syncthreads();
     if (threadIdx.x == 0) {
-      const uint32_t nch = (end - beg0 + kHeavyChunk - 1) / kHeavyChunk;
+      const uint32_t nch = heavy_chunks(end - beg0);
       s_last = atomicAdd(&hb->done[slot], 1u) == nch - 1 ? 1u : 0u;
     }
     __syncthreads();
@@ -1129,90 +1154,75 @@ __device__ __forceinline__ void brick_unit(const SceneParams& sp, int N, uint32_
     if (threadIdx.x == 0) hb->done[slot] = 0;
     __syncthreads();
   }
-  // (the triangle setups are done with: their memory holds the fused mips)
+  // (the round is done with: its memory holds the fused mips)
   if (dirty && threadIdx.x == 0) dirty[brick] = 1;
-  brick_finalize<STORAGE>(sp, N, b3, acc, l0, counts, st, inj, l0_lin, bm, &setup[0]);
+  brick_finalize<STORAGE, SURF>(sp, N, b3, acc, l0, counts, st, inj, l0_lin, bm, &rd);
 }
 
-// One CTA per brick, after `n_extra` CTAs that run the extra chunks of
-// split bricks from the launch-wide item queue (first in the grid, so that
-// the dense bricks' chunks start with the first bricks, not in the tail).
-// (FUSE: the fused mips' level-1 reduction holds 32 unpacked children; the
-// kernel is held to the registers of 7 resident CTAs, as without it.)
+// The list of bricks with work in `words` (4 + bricks words).
+BrickUnits brick_units(uint32_t* words, uint32_t bricks, const uint8_t* dirty) {
+  BrickUnits u;
+  u.list = words + 4;
+  u.count = words;
+  u.cap = bricks;
+  u.dirty = dirty;
+  return u;
+}
+
+// Runs f(brick, chunk, extra) for the units this CTA takes: one by its index,
+// then from the counter, fetched while the unit before it runs.  The extra
+// chunks of the split bricks come first, so that they do not end the launch,
+// then the long bricks, then the others.  (A CTA per brick of the grid spent
+// 512^3 voxelization 280 us on the empty ones, seven in eight.)
+template <class F>
+__device__ __forceinline__ void for_units(const HeavyBricks& hb, const BrickUnits& u, FrameStatus* st, F&& f) {
+  __shared__ uint32_t s_next[2];
+  const uint32_t n_items = hb.slot ? min(hb.counters[1], hb.item_cap) : 0u, n_long = u.count[0];
+  const uint32_t total = n_items + n_long + u.count[1];
+  if (hb.slot && blockIdx.x == 0 && threadIdx.x < 2) (&st->heavy_total)[threadIdx.x] = hb.counters[threadIdx.x];
+  int turn = 0;
+  for (uint32_t q = blockIdx.x; q < total; turn ^= 1) {
+    if (threadIdx.x == 0) s_next[turn] = gridDim.x + atomicAdd(&u.count[2], 1u);
+    const uint32_t i = q - n_items;
+    const bool extra = q < n_items;
+    const uint2 w = extra ? hb.items[q] : make_uint2(u.list[i < n_long ? i : u.cap - 1u - (i - n_long)], 0u);
+    if (w.x != 0xffffffffu) f(w.x, w.y, extra);  // (an unused item: CTA-uniform)
+    __syncthreads();  // the unit is done with its shared memory
+    q = s_next[turn];
+  }
+}
+
+// (FUSE: with the fused mips.)
 template <int MODE, int STORAGE, bool FUSE = false>
-__global__ void __launch_bounds__(kThreads, FUSE ? 7 : brick_min_blocks<MODE>()) k_bricks(SceneParams sp, int N, const uint32_t* __restrict__ offset,
+__global__ void __launch_bounds__(kThreads, brick_min_blocks<STORAGE>()) k_bricks(SceneParams sp, int N, const uint32_t* __restrict__ offset,
                                                      const uint32_t* __restrict__ list, uint32_t cap,
                                                      cudaSurfaceObject_t l0, uint32_t* __restrict__ counts,
                                                      FrameStatus* st, InjGrids inj, void* l0_lin, HeavyBricks hb,
-                                                     uint32_t n_extra, const __grid_constant__ BrickMips bm) {
+                                                     BrickUnits units, const TriRec* __restrict__ recs,
+                                                     const __grid_constant__ BrickMips bm) {
   __shared__ AccT<STORAGE> acc;
-  __shared__ SetupOf<MODE> setup[kSetupSlots];
-  __shared__ int excl[kExclSlots];
-  __shared__ uint32_t s_next;
-  const bool extra = blockIdx.x < n_extra;
-  const uint32_t n_items = extra ? min(hb.counters[1], hb.item_cap) : 0u;
-  if (extra && blockIdx.x == 0 && threadIdx.x < 2) (&st->heavy_total)[threadIdx.x] = hb.counters[threadIdx.x];
-  for (bool first = true;; first = false) {
-    uint32_t brick, chunk = 0;
-    if (!extra) {
-      if (!first) return;
-      brick = blockIdx.x - n_extra;
-    } else {
-      if (threadIdx.x == 0) s_next = atomicAdd(&hb.counters[2], 1u);
-      __syncthreads();
-      const uint32_t it = s_next;
-      __syncthreads();  // s_next read by every thread before the next write
-      if (it >= n_items) return;
-      const uint2 w = hb.items[it];
-      if (w.x == 0xffffffffu) continue;  // CTA-uniform
-      brick = w.x;
-      chunk = w.y;
-    }
-    brick_unit<MODE, STORAGE>(sp, N, brick, offset, list, cap, l0, counts, st, acc, setup, excl, inj, l0_lin, &hb,
-                              brick, chunk, extra, FUSE ? &bm : nullptr, bm.dirty);
-    __syncthreads();  // done with acc
-  }
+  __shared__ __align__(8) RoundOf<MODE> rd;
+  for_units(hb, units, st, [&](uint32_t brick, uint32_t chunk, bool extra) {
+    brick_unit<MODE, STORAGE>(sp, recs, N, brick, offset, list, cap, l0, counts, st, acc, rd, inj, l0_lin, &hb, brick, chunk,
+                              extra, FUSE ? &bm : nullptr, bm.dirty);
+  });
 }
 
-// Every scene's bricks in one persistent launch; a CTA takes its next unit
-// from the atomic counter w.queue (brick costs range from an empty brick to
-// thousands of triangle samples).  The queue hands out the extra chunks of
-// the split bricks first (global brick indices), then the bricks.
+// Every scene's bricks in one launch.
 template <int MODE, int STORAGE, bool FUSE = false>
-__global__ void __launch_bounds__(kThreads, FUSE ? 7 : brick_min_blocks<MODE>())
-    k_bricks_batch(BatchWork w, BatchBuffers bb) {
+__global__ void __launch_bounds__(kThreads, brick_min_blocks<STORAGE>())
+    k_bricks_batch(BatchWork w, BatchBuffers bb, BrickUnits units) {
   __shared__ AccT<STORAGE> acc;
-  __shared__ SetupOf<MODE> setup[kSetupSlots];
-  __shared__ int excl[kExclSlots];
-  __shared__ uint32_t s_next;
+  __shared__ __align__(8) RoundOf<MODE> rd;
   const HeavyBricks& hb = bb.heavy;
-  const uint32_t n_items = hb.slot ? min(hb.counters[1], hb.item_cap) : 0u;
-  const uint32_t total = n_items + w.total;
-  if (hb.slot && blockIdx.x == 0 && threadIdx.x < 2) (&bb.status->heavy_total)[threadIdx.x] = hb.counters[threadIdx.x];
-  for (;;) {
-    if (threadIdx.x == 0) s_next = atomicAdd(w.queue, 1u);
-    __syncthreads();
-    const uint32_t q = s_next;
-    __syncthreads();  // s_next read by every thread before the next write
-    if (q >= total) return;
-    uint32_t g, chunk = 0;
-    const bool item = q < n_items;
-    if (item) {
-      const uint2 it = hb.items[q];
-      if (it.x == 0xffffffffu) continue;  // CTA-uniform
-      g = it.x;
-      chunk = it.y;
-    } else {
-      g = q - n_items;
-    }
+  for_units(hb, units, bb.status, [&](uint32_t g, uint32_t chunk, bool extra) {
     const int s = batch_scene_of(w, g);
     const BatchScene& S = w.scenes[s];
-    brick_unit<MODE, STORAGE>(S.sp, S.N, g - __ldg(w.prefix + s), bb.brick_offset + S.brick_base, bb.pair_list,
-                              bb.pair_cap, S.ms.l0_surf, nullptr, bb.status, acc, setup, excl, InjGrids{}, nullptr,
-                              &hb, g, chunk, item, FUSE ? bb.mips + s : nullptr,
+    brick_unit<MODE, STORAGE>(S.sp, bb.tri_rec + __ldg(bb.tri_prefix + s), S.N, g - __ldg(w.prefix + s), bb.brick_offset + S.brick_base, bb.pair_list,
+                              bb.pair_cap, S.ms.l0_surf, nullptr, bb.status, acc, rd, InjGrids{}, nullptr,
+                              &hb, g, chunk, extra, FUSE ? bb.mips + s : nullptr,
                               bb.dirty ? bb.dirty + S.brick_base : nullptr);
-    __syncthreads();  // done with acc
-  }
+  });
 }
 
 // Persistent grid of a batched kernel: `per_sm` CTAs per SM, but never more
@@ -1226,70 +1236,31 @@ unsigned resident_grid(K kern, int threads, size_t smem, int sms, int per_sm, ui
   return (unsigned)std::max<uint32_t>(1u, std::min<uint32_t>((uint32_t)n, items));
 }
 
-// The same brick CTA writing RGBA8 level 0 into linear memory (x fastest)
+// The same brick work writing RGBA8 level 0 into linear memory (x fastest)
 // instead of a surface: the output of vct_voxelize_noalloc.
 template <int MODE>
-__global__ void __launch_bounds__(kThreads) k_bricks_linear(SceneParams sp, int N, const uint32_t* __restrict__ offset,
-                                                            const uint32_t* __restrict__ list, uint32_t cap,
-                                                            uchar4* __restrict__ out) {
-  typedef typename std::conditional<MODE == VCT_VOX_CONSERVATIVE, SetupSat, SetupRef>::type Setup;
+__global__ void __launch_bounds__(kThreads, 7)
+    k_bricks_linear(SceneParams sp, int N, const uint32_t* __restrict__ offset, const uint32_t* __restrict__ list,
+                    uint32_t cap, uchar4* __restrict__ out, FrameStatus* st, HeavyBricks hb, BrickUnits units) {
   __shared__ Acc acc;
-  __shared__ Setup setup[kWarps][32];
-  __shared__ int excl[kWarps][33];
-  const int nb = N / kBrick;
-  const uint32_t brick = blockIdx.x;
-  const int b3[3] = {(int)(brick % nb), (int)((brick / nb) % nb), (int)(brick / ((uint32_t)nb * nb))};
-  for (int i = threadIdx.x; i < kBrickVox; i += kThreads) acc.clear(i);
-  __syncthreads();
-  const uint32_t beg = min(offset[brick], cap), end = min(offset[brick + 1], cap);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (uint32_t base = beg + warp * 32; base < end; base += kWarps * 32) {
-    const uint32_t e = base + lane;
-    int cnt = 0;
-    if (e < end) {
-      if (MODE == VCT_VOX_CONSERVATIVE)
-        cnt = setup_sat(sp, N, __ldg(list + e), b3, reinterpret_cast<SetupSat&>(setup[warp][lane]));
-      else
-        cnt = setup_ref(sp, N, __ldg(list + e), b3, reinterpret_cast<SetupRef&>(setup[warp][lane]));
-    }
-    int incl = cnt;
-    for (int o = 1; o < 32; o <<= 1) {
-      int v = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += v;
-    }
-    excl[warp][lane] = incl - cnt;
-    const int total = __shfl_sync(0xffffffffu, incl, 31);
-    __syncwarp();
-    for (int it = lane; it < total; it += 32) {
-      int lo = 0, hi = 31;
-      while (lo < hi) {
-        int mid = (lo + hi + 1) >> 1;
-        if (excl[warp][mid] <= it) lo = mid; else hi = mid - 1;
-      }
-      const int local = it - excl[warp][lo];
-      if (MODE == VCT_VOX_CONSERVATIVE)
-        item_sat(sp, N, b3, reinterpret_cast<const SetupSat&>(setup[warp][lo]), local, acc);
-      else
-        item_ref(sp, N, b3, reinterpret_cast<const SetupRef&>(setup[warp][lo]), local, acc);
-    }
-    __syncwarp();
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < kBrickVox; i += kThreads) {
-    const uint32_t n = acc.n[i];
-    const int x = b3[0] * kBrick + (i & 7), y = b3[1] * kBrick + ((i >> 3) & 7), z = b3[2] * kBrick + (i >> 6);
-    uchar4 o = make_uchar4(0, 0, 0, 0);
-    if (n) {
-      const unsigned long long den = 2ull * n * 65535ull;
-      unsigned char q[4];
-      for (int ch = 0; ch < 4; ++ch) {
-        unsigned long long v = ((unsigned long long)acc.c[ch][i] * 510ull + (unsigned long long)n * 65535ull) / den;
-        q[ch] = (unsigned char)(v > 255ull ? 255ull : v);
-      }
-      o = make_uchar4(q[0], q[1], q[2], q[3]);
-    }
-    out[((size_t)z * N + y) * N + x] = o;
-  }
+  __shared__ __align__(8) RoundOf<MODE> rd;
+  for_units(hb, units, st, [&](uint32_t brick, uint32_t chunk, bool extra) {
+    brick_unit<MODE, VCT_STORAGE_RGBA8, false, false>(sp, nullptr, N, brick, offset, list, cap, 0, nullptr, st, acc,
+                                                      rd, InjGrids{}, out, &hb, brick, chunk, extra);
+  });
+}
+
+template <class K>
+int resident_per_sm(K kern) {
+  int f = 1;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&f, kern, kThreads, 0) != cudaSuccess || f < 1) f = 1;
+  return f;
+}
+int sm_count() {
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms;
 }
 
 }  // namespace
@@ -1298,26 +1269,39 @@ cudaError_t launch_voxelize_linear(const SceneParams& sp, int N, int mode, const
                                    cudaStream_t st) {
   const int nb = N / kBrick;
   const size_t n_bricks = (size_t)nb * nb * nb;
+  const HeavyBricks& hb = vb.heavy;
+  auto* kern = mode == VCT_VOX_CONSERVATIVE ? k_bricks_linear<VCT_VOX_CONSERVATIVE>
+                                            : k_bricks_linear<VCT_VOX_REF_RASTER2X>;
+  const unsigned grid = (unsigned)std::min<size_t>((size_t)sm_count() * resident_per_sm(kern), n_bricks + hb.item_cap);
   cudaError_t e = cudaMemsetAsync(vb.brick_count, 0, n_bricks * sizeof(uint32_t), st);
   if (e != cudaSuccess) return e;
+  e = cudaMemsetAsync(vb.big_count, 0, sizeof(uint32_t), st);
+  if (e != cudaSuccess) return e;
   const unsigned tri_blocks = (sp.total_tris + 255) / 256;
-  if (tri_blocks)
-    k_bin<false><<<tri_blocks, 256, 0, st>>>(sp, N, vb.brick_count, nullptr, nullptr, 0, vb.status, nullptr, 0,
-                                             nullptr, nullptr);
-  e = launch_exclusive_scan(vb.brick_count, vb.brick_offset, vb.brick_cursor, n_bricks, vb.scan_tmp, st);
+  const dim3 big_grid(128, kBigSplit);
+  if (tri_blocks) {
+    k_bin<false><<<tri_blocks, 256, 0, st>>>(sp, N, vb.brick_count, nullptr, nullptr, 0, vb.status, vb.big, vb.big_cap,
+                                             vb.big_count, vb.bin_rec, nullptr);
+    k_bin_big<false><<<big_grid, 256, 0, st>>>(N, vb.big, vb.big_cap, vb.big_count, vb.brick_count, nullptr, nullptr,
+                                               0, nullptr);
+  }
+  ScanFuse fuse;
+  std::memset(&fuse, 0, sizeof(fuse));
+  fuse.hb = hb;
+  fuse.units = brick_units(vb.units, (uint32_t)n_bricks, nullptr);
+  fuse.cap = vb.pair_cap;
+  fuse.slots = grid;
+  fuse.total_copy = &vb.status->pair_total;
+  e = launch_exclusive_scan(vb.brick_count, vb.brick_offset, vb.brick_cursor, n_bricks, vb.scan_tmp, st, nullptr,
+                            &fuse);
   if (e != cudaSuccess) return e;
-  e = cudaMemcpyAsync(&vb.status->pair_total, vb.brick_offset + n_bricks, sizeof(uint32_t), cudaMemcpyDeviceToDevice,
-                      st);
-  if (e != cudaSuccess) return e;
-  if (tri_blocks)
+  if (tri_blocks) {
     k_bin<true><<<tri_blocks, 256, 0, st>>>(sp, N, nullptr, vb.brick_cursor, vb.pair_list, vb.pair_cap, vb.status,
-                                            nullptr, 0, nullptr, nullptr);
-  if (mode == VCT_VOX_CONSERVATIVE)
-    k_bricks_linear<VCT_VOX_CONSERVATIVE><<<(unsigned)n_bricks, kThreads, 0, st>>>(sp, N, vb.brick_offset,
-                                                                                 vb.pair_list, vb.pair_cap, out);
-  else
-    k_bricks_linear<VCT_VOX_REF_RASTER2X><<<(unsigned)n_bricks, kThreads, 0, st>>>(sp, N, vb.brick_offset,
-                                                                                 vb.pair_list, vb.pair_cap, out);
+                                            vb.big, vb.big_cap, vb.big_count, vb.bin_rec, nullptr);
+    k_bin_big<true><<<big_grid, 256, 0, st>>>(N, vb.big, vb.big_cap, vb.big_count, nullptr, vb.brick_cursor,
+                                              vb.pair_list, vb.pair_cap, nullptr);
+  }
+  kern<<<grid, kThreads, 0, st>>>(sp, N, vb.brick_offset, vb.pair_list, vb.pair_cap, out, vb.status, hb, fuse.units);
   return cudaGetLastError();
 }
 
@@ -1341,26 +1325,26 @@ void dispatch_bricks(int mode, int storage, bool attr, F&& f) {
 }
 
 // CTAs of a kernel resident on one SM (cached per kernel).
-template <class K>
-int resident_per_sm(K kern) {
-  int f = 1;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&f, kern, kThreads, 0) != cudaSuccess || f < 1) f = 1;
-  return f;
-}
 
 cudaError_t launch_voxelize(const SceneParams& sp, int N, int mode, int storage, const VoxBuffers& vb,
                             cudaSurfaceObject_t l0, cudaStream_t st, int* launches, const InjGrids* inj) {
   int nl = 0;
   const int nb = N / kBrick;
   const size_t n_bricks = (size_t)nb * nb * nb;
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int sms = sm_count();
+  const bool fuse_mips = vb.mips && !inj && (storage == VCT_STORAGE_RGBA8 || storage == VCT_STORAGE_RGBA16F);
   int fit = 1;
   dispatch_bricks(mode, storage, inj != nullptr, [&](auto mode_tag, auto storage_tag) {
-    static const int f = resident_per_sm(k_bricks<decltype(mode_tag)::value, decltype(storage_tag)::value>);
-    fit = f;
+    constexpr int M = decltype(mode_tag)::value, S = decltype(storage_tag)::value;
+    static const int plain = resident_per_sm(k_bricks<M, S>);
+    fit = plain;
+    if constexpr (S == VCT_STORAGE_RGBA8 || S == VCT_STORAGE_RGBA16F) {
+      static const int fused = resident_per_sm(k_bricks<M, S, true>);
+      if (fuse_mips) fit = fused;
+    }
   });
+  const uint8_t* dirty = inj || vb.counts ? nullptr : vb.dirty;
+  const BrickUnits units = brick_units(vb.units, (uint32_t)n_bricks, dirty);
   cudaError_t e = cudaMemsetAsync(vb.brick_count, 0, n_bricks * sizeof(uint32_t), st);
   if (e != cudaSuccess) return e;
   const unsigned tri_blocks = (sp.total_tris + 255) / 256;
@@ -1371,7 +1355,7 @@ cudaError_t launch_voxelize(const SceneParams& sp, int N, int mode, int storage,
   }
   if (tri_blocks) {
     k_bin<false><<<tri_blocks, 256, 0, st>>>(sp, N, vb.brick_count, nullptr, nullptr, 0, vb.status, vb.big,
-                                             vb.big_cap, vb.big_count, vb.bin_rec);
+                                             vb.big_cap, vb.big_count, vb.bin_rec, vb.tri_rec);
     ++nl;
     if (vb.big) {
       k_bin_big<false><<<big_grid, 256, 0, st>>>(N, vb.big, vb.big_cap, vb.big_count, vb.brick_count, nullptr, nullptr,
@@ -1385,6 +1369,7 @@ cudaError_t launch_voxelize(const SceneParams& sp, int N, int mode, int storage,
   ScanFuse fuse;
   std::memset(&fuse, 0, sizeof(fuse));
   fuse.hb = hb;
+  fuse.units = units;
   fuse.cap = vb.pair_cap;
   fuse.slots = (uint32_t)(sms * fit);
   fuse.total_copy = &vb.status->pair_total;
@@ -1396,7 +1381,7 @@ cudaError_t launch_voxelize(const SceneParams& sp, int N, int mode, int storage,
   }
   if (tri_blocks) {
     k_bin<true><<<tri_blocks, 256, 0, st>>>(sp, N, nullptr, vb.brick_cursor, vb.pair_list, vb.pair_cap, vb.status,
-                                            vb.big, vb.big_cap, vb.big_count, vb.bin_rec);
+                                            vb.big, vb.big_cap, vb.big_count, vb.bin_rec, vb.tri_rec);
     ++nl;
     if (vb.big) {
       k_bin_big<true><<<big_grid, 256, 0, st>>>(N, vb.big, vb.big_cap, vb.big_count, nullptr, vb.brick_cursor,
@@ -1406,24 +1391,22 @@ cudaError_t launch_voxelize(const SceneParams& sp, int N, int mode, int storage,
   }
   const InjGrids g = inj ? *inj : InjGrids{};
   void* lin = inj ? nullptr : vb.level0_lin;
-  const bool fuse_mips = vb.mips && !inj && (storage == VCT_STORAGE_RGBA8 || storage == VCT_STORAGE_RGBA16F);
   BrickMips bm;
   std::memset(&bm, 0, sizeof(bm));
   if (fuse_mips) bm = *vb.mips;
   bm.dirty = inj ? nullptr : vb.dirty;  // (kernel parameter of every brick kernel)
-  // Before the bricks: two CTAs per SM that run the extra chunks.
-  const uint32_t n_extra = hb.slot ? std::min<uint32_t>(hb.item_cap, (uint32_t)(sms * std::min(fit, 2))) : 0u;
+  const unsigned grid = (unsigned)std::min<size_t>((size_t)sms * fit, n_bricks + (hb.slot ? hb.item_cap : 0u));
   dispatch_bricks(mode, storage, inj != nullptr, [&](auto mode_tag, auto storage_tag) {
     constexpr int M = decltype(mode_tag)::value, S = decltype(storage_tag)::value;
     if constexpr (S == VCT_STORAGE_RGBA8 || S == VCT_STORAGE_RGBA16F) {
       if (fuse_mips) {
-        k_bricks<M, S, true><<<(unsigned)(n_extra + n_bricks), kThreads, 0, st>>>(
-            sp, N, vb.brick_offset, vb.pair_list, vb.pair_cap, l0, vb.counts, vb.status, g, lin, hb, n_extra, bm);
+        k_bricks<M, S, true><<<grid, kThreads, 0, st>>>(
+            sp, N, vb.brick_offset, vb.pair_list, vb.pair_cap, l0, vb.counts, vb.status, g, lin, hb, units, vb.tri_rec, bm);
         return;
       }
     }
-    k_bricks<M, S><<<(unsigned)(n_extra + n_bricks), kThreads, 0, st>>>(
-        sp, N, vb.brick_offset, vb.pair_list, vb.pair_cap, l0, vb.counts, vb.status, g, lin, hb, n_extra, bm);
+    k_bricks<M, S><<<grid, kThreads, 0, st>>>(
+        sp, N, vb.brick_offset, vb.pair_list, vb.pair_cap, l0, vb.counts, vb.status, g, lin, hb, units, vb.tri_rec, bm);
   });
   ++nl;
   if (launches) *launches += nl;
@@ -1470,11 +1453,13 @@ cudaError_t launch_voxelize_batch(const BatchWork& tris, const BatchWork& bricks
                                                0, tris.scenes);
     nl += 2;
   }
-  // Offsets, pair_total, and the dense-brick plan against the persistent
-  // grid's CTAs.
+  // Offsets, pair_total, the dense-brick plan against the persistent grid's
+  // CTAs, and the bricks with work.
+  const BrickUnits units = brick_units(bb.units, total_bricks, bb.dirty);
   ScanFuse fuse;
   std::memset(&fuse, 0, sizeof(fuse));
   fuse.hb = hb;
+  fuse.units = units;
   fuse.cap = bb.pair_cap;
   fuse.slots = grid;
   fuse.total_copy = &bb.status->pair_total;
@@ -1488,12 +1473,10 @@ cudaError_t launch_voxelize_batch(const BatchWork& tris, const BatchWork& bricks
                                               bb.pair_list, bb.pair_cap, tris.scenes);
     nl += 2;
   }
-  e = cudaMemsetAsync(bricks.queue, 0, sizeof(uint32_t), st);
-  if (e != cudaSuccess) return e;
   dispatch_bricks(mode, storage, false, [&](auto mode_tag, auto storage_tag) {
     constexpr int M = decltype(mode_tag)::value, S = decltype(storage_tag)::value;
-    if (fuse_mips) k_bricks_batch<M, S, true><<<grid, kThreads, 0, st>>>(bricks, bb);
-    else k_bricks_batch<M, S><<<grid, kThreads, 0, st>>>(bricks, bb);
+    if (fuse_mips) k_bricks_batch<M, S, true><<<grid, kThreads, 0, st>>>(bricks, bb, units);
+    else k_bricks_batch<M, S><<<grid, kThreads, 0, st>>>(bricks, bb, units);
   });
   ++nl;
   if (launches) *launches += nl;

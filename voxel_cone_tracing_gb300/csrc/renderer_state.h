@@ -180,7 +180,7 @@ struct HeavyStore {
   // owner's stream, so the zeroing is ordered before its next frame.
   vct_status reserve(size_t n_bricks, uint32_t slots, uint32_t n_items, cudaStream_t st) {
     VCT_CHECK(slot.ensure(n_bricks));
-    VCT_CHECK(counters.ensure(3));
+    VCT_CHECK(counters.ensure(2));
     if (slots > slot_cap) {
       // the slots and their counters start at zero and every frame leaves them so
       VCT_CHECK(brick.ensure(slots));
@@ -408,9 +408,10 @@ struct vct_renderer {
   DevBuf<uint32_t> d_obj_material;
   DevBuf<DevInstance> d_inst;
   HostBuf<DevInstance> h_inst;
-  DevBuf<uint32_t> brick_count, brick_offset, brick_cursor, pair_list, scan_tmp, counts;
+  DevBuf<uint32_t> brick_count, brick_offset, brick_cursor, brick_units, pair_list, scan_tmp, counts;
   DevBuf<BinRec> bin_big;           // large-triangle binning records
   DevBuf<uint2> bin_rec;            // per triangle: counting pass -> filling pass
+  DevBuf<TriRec> tri_rec;           // per triangle: counting pass -> bricks
   DevBuf<uint32_t> bin_big_count;
   uint32_t bin_big_cap = 0;
   HeavyStore heavy;                 // dense bricks split across CTAs
@@ -549,6 +550,7 @@ struct vct_renderer {
     VCT_CHECK(brick_count.ensure(nb));
     VCT_CHECK(brick_offset.ensure(nb + 1));
     VCT_CHECK(brick_cursor.ensure(nb));
+    VCT_CHECK(brick_units.ensure(nb + 4));
     VCT_CHECK(brick_dirty.ensure(nb));
     VCT_CHECK(scan_tmp.ensure(scan_tmp_words(nb)));
     VCT_CHECK(heavy.reserve(nb, 256, 16384, stream));
@@ -702,6 +704,7 @@ struct vct_renderer {
     const uint32_t pairs_needed = (uint32_t)std::min<uint64_t>(0xffffff00ull, 4ull * total + 65536ull);
     if (pair_list.n < pairs_needed) VCT_CHECK(pair_list.ensure(pairs_needed));
     VCT_CHECK(bin_rec.ensure(std::max<size_t>(total, 1)));
+    VCT_CHECK(tri_rec.ensure(std::max<size_t>(total, 1)));
 
     VoxBuffers vb;
     vb.brick_count = brick_count.p;
@@ -716,8 +719,10 @@ struct vct_renderer {
     vb.big_cap = bin_big_cap;
     vb.big_count = bin_big_count.p;
     vb.level0_lin = have_l0_map ? (void*)l0_lin.p : nullptr;
+    vb.units = brick_units.p;
     vb.heavy = kHeavySplit ? heavy.view() : HeavyBricks{};
     vb.bin_rec = bin_rec.p;
+    vb.tri_rec = tri_rec.p;
     // Anisotropic maps: the brick kernel writes mip levels 1-3 itself (not
     // for light injection, whose level 0 comes from k_inject).
     BrickMips bm;

@@ -71,14 +71,28 @@ struct FrameStatus {
 };
 
 // Dense bricks: a brick with more than kHeavyChunk (triangle, brick) pairs
-// is split into chunks of kHeavyChunk pairs processed by different CTAs of
+// is split into chunks of up to kHeavyChunk pairs processed by different CTAs of
 // the same launch.  Every chunk adds its sums atomically into the brick's
 // global accumulator slot (integer sums: exact and order-free); the CTA that
 // finishes the last chunk (a per-slot counter) writes the brick's texels and
 // zeroes the slot and its counter again, so slots are zero between frames.
 // A brick that gets no slot (the lists are full) is processed whole by one
 // CTA, which is also exact.
-constexpr uint32_t kHeavyChunk = 1024;
+//
+// Split are bricks of more than kHeavyChunk pairs that are also more than
+// kHeavyShare times a resident CTA's share of the launch: only such a brick
+// can end it.  Voxelization, us, 500,000 triangles at 256^3 / 120,000 at 128^3,
+// conservative / 200,000 at 128^3 into linear memory: 1024 pairs and one share
+// 266 / 171 / 137, 512 and two 260 / 166 / 113, 384 and two 262 / 163 / 115;
+// 512 and one share 289 / 162 / 115 (in uneven chunks).
+constexpr uint32_t kHeavyChunk = 512;
+constexpr uint32_t kHeavyShare = 2;
+// Chunks of a dense brick's pairs, and pairs per chunk: equal, in rounds of 128.
+__host__ __device__ inline uint32_t heavy_chunks(uint32_t pairs) { return (pairs + kHeavyChunk - 1) / kHeavyChunk; }
+__host__ __device__ inline uint32_t heavy_span(uint32_t pairs) {
+  const uint32_t n = heavy_chunks(pairs);
+  return ((pairs + n - 1) / n + 127u) / 128u * 128u;
+}
 #ifndef VCT_HEAVY_SPLIT
 #define VCT_HEAVY_SPLIT 1  // build with -DVCT_HEAVY_SPLIT=0 to time whole-brick CTAs only
 #endif
@@ -89,8 +103,27 @@ struct HeavyBricks {
   uint32_t* done;      // per slot: chunks finished in this frame
   void* acc;           // per slot: the brick's sums (the voxelizer's accumulator type)
   uint2* items;        // (brick, chunk >= 1), (0xffffffff, 0) = unused
-  uint32_t* counters;  // [0] slots taken, [1] items taken, [2] next item to run
+  uint32_t* counters;  // [0] slots taken, [1] items taken
   uint32_t slot_cap, item_cap;
+};
+
+// The bricks a frame has work for, in a launch of resident CTAs that take
+// them in turn: those with pairs (long: more than kLongBrick), and the empty ones whose texels an earlier
+// frame left non-zero.  Most of a grid is neither.
+constexpr uint32_t kLongBrick = 128;  // pairs; shorter bricks are taken several at a time
+struct BrickUnits {
+  uint32_t* list;        // long bricks from the front, short ones from the back
+  uint32_t* count;       // [0] long, [1] short, [2] units taken beyond a first one each
+  uint32_t cap;          // bricks
+  const uint8_t* dirty;  // null: empty bricks are written too
+};
+
+// A triangle as the brick kernels take it: grid-space positions, unit
+// normals, material id (as bits).  Written by the counting pass, which has the
+// positions at hand; a brick's setup then reads 80 bytes in place of the
+// instance, three indices, three vertices and two material tables.
+struct TriRec {
+  float4 q[5];
 };
 
 // A triangle with many candidate bricks, binned by k_bin_big.
@@ -215,13 +248,15 @@ struct VoxBuffers {
   uint32_t* scan_tmp;      // block sums
   uint32_t* counts;        // N^3 or nullptr
   FrameStatus* status;
-  BinRec* big;             // large-triangle records (nullptr: bin them in-warp)
+  BinRec* big;             // large-triangle records
   uint32_t big_cap;
   uint32_t* big_count;
   void* level0_lin;        // level 0 also in linear memory (x fastest), or null
   HeavyBricks heavy;       // dense-brick splitting (heavy.slot null: off)
+  uint32_t* units;         // 4 + n_bricks words for BrickUnits
   uint2* bin_rec;          // per triangle: the counting pass's bricks, replayed
-                           // by the filling pass (total_tris; null: recompute)
+                           // by the filling pass
+  TriRec* tri_rec;         // per triangle (null in the linear path)
   const BrickMips* mips;   // anisotropic maps: the brick kernel writes levels 1-3 too (null: off)
   // Per brick: 1 when its level-0 texels (and linear copy, and fused levels
   // 1-3 and occupancy bytes) may hold non-zero data from an earlier frame;
@@ -338,7 +373,10 @@ struct BatchBuffers {
   RasterBuffers rb;       // vis / gb_pos / gb_nrm point at pixel 0 of the batch
   uchar4* frame;
   HeavyBricks heavy;      // over the batch-wide (global) brick indices
+  uint32_t* units;        // 4 + total bricks words for BrickUnits
   uint2* bin_rec;         // per (padded) batch triangle, as VoxBuffers::bin_rec
+  TriRec* tri_rec;        // per (padded) batch triangle
+  const uint32_t* tri_prefix;  // a scene's first (padded) batch triangle
   uint8_t* dirty;         // per batch brick (global index), as VoxBuffers::dirty
   const BrickMips* mips;  // per scene: the brick kernel writes levels 1-3 too (null: off)
 };
@@ -420,10 +458,11 @@ cudaError_t launch_trace_px(const SceneParams& sp, const CameraParams& cp, const
 // hold scan_tmp_words(n) words.
 size_t scan_tmp_words(size_t n);
 // Work fused into the exclusive scan of the brick counts (no launches of
-// its own): the dense-brick plan, one brick per thread of the add-back
-// kernel, and a copy of the total.
+// its own): the dense-brick plan and the list of bricks with work, one brick per
+// thread of the add-back kernel, and a copy of the total.
 struct ScanFuse {
   HeavyBricks hb;        // hb.slot null: no plan
+  BrickUnits units;      // units.list null: none
   uint32_t cap;          // pair-list capacity (offsets beyond it are clamped)
   uint32_t slots;        // CTAs of the brick launch resident at once
   uint32_t* total_copy;  // also receives the total (or null)
@@ -432,20 +471,19 @@ cudaError_t launch_exclusive_scan(const uint32_t* in, uint32_t* out, uint32_t* c
                                   cudaStream_t st, int* launches = nullptr, const ScanFuse* fuse = nullptr);
 
 // The split plan of brick b with pairs [beg, end) of `pairs` in all: the
-// brick is dense when it has more than kHeavyChunk pairs and more than the
-// launch's pairs per resident CTA (a lighter brick cannot hold up the
-// launch's end).  A dense brick gets an accumulator slot and one work item
-// per extra chunk of kHeavyChunk pairs; every brick's slot is written (-1:
+// brick is dense when it has more than kHeavyChunk pairs and more than
+// kHeavyShare times the launch's pairs per resident CTA.  A dense brick gets an accumulator slot and one work item
+// per extra chunk; every brick's slot is written (-1:
 // not split).  A brick whose slot or items do not fit is left whole.
 // counters[0..1] count the dense bricks and their extra chunks (all of
 // them, also those that did not fit).
 __device__ __forceinline__ void heavy_plan_brick(uint32_t b, uint32_t beg, uint32_t end, uint32_t pairs,
                                                  uint32_t slots, const HeavyBricks& hb) {
-  const unsigned long long fair = ((unsigned long long)pairs + slots - 1) / (slots ? slots : 1u);
+  const unsigned long long fair = kHeavyShare * (((unsigned long long)pairs + slots - 1) / (slots ? slots : 1u));
   const uint32_t dense = fair > kHeavyChunk ? (fair > 0xffffffffull ? 0xffffffffu : (uint32_t)fair) : kHeavyChunk;
   int32_t slot = -1;
   if (end - beg > dense) {
-    const uint32_t nch = (end - beg + kHeavyChunk - 1) / kHeavyChunk;
+    const uint32_t nch = heavy_chunks(end - beg);
     const uint32_t s = atomicAdd(&hb.counters[0], 1u);
     const uint32_t e = atomicAdd(&hb.counters[1], nch - 1);
     const bool ok = s < hb.slot_cap && e + (nch - 1) <= hb.item_cap;
