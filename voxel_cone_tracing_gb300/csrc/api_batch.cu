@@ -512,7 +512,11 @@ vct_status build_batch(vct_batch* b, const vct_batch_scene* descs, uint32_t n) {
   VCT_CHECK(b->tri_rec.ensure(std::max<size_t>(b->tris.total(), 1)));
   VCT_CHECK(b->bin_big_count.ensure(1));
   VCT_CHECK(b->grow_bin_big(1 << 12));
+  // (zero between frames)
+  VCT_CUDA(cudaMemsetAsync(b->brick_count.p, 0, nbk * sizeof(uint32_t), b->stream));
+  VCT_CUDA(cudaMemsetAsync(b->bin_big_count.p, 0, sizeof(uint32_t), b->stream));
   VCT_CHECK(b->rbig_count.ensure(1));
+  VCT_CUDA(cudaMemsetAsync(b->rbig_count.p, 0, sizeof(*b->rbig_count.p), b->stream));
   VCT_CHECK(b->grow_rbig(1 << 16));
   VCT_CHECK(b->queue.ensure(1));
   VCT_CHECK(b->vis.ensure(px));

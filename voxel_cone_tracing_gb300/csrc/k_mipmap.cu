@@ -656,6 +656,7 @@ __device__ __forceinline__ int occ_level(const MapSet& ms, uint32_t& g) {
 
 template <bool DILATE>
 __global__ void __launch_bounds__(256) k_occupancy(MapSet ms, uint32_t total) {
+  follows_previous();
   for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < total; g += gridDim.x * blockDim.x) {
     uint32_t w = g;
     const int c = occ_level(ms, w);
@@ -666,6 +667,7 @@ __global__ void __launch_bounds__(256) k_occupancy(MapSet ms, uint32_t total) {
 
 template <bool DILATE>
 __global__ void __launch_bounds__(256) k_occupancy_batch(BatchWork bw) {
+  follows_previous();
   for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < bw.total; g += gridDim.x * blockDim.x) {
     const int s = batch_scene_of(bw, g);
     const MapSet& ms = bw.scenes[s].ms;
@@ -726,16 +728,18 @@ cudaError_t launch_mipmap(const MapSet& ms, int mip_mode, cudaStream_t st, int* 
   MapSet mo = ms;
   mo.occ_k = ms.L - 1;
   const uint32_t total = occ_words(mo);
-  k_occupancy<false><<<(total + 255) / 256, 256, 0, st>>>(mo, total);
-  k_occupancy<true><<<(total + 255) / 256, 256, 0, st>>>(mo, total);
+  e = launch_next(k_occupancy<false>, (total + 255) / 256, 256, st, mo, total);
+  if (e == cudaSuccess) e = launch_next(k_occupancy<true>, (total + 255) / 256, 256, st, mo, total);
+  if (e != cudaSuccess) return e;
   if (launches) *launches += 2;
   return cudaGetLastError();
 }
 
 cudaError_t launch_occupancy_batch(const BatchWork& words, cudaStream_t st, int* launches) {
   if (!words.total) return cudaSuccess;
-  k_occupancy_batch<false><<<(words.total + 255) / 256, 256, 0, st>>>(words);
-  k_occupancy_batch<true><<<(words.total + 255) / 256, 256, 0, st>>>(words);
+  cudaError_t e = launch_next(k_occupancy_batch<false>, (words.total + 255) / 256, 256, st, words);
+  if (e == cudaSuccess) e = launch_next(k_occupancy_batch<true>, (words.total + 255) / 256, 256, st, words);
+  if (e != cudaSuccess) return e;
   if (launches) *launches += 2;
   return cudaGetLastError();
 }

@@ -318,6 +318,7 @@ __device__ __forceinline__ uint32_t warp_last_not_above(const uint32_t* __restri
 // the setup thread were no alternative: one thread writes a whole screen's
 // (64x64 tiles 155 us for all of the G-buffer, 32x32 210).
 __global__ void __launch_bounds__(256) k_gb_big(RasterBuffers rb, int W, const BatchScene* scenes) {
+  follows_previous();
   const uint32_t total = (uint32_t)*rb.big_count, records = (uint32_t)(*rb.big_count >> 32);
   const int lane = threadIdx.x & 31;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -427,11 +428,15 @@ __device__ __forceinline__ void resolve_px(const SceneParams& sp, const CameraPa
 }
 
 __global__ void __launch_bounds__(256) k_gb_resolve(SceneParams sp, CameraParams cp, RasterBuffers rb) {
+  follows_previous();
+  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *rb.big_count = 0;  // for the next frame
   resolve_px(sp, cp, rb, blockIdx.x * 16 + (threadIdx.x & 15), blockIdx.y * 16 + (threadIdx.x >> 4));
 }
 
 // 16x16-pixel tiles of every batch scene.
 __global__ void __launch_bounds__(256) k_gb_resolve_batch(BatchWork w, RasterBuffers rb) {
+  follows_previous();
+  if (blockIdx.x == 0 && threadIdx.x == 0) *rb.big_count = 0;  // for the next frame
   for (uint32_t g = blockIdx.x; g < w.total; g += gridDim.x) {
     const int s = batch_scene_of(w, g);
     const BatchScene& S = w.scenes[s];
@@ -449,15 +454,15 @@ cudaError_t launch_gbuffer(const SceneParams& sp, const CameraParams& cp, const 
                            int* launches) {
   cudaError_t e = cudaMemsetAsync(rb.vis, 0xff, (size_t)cp.W * cp.H * sizeof(unsigned long long), st);
   if (e != cudaSuccess) return e;
-  e = cudaMemsetAsync(rb.big_count, 0, sizeof(*rb.big_count), st);
-  if (e != cudaSuccess) return e;
   if (sp.total_tris) k_gb_setup<<<(sp.total_tris + kSetup - 1) / kSetup, kSetup, 0, st>>>(sp, cp, rb);
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  k_gb_big<<<sms * 6, 256, 0, st>>>(rb, cp.W, nullptr);
+  e = launch_next(k_gb_big, sms * 6, 256, st, rb, cp.W, nullptr);
+  if (e != cudaSuccess) return e;
   dim3 grid((cp.W + 15) / 16, (cp.H + 15) / 16);
-  k_gb_resolve<<<grid, 256, 0, st>>>(sp, cp, rb);
+  e = launch_next(k_gb_resolve, grid, 256, st, sp, cp, rb);
+  if (e != cudaSuccess) return e;
   if (launches) *launches += (sp.total_tris ? 1 : 0) + 2;
   return cudaGetLastError();
 }
@@ -467,17 +472,17 @@ cudaError_t launch_gbuffer_batch(const BatchWork& tris, const BatchWork& tiles, 
   const RasterBuffers& rb = bb.rb;
   cudaError_t e = cudaMemsetAsync(rb.vis, 0xff, total_px * sizeof(unsigned long long), st);
   if (e != cudaSuccess) return e;
-  e = cudaMemsetAsync(rb.big_count, 0, sizeof(*rb.big_count), st);
-  if (e != cudaSuccess) return e;
   int nl = 0;
   if (tris.total) {
     const unsigned grid = (unsigned)std::max(1, std::min<int>(sms * 32, (int)((tris.total + kSetup - 1) / kSetup)));
     k_gb_setup_batch<<<grid, kSetup, 0, st>>>(tris, rb);
     ++nl;
   }
-  k_gb_big<<<sms * 6, 256, 0, st>>>(rb, 0, tris.scenes);
+  e = launch_next(k_gb_big, sms * 6, 256, st, rb, 0, tris.scenes);
+  if (e != cudaSuccess) return e;
   const unsigned rgrid = (unsigned)std::max(1, std::min<int>(sms * 8, (int)tiles.total));
-  k_gb_resolve_batch<<<rgrid, 256, 0, st>>>(tiles, rb);
+  e = launch_next(k_gb_resolve_batch, rgrid, 256, st, tiles, rb);
+  if (e != cudaSuccess) return e;
   nl += 2;
   if (launches) *launches += nl;
   return cudaGetLastError();

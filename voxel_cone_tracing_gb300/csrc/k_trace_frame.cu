@@ -341,6 +341,7 @@ __global__ void __launch_bounds__(256, SHARE ? VCT_SHADE_MIN_BLOCKS : 6)
             const float4* __restrict__ gb_pos, const float4* __restrict__ gb_nrm, uchar4* __restrict__ frame,
             float4* __restrict__ frame_f32, TraceWork tw, const float4* __restrict__ diffuse,
             const __grid_constant__ ConeStep first, const __grid_constant__ ConeRing ring) {
+  follows_previous();  // (the maps it samples were whole before k_march)
   int px, py;
   share_tile_px(blockIdx.x * 16, blockIdx.y * 16, px, py);
   const size_t p = (size_t)py * cp.W + px;
@@ -498,9 +499,14 @@ cudaError_t run_frame(const SceneParams& sp, const CameraParams& cp, const MapSe
   const float4* diffuse = !tp.enable_diffuse ? nullptr : (tp.diffuse_in ? tp.diffuse_in : tw.diffuse);
   const dim3 grid((cp.W + 15) / 16, (cp.H + 15) / 16);
   auto shade = share ? k_shade<ISO, true> : k_shade<ISO, false>;
-  shade<<<grid, 256, 0, st>>>(sp, cp, ms, tp, gb_pos, gb_nrm, frame, frame_f32, tw, diffuse, cone.step[0], sched.ring);
+  cudaError_t e = cudaSuccess;
+  if (mp.per_tile)
+    e = launch_next(shade, grid, 256, st, sp, cp, ms, tp, gb_pos, gb_nrm, frame, frame_f32, tw, diffuse, cone.step[0],
+                    sched.ring);
+  else
+    shade<<<grid, 256, 0, st>>>(sp, cp, ms, tp, gb_pos, gb_nrm, frame, frame_f32, tw, diffuse, cone.step[0], sched.ring);
   if (launches) ++*launches;
-  return cudaGetLastError();
+  return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 }  // namespace

@@ -328,6 +328,7 @@ __global__ void __launch_bounds__(256) k_bin(SceneParams sp, int N, uint32_t* __
                                              uint32_t cap, FrameStatus* st, BinRec* __restrict__ big,
                                              uint32_t big_cap, uint32_t* __restrict__ big_count,
                                              uint2* __restrict__ rec, TriRec* __restrict__ recs) {
+  follows_previous();
   bin_tri<FILL>(sp, N, blockIdx.x * blockDim.x + threadIdx.x, count, cursor, list, cap, st, big, big_cap, big_count,
                 0u, rec, recs);
 }
@@ -336,6 +337,7 @@ __global__ void __launch_bounds__(256) k_bin(SceneParams sp, int N, uint32_t* __
 // are padded to multiples of 32, so a warp bins one scene.
 template <bool FILL>
 __global__ void __launch_bounds__(256) k_bin_batch(BatchWork w, BatchBuffers bb) {
+  follows_previous();
   for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < w.total; g += gridDim.x * blockDim.x) {
     const int s = batch_scene_of(w, g);
     const BatchScene& S = w.scenes[s];
@@ -355,6 +357,7 @@ __global__ void __launch_bounds__(256) k_bin_big(int N, const BinRec* __restrict
                                                  const uint32_t* __restrict__ big_count, uint32_t* __restrict__ count,
                                                  uint32_t* __restrict__ cursor, uint32_t* __restrict__ list,
                                                  uint32_t cap, const BatchScene* __restrict__ scenes) {
+  follows_previous();
   const uint32_t n = min(*big_count, big_cap);
   for (uint32_t r = blockIdx.x; r < n; r += gridDim.x) {
     const BinRec& rec = big[r];
@@ -1160,12 +1163,13 @@ __device__ __forceinline__ void brick_unit(const SceneParams& sp, const TriRec* 
 }
 
 // The list of bricks with work in `words` (4 + bricks words).
-BrickUnits brick_units(uint32_t* words, uint32_t bricks, const uint8_t* dirty) {
+BrickUnits brick_units(uint32_t* words, uint32_t bricks, const uint8_t* dirty, uint32_t* reset) {
   BrickUnits u;
   u.list = words + 4;
   u.count = words;
   u.cap = bricks;
   u.dirty = dirty;
+  u.reset = reset;
   return u;
 }
 
@@ -1177,6 +1181,8 @@ BrickUnits brick_units(uint32_t* words, uint32_t bricks, const uint8_t* dirty) {
 template <class F>
 __device__ __forceinline__ void for_units(const HeavyBricks& hb, const BrickUnits& u, FrameStatus* st, F&& f) {
   __shared__ uint32_t s_next[2];
+  follows_previous();
+  if (u.reset && blockIdx.x == 0 && threadIdx.x == 0) *u.reset = 0u;
   const uint32_t n_items = hb.slot ? min(hb.counters[1], hb.item_cap) : 0u, n_long = u.count[0];
   const uint32_t total = n_items + n_long + u.count[1];
   if (hb.slot && blockIdx.x == 0 && threadIdx.x < 2) (&st->heavy_total)[threadIdx.x] = hb.counters[threadIdx.x];
@@ -1263,6 +1269,15 @@ int sm_count() {
   return sms;
 }
 
+// The filling passes of one renderer's triangles.
+cudaError_t fill_lists(const SceneParams& sp, int N, const VoxBuffers& vb, unsigned tri_blocks, cudaStream_t st) {
+  cudaError_t e = launch_next(k_bin<true>, tri_blocks, 256, st, sp, N, nullptr, vb.brick_cursor, vb.pair_list,
+                              vb.pair_cap, vb.status, vb.big, vb.big_cap, vb.big_count, vb.bin_rec, nullptr);
+  if (e != cudaSuccess) return e;
+  return launch_next(k_bin_big<true>, dim3(128, kBigSplit), 256, st, N, vb.big, vb.big_cap, vb.big_count, nullptr,
+                     vb.brick_cursor, vb.pair_list, vb.pair_cap, nullptr);
+}
+
 }  // namespace
 
 cudaError_t launch_voxelize_linear(const SceneParams& sp, int N, int mode, const VoxBuffers& vb, uchar4* out,
@@ -1282,13 +1297,14 @@ cudaError_t launch_voxelize_linear(const SceneParams& sp, int N, int mode, const
   if (tri_blocks) {
     k_bin<false><<<tri_blocks, 256, 0, st>>>(sp, N, vb.brick_count, nullptr, nullptr, 0, vb.status, vb.big, vb.big_cap,
                                              vb.big_count, vb.bin_rec, nullptr);
-    k_bin_big<false><<<big_grid, 256, 0, st>>>(N, vb.big, vb.big_cap, vb.big_count, vb.brick_count, nullptr, nullptr,
-                                               0, nullptr);
+    e = launch_next(k_bin_big<false>, big_grid, 256, st, N, vb.big, vb.big_cap, vb.big_count, vb.brick_count, nullptr,
+                    nullptr, 0u, nullptr);
+    if (e != cudaSuccess) return e;
   }
   ScanFuse fuse;
   std::memset(&fuse, 0, sizeof(fuse));
   fuse.hb = hb;
-  fuse.units = brick_units(vb.units, (uint32_t)n_bricks, nullptr);
+  fuse.units = brick_units(vb.units, (uint32_t)n_bricks, nullptr, nullptr);
   fuse.cap = vb.pair_cap;
   fuse.slots = grid;
   fuse.total_copy = &vb.status->pair_total;
@@ -1296,13 +1312,11 @@ cudaError_t launch_voxelize_linear(const SceneParams& sp, int N, int mode, const
                             &fuse);
   if (e != cudaSuccess) return e;
   if (tri_blocks) {
-    k_bin<true><<<tri_blocks, 256, 0, st>>>(sp, N, nullptr, vb.brick_cursor, vb.pair_list, vb.pair_cap, vb.status,
-                                            vb.big, vb.big_cap, vb.big_count, vb.bin_rec, nullptr);
-    k_bin_big<true><<<big_grid, 256, 0, st>>>(N, vb.big, vb.big_cap, vb.big_count, nullptr, vb.brick_cursor,
-                                              vb.pair_list, vb.pair_cap, nullptr);
+    e = fill_lists(sp, N, vb, tri_blocks, st);
+    if (e != cudaSuccess) return e;
   }
-  kern<<<grid, kThreads, 0, st>>>(sp, N, vb.brick_offset, vb.pair_list, vb.pair_cap, out, vb.status, hb, fuse.units);
-  return cudaGetLastError();
+  return launch_next(kern, grid, kThreads, st, sp, N, vb.brick_offset, vb.pair_list, vb.pair_cap, out, vb.status, hb,
+                     fuse.units);
 }
 
 // Calls f(mode tag, storage tag) for the brick kernel a frame uses.
@@ -1344,24 +1358,16 @@ cudaError_t launch_voxelize(const SceneParams& sp, int N, int mode, int storage,
     }
   });
   const uint8_t* dirty = inj || vb.counts ? nullptr : vb.dirty;
-  const BrickUnits units = brick_units(vb.units, (uint32_t)n_bricks, dirty);
-  cudaError_t e = cudaMemsetAsync(vb.brick_count, 0, n_bricks * sizeof(uint32_t), st);
-  if (e != cudaSuccess) return e;
+  const BrickUnits units = brick_units(vb.units, (uint32_t)n_bricks, dirty, vb.big_count);
+  cudaError_t e = cudaSuccess;
   const unsigned tri_blocks = (sp.total_tris + 255) / 256;
-  const dim3 big_grid(128, kBigSplit);
-  if (vb.big) {
-    e = cudaMemsetAsync(vb.big_count, 0, sizeof(uint32_t), st);
-    if (e != cudaSuccess) return e;
-  }
   if (tri_blocks) {
     k_bin<false><<<tri_blocks, 256, 0, st>>>(sp, N, vb.brick_count, nullptr, nullptr, 0, vb.status, vb.big,
                                              vb.big_cap, vb.big_count, vb.bin_rec, vb.tri_rec);
-    ++nl;
-    if (vb.big) {
-      k_bin_big<false><<<big_grid, 256, 0, st>>>(N, vb.big, vb.big_cap, vb.big_count, vb.brick_count, nullptr, nullptr,
-                                                 0, nullptr);
-      ++nl;
-    }
+    e = launch_next(k_bin_big<false>, dim3(128, kBigSplit), 256, st, N, vb.big, vb.big_cap, vb.big_count,
+                    vb.brick_count, nullptr, nullptr, 0u, nullptr);
+    if (e != cudaSuccess) return e;
+    nl += 2;
   }
   // Offsets, pair_total <- offset[n_bricks], and the dense-brick plan
   // against the brick CTAs resident at once.
@@ -1373,21 +1379,15 @@ cudaError_t launch_voxelize(const SceneParams& sp, int N, int mode, int storage,
   fuse.cap = vb.pair_cap;
   fuse.slots = (uint32_t)(sms * fit);
   fuse.total_copy = &vb.status->pair_total;
+  fuse.big_total = &vb.status->bigtri_total;
+  fuse.big_count = vb.big_count;
+  fuse.clear = true;
   e = launch_exclusive_scan(vb.brick_count, vb.brick_offset, vb.brick_cursor, n_bricks, vb.scan_tmp, st, &nl, &fuse);
   if (e != cudaSuccess) return e;
-  if (vb.big) {
-    e = cudaMemcpyAsync(&vb.status->bigtri_total, vb.big_count, sizeof(uint32_t), cudaMemcpyDeviceToDevice, st);
-    if (e != cudaSuccess) return e;
-  }
   if (tri_blocks) {
-    k_bin<true><<<tri_blocks, 256, 0, st>>>(sp, N, nullptr, vb.brick_cursor, vb.pair_list, vb.pair_cap, vb.status,
-                                            vb.big, vb.big_cap, vb.big_count, vb.bin_rec, vb.tri_rec);
-    ++nl;
-    if (vb.big) {
-      k_bin_big<true><<<big_grid, 256, 0, st>>>(N, vb.big, vb.big_cap, vb.big_count, nullptr, vb.brick_cursor,
-                                                vb.pair_list, vb.pair_cap, nullptr);
-      ++nl;
-    }
+    e = fill_lists(sp, N, vb, tri_blocks, st);
+    if (e != cudaSuccess) return e;
+    nl += 2;
   }
   const InjGrids g = inj ? *inj : InjGrids{};
   void* lin = inj ? nullptr : vb.level0_lin;
@@ -1400,14 +1400,13 @@ cudaError_t launch_voxelize(const SceneParams& sp, int N, int mode, int storage,
     constexpr int M = decltype(mode_tag)::value, S = decltype(storage_tag)::value;
     if constexpr (S == VCT_STORAGE_RGBA8 || S == VCT_STORAGE_RGBA16F) {
       if (fuse_mips) {
-        k_bricks<M, S, true><<<grid, kThreads, 0, st>>>(
-            sp, N, vb.brick_offset, vb.pair_list, vb.pair_cap, l0, vb.counts, vb.status, g, lin, hb, units, vb.tri_rec, bm);
+        e = launch_next(k_bricks<M, S, true>, grid, kThreads, st, sp, N, vb.brick_offset, vb.pair_list, vb.pair_cap, l0, vb.counts, vb.status, g, lin, hb, units, vb.tri_rec, bm);
         return;
       }
     }
-    k_bricks<M, S><<<grid, kThreads, 0, st>>>(
-        sp, N, vb.brick_offset, vb.pair_list, vb.pair_cap, l0, vb.counts, vb.status, g, lin, hb, units, vb.tri_rec, bm);
+    e = launch_next(k_bricks<M, S>, grid, kThreads, st, sp, N, vb.brick_offset, vb.pair_list, vb.pair_cap, l0, vb.counts, vb.status, g, lin, hb, units, vb.tri_rec, bm);
   });
+  if (e != cudaSuccess) return e;
   ++nl;
   if (launches) *launches += nl;
   return cudaGetLastError();
@@ -1440,22 +1439,20 @@ cudaError_t launch_voxelize_batch(const BatchWork& tris, const BatchWork& bricks
                 : resident_grid(k_bricks_batch<M, S>, kThreads, 0, sms, shape.bricks_ctas_per_sm,
                                 bricks.total + (hb.slot ? hb.item_cap : 0u));
   });
-  cudaError_t e = cudaMemsetAsync(bb.brick_count, 0, (size_t)total_bricks * sizeof(uint32_t), st);
-  if (e != cudaSuccess) return e;
-  e = cudaMemsetAsync(bb.big_count, 0, sizeof(uint32_t), st);
-  if (e != cudaSuccess) return e;
+  cudaError_t e = cudaSuccess;
   const unsigned bin_grid = resident_grid(k_bin_batch<false>, 256, 0, sms, shape.bin_ctas_per_sm,
                                           (tris.total + 255) / 256);
   const dim3 big_grid(128, kBigSplit);
   if (tris.total) {
     k_bin_batch<false><<<bin_grid, 256, 0, st>>>(tris, bb);
-    k_bin_big<false><<<big_grid, 256, 0, st>>>(0, bb.big, bb.big_cap, bb.big_count, bb.brick_count, nullptr, nullptr,
-                                               0, tris.scenes);
+    e = launch_next(k_bin_big<false>, big_grid, 256, st, 0, bb.big, bb.big_cap, bb.big_count, bb.brick_count, nullptr,
+                    nullptr, 0u, tris.scenes);
+    if (e != cudaSuccess) return e;
     nl += 2;
   }
   // Offsets, pair_total, the dense-brick plan against the persistent grid's
   // CTAs, and the bricks with work.
-  const BrickUnits units = brick_units(bb.units, total_bricks, bb.dirty);
+  const BrickUnits units = brick_units(bb.units, total_bricks, bb.dirty, bb.big_count);
   ScanFuse fuse;
   std::memset(&fuse, 0, sizeof(fuse));
   fuse.hb = hb;
@@ -1463,21 +1460,24 @@ cudaError_t launch_voxelize_batch(const BatchWork& tris, const BatchWork& bricks
   fuse.cap = bb.pair_cap;
   fuse.slots = grid;
   fuse.total_copy = &bb.status->pair_total;
+  fuse.big_total = &bb.status->bigtri_total;
+  fuse.big_count = bb.big_count;
+  fuse.clear = true;
   e = launch_exclusive_scan(bb.brick_count, bb.brick_offset, bb.brick_cursor, total_bricks, scan_tmp, st, &nl, &fuse);
   if (e != cudaSuccess) return e;
-  e = cudaMemcpyAsync(&bb.status->bigtri_total, bb.big_count, sizeof(uint32_t), cudaMemcpyDeviceToDevice, st);
-  if (e != cudaSuccess) return e;
   if (tris.total) {
-    k_bin_batch<true><<<bin_grid, 256, 0, st>>>(tris, bb);
-    k_bin_big<true><<<big_grid, 256, 0, st>>>(0, bb.big, bb.big_cap, bb.big_count, nullptr, bb.brick_cursor,
-                                              bb.pair_list, bb.pair_cap, tris.scenes);
+    e = launch_next(k_bin_batch<true>, bin_grid, 256, st, tris, bb);
+    if (e != cudaSuccess) return e;
+    e = launch_next(k_bin_big<true>, big_grid, 256, st, 0, bb.big, bb.big_cap, bb.big_count, nullptr, bb.brick_cursor,
+                    bb.pair_list, bb.pair_cap, tris.scenes);
+    if (e != cudaSuccess) return e;
     nl += 2;
   }
   dispatch_bricks(mode, storage, false, [&](auto mode_tag, auto storage_tag) {
     constexpr int M = decltype(mode_tag)::value, S = decltype(storage_tag)::value;
-    if (fuse_mips) k_bricks_batch<M, S, true><<<grid, kThreads, 0, st>>>(bricks, bb, units);
-    else k_bricks_batch<M, S><<<grid, kThreads, 0, st>>>(bricks, bb, units);
+    e = launch_next(fuse_mips ? k_bricks_batch<M, S, true> : k_bricks_batch<M, S>, grid, kThreads, st, bricks, bb, units);
   });
+  if (e != cudaSuccess) return e;
   ++nl;
   if (launches) *launches += nl;
   return cudaGetLastError();

@@ -553,6 +553,9 @@ struct vct_renderer {
     VCT_CHECK(brick_units.ensure(nb + 4));
     VCT_CHECK(brick_dirty.ensure(nb));
     VCT_CHECK(scan_tmp.ensure(scan_tmp_words(nb)));
+    // The binning counters start at zero, and every frame leaves them so.
+    VCT_CUDA(cudaMemsetAsync(brick_count.p, 0, brick_count.n * sizeof(uint32_t), stream));
+    VCT_CUDA(cudaMemsetAsync(bin_big_count.p, 0, sizeof(uint32_t), stream));
     VCT_CHECK(heavy.reserve(nb, 256, 16384, stream));
     if (cfg.keep_counts) VCT_CHECK(counts.ensure((size_t)r * r * r));
     have_frame = false;
@@ -603,6 +606,7 @@ struct vct_renderer {
     VCT_CHECK(h_status.ensure(1));
     std::memset(h_status.p, 0, sizeof(FrameStatus));
     VCT_CHECK(big_count.ensure(1));
+    VCT_CUDA(cudaMemsetAsync(big_count.p, 0, sizeof(*big_count.p), stream));
     VCT_CHECK(grow_big(1 << 16));
     VCT_CHECK(grow_bin_big(1 << 12));
     return alloc_maps((uint32_t)cfg.grid_res);
