@@ -171,22 +171,25 @@ __device__ bool tri_box_f32(const float v[3][3], const float c[3], const float h
   return true;
 }
 
-// One (triangle, candidate brick) test of the binning passes.
+// May triangle v (voxel units) touch brick (bx, by, bz)?
+__device__ __forceinline__ bool touches_brick(const float v[3][3], int bx, int by, int bz) {
+  const int b3[3] = {bx, by, bz};
+  float c[3], h[3];
+  for (int d = 0; d < 3; ++d) {
+    float lo = (float)(b3[d] * kBrick) - kBinMargin - (b3[d] == 0 ? 1.0f : 0.0f);
+    float hi = (float)(b3[d] * kBrick + kBrick) + kBinMargin;
+    c[d] = 0.5f * (lo + hi);
+    h[d] = 0.5f * (hi - lo);
+  }
+  return tri_box_f32(v, c, h);
+}
+
+// One (triangle, candidate brick) pair of the binning passes.
 template <bool FILL>
-__device__ __forceinline__ bool bin_one(const float v[3][3], int bx, int by, int bz, int nb, bool test, uint32_t t,
+__device__ __forceinline__ void bin_one(const float v[3][3], int bx, int by, int bz, int nb, uint32_t t,
                                         uint32_t* __restrict__ count, uint32_t* __restrict__ cursor,
                                         uint32_t* __restrict__ list, uint32_t cap) {
-  if (test) {
-    const int b3[3] = {bx, by, bz};
-    float c[3], h[3];
-    for (int d = 0; d < 3; ++d) {
-      float lo = (float)(b3[d] * kBrick) - kBinMargin - (b3[d] == 0 ? 1.0f : 0.0f);
-      float hi = (float)(b3[d] * kBrick + kBrick) + kBinMargin;
-      c[d] = 0.5f * (lo + hi);
-      h[d] = 0.5f * (hi - lo);
-    }
-    if (!tri_box_f32(v, c, h)) return false;
-  }
+  if (!touches_brick(v, bx, by, bz)) return;
   const uint32_t brick = ((uint32_t)bz * nb + by) * nb + bx;
   if (FILL) {
     uint32_t slot = atomicAdd(cursor + brick, 1u);
@@ -194,7 +197,6 @@ __device__ __forceinline__ bool bin_one(const float v[3][3], int bx, int by, int
   } else {
     atomicAdd(count + brick, 1u);
   }
-  return true;
 }
 
 constexpr int kSoloBricks = 8;  // candidate bricks a lane bins on its own
@@ -227,21 +229,10 @@ __device__ __forceinline__ void bin_tri(const SceneParams& sp, int N, uint32_t t
   int blo[3] = {0, 0, 0}, bhi[3] = {-1, -1, -1};
   int vol = 0;
   bool again = true;  // (filling pass) this lane's triangle is binned from scratch
+  uint2 r = make_uint2(0u, 0u);
   if (FILL && t < sp.total_tris) {
-    // Replay the counting pass's bricks (same pairs, no triangle reload).
-    const uint2 r = rec[t];
+    r = rec[t];
     again = (r.y & kRecAgain) != 0u;
-    if (!again) {
-      const int x0 = (int)(r.x & 1023u), y0 = (int)((r.x >> 10) & 1023u), z0 = (int)(r.x >> 20);
-      const int ex = (int)((r.y >> 8) & 7u) + 1, ey = (int)((r.y >> 11) & 7u) + 1;
-      for (uint32_t m = r.y & 0xffu; m; m &= m - 1) {
-        const int i = __ffs(m) - 1;
-        const uint32_t brick = ((uint32_t)(z0 + i / (ex * ey)) * nb + (uint32_t)(y0 + (i / ex) % ey)) * nb +
-                               (uint32_t)(x0 + i % ex);
-        const uint32_t slot = atomicAdd(cursor + brick, 1u);
-        if (slot < cap) list[slot] = t;
-      }
-    }
   }
   if (again && t < sp.total_tris) {
     TriLoad tl;
@@ -270,17 +261,39 @@ __device__ __forceinline__ void bin_tri(const SceneParams& sp, int N, uint32_t t
         vol = (bhi[0] - blo[0] + 1) * (bhi[1] - blo[1] + 1) * (bhi[2] - blo[2] + 1);
     }
   }
-  if (vol > 0 && vol <= kSoloBricks) {
+  if (!FILL && vol > 0 && vol <= kSoloBricks) {
     uint32_t mask = 0u;
     int i = 0;
     for (int bz = blo[2]; bz <= bhi[2]; ++bz)
       for (int by = blo[1]; by <= bhi[1]; ++by)
         for (int bx = blo[0]; bx <= bhi[0]; ++bx, ++i)
-          if (bin_one<FILL>(v, bx, by, bz, nb, vol > 1, t, count, cursor, list, cap)) mask |= 1u << i;
-    if (!FILL)
-      rec[t] = make_uint2((uint32_t)blo[0] | (uint32_t)blo[1] << 10 | (uint32_t)blo[2] << 20,
-                          mask | (uint32_t)(bhi[0] - blo[0]) << 8 | (uint32_t)(bhi[1] - blo[1]) << 11 |
-                              (uint32_t)(bhi[2] - blo[2]) << 14);
+          if (vol == 1 || touches_brick(v, bx, by, bz)) mask |= 1u << i;
+    r = make_uint2((uint32_t)blo[0] | (uint32_t)blo[1] << 10 | (uint32_t)blo[2] << 20,
+                   mask | (uint32_t)(bhi[0] - blo[0]) << 8 | (uint32_t)(bhi[1] - blo[1]) << 11 |
+                       (uint32_t)(bhi[2] - blo[2]) << 14);
+    rec[t] = r;
+  }
+  // The warp's triangles lie side by side, so most of its lanes meet in a brick
+  // or two: one atomic for all of a brick's.  Counting and filling, us, with an
+  // atomic per pair and now: 500,000 triangles 44 and 35, 37 and 18; 16 scenes
+  // 251 and 148, 110 and 53.  What is left is the triangles' loads and records.
+  uint32_t m = r.y & 0xffu;
+  for (unsigned any = __ballot_sync(0xffffffffu, m != 0u); any; any = __ballot_sync(0xffffffffu, m != 0u)) {
+    if (!m) continue;
+    const int i = __ffs((int)m) - 1, ex = (int)((r.y >> 8) & 7u) + 1, ey = (int)((r.y >> 11) & 7u) + 1;
+    m &= m - 1;
+    const uint32_t brick = ((r.x >> 20) + (uint32_t)(i / (ex * ey))) * nb * nb +
+                           (((r.x >> 10) & 1023u) + (uint32_t)((i / ex) % ey)) * nb + (r.x & 1023u) + (uint32_t)(i % ex);
+    const unsigned peers = __match_any_sync(any, brick);
+    const int lead = __ffs((int)peers) - 1;
+    if (FILL) {
+      uint32_t slot = 0;
+      if (lane == lead) slot = atomicAdd(cursor + brick, (uint32_t)__popc(peers));
+      slot = __shfl_sync(peers, slot, lead) + (uint32_t)__popc(peers & ((1u << lane) - 1u));
+      if (slot < cap) list[slot] = t;
+    } else if (lane == lead) {
+      atomicAdd(count + brick, (uint32_t)__popc(peers));
+    }
   }
   bool in_warp = vol > kSoloBricks;
   if (!FILL && t < sp.total_tris && (in_warp || vol <= 0)) {
@@ -291,15 +304,15 @@ __device__ __forceinline__ void bin_tri(const SceneParams& sp, int N, uint32_t t
       const uint32_t slot = atomicAdd(big_count, 1u);
       if (slot < big_cap) {
         in_warp = false;
-        BinRec r;
+        BinRec b;
         for (int k = 0; k < 3; ++k)
-          for (int d = 0; d < 3; ++d) r.v[k][d] = v[k][d];
-        for (int d = 0; d < 3; ++d) { r.blo[d] = blo[d]; r.bhi[d] = bhi[d]; }
-        r.t = t;
-        r.vol = (uint32_t)vol;
-        r.scene = scene;
-        r.pad = 0;
-        big[slot] = r;
+          for (int d = 0; d < 3; ++d) b.v[k][d] = v[k][d];
+        for (int d = 0; d < 3; ++d) { b.blo[d] = blo[d]; b.bhi[d] = bhi[d]; }
+        b.t = t;
+        b.vol = (uint32_t)vol;
+        b.scene = scene;
+        b.pad = 0;
+        big[slot] = b;
       }
     }
     rec[t] = make_uint2(0u, in_warp ? kRecAgain : 0u);
@@ -318,7 +331,7 @@ __device__ __forceinline__ void bin_tri(const SceneParams& sp, int N, uint32_t t
     const int n = __shfl_sync(0xffffffffu, vol, src);
     const uint32_t ts = __shfl_sync(0xffffffffu, t, src);
     for (int i = lane; i < n; i += 32)
-      bin_one<FILL>(w, x0 + i % nx, y0 + (i / nx) % ny, z0 + i / (nx * ny), nb, true, ts, count, cursor, list, cap);
+      bin_one<FILL>(w, x0 + i % nx, y0 + (i / nx) % ny, z0 + i / (nx * ny), nb, ts, count, cursor, list, cap);
   }
 }
 
@@ -376,7 +389,7 @@ __global__ void __launch_bounds__(256) k_bin_big(int N, const BinRec* __restrict
     const int nx = rec.bhi[0] - rec.blo[0] + 1, ny = rec.bhi[1] - rec.blo[1] + 1;
     for (uint32_t i = blockIdx.y * blockDim.x + threadIdx.x; i < rec.vol; i += gridDim.y * blockDim.x)
       bin_one<FILL>(v, rec.blo[0] + (int)(i % nx), rec.blo[1] + (int)((i / nx) % ny), rec.blo[2] + (int)(i / (nx * ny)),
-                    nb, true, rec.t, cnt, cur, list, cap);
+                    nb, rec.t, cnt, cur, list, cap);
   }
 }
 
