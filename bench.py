@@ -681,7 +681,7 @@ def run_ours(args):
         "e2e": {"value": round(e2e_ms, 4), "unit": UNIT, "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                 "statistic": "median of per-step host wall times", "mean": round(e2e_mean, 4)},
         "gpu_launches": int(sum(st["kernel_launches"] for st in stages)),
-        "roofline": {"kernel": "k_trace_share", "bound": "tex", "achieved": round(achieved_tex, 2),
+        "roofline": {"kernel": "k_march + k_shade", "bound": "tex", "achieved": round(achieved_tex, 2),
                      "peak": round(rate_quad / 1e9, 2), "unit": "Gfetch/s", "frac": round(achieved_tex * 1e9 / rate_quad, 4),
                      "traffic": traffic, "peak_source": "measured in this run (vct_measure_texture_rate)",
                      "fetches": {"two_level_per_pixel": TRACE_FETCH_QUAD_PER_PIXEL,
