@@ -176,8 +176,9 @@ struct HeavyStore {
     return std::max({heavy_slot_bytes(VCT_STORAGE_RGBA8), heavy_slot_bytes(VCT_STORAGE_RGBA16F),
                      heavy_slot_bytes(kStorageAttr)});
   }
-  // Called between frames (no kernel of the owner in flight); `st` is the
-  // owner's stream, so the zeroing is ordered before its next frame.
+  // Called between frames (no kernel of the owner in flight); the zeroing, on
+  // the owner's stream `st`, is complete on return: the owner's next frame may
+  // run on another stream.
   vct_status reserve(size_t n_bricks, uint32_t slots, uint32_t n_items, cudaStream_t st) {
     VCT_CHECK(slot.ensure(n_bricks));
     VCT_CHECK(counters.ensure(2));
@@ -188,6 +189,7 @@ struct HeavyStore {
       VCT_CHECK(acc.ensure((size_t)slots * slot_bytes()));
       VCT_CUDA(cudaMemsetAsync(done.p, 0, (size_t)slots * sizeof(uint32_t), st));
       VCT_CUDA(cudaMemsetAsync(acc.p, 0, (size_t)slots * slot_bytes(), st));
+      VCT_CUDA(cudaStreamSynchronize(st));
       slot_cap = slots;
     }
     if (n_items > item_cap) {
@@ -559,6 +561,7 @@ struct vct_renderer {
     VCT_CHECK(heavy.reserve(nb, 256, 16384, stream));
     if (cfg.keep_counts) VCT_CHECK(counts.ensure((size_t)r * r * r));
     have_frame = false;
+    VCT_CUDA(cudaStreamSynchronize(stream));  // (the memsets, before the caller may change streams)
     return VCT_OK;
   }
 
