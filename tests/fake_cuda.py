@@ -39,6 +39,7 @@ def scene(w=32, h=16):
     return scenes.scene_sphere(seed=1, freq=4, width=w, height=h)
 def loaded(**cfg):
     r, s = R.Renderer(32, 16, **dict(dict(grid_res=32), **cfg)), scene()
+    r.set_voxel_view_dir(7, 0.0)
     return r, s, R.load_scene(r, s)
 def frame(r, s, ids):
     R.queue_scene(r, s, ids)

@@ -1,5 +1,9 @@
 """The order of what the host code puts on its streams, on a CUDA runtime that
 runs nothing (fake_cuda.py); no GPU."""
+import re
+
+import pytest
+
 from tests.fake_cuda import run, unfinished
 
 
@@ -31,3 +35,44 @@ def test_setup_is_complete_when_a_call_returns(tmp_path):
     for name, log in out.items():
         assert any(line.startswith("memset") for line in log), name
         assert not unfinished(log), (name, unfinished(log))
+
+
+@pytest.mark.parametrize("kind", ["renderer", "side streams", "batch", "graph"])
+@pytest.mark.parametrize("kernel", ["k_bin", "k_scan_tiles", "k_bricks", "k_gb_setup", "k_gb_big", "k_march"])
+def test_counters_are_zero_after_a_failed_frame(tmp_path, kind, kernel):
+    """A frame leaves the binning and raster counters zero by its last kernels.
+    After one whose launches failed part of the way, the next frame clears them
+    before its first kernel, once what was launched has run."""
+    out = run(tmp_path, f"""
+        kind, kernel = {kind!r}, {kernel!r}
+        if kind in ("batch", "graph"):
+            fake.fake_clear()
+            b = R.Batch([(scene(), 32, 16, 32, 0)], use_graph=kind == "graph")
+            b.shape = dict(b.shape, trace_per_scene=1)
+            take("set-up")
+            render = b.render
+        else:
+            fake.fake_clear()
+            r, s, ids = loaded(overlap_raster=int(kind == "side streams"))
+            take("set-up")
+            render = lambda: frame(r, s, ids)
+        fake.fake_fail(kernel.encode(), 0)
+        out["failed"] = fails(render)
+        take("bad")
+        render()
+        take("good")
+        (b if kind in ("batch", "graph") else r).synchronize()
+        fake.fake_clear()
+        render()
+        take("next")
+    """)
+    assert out["failed"]
+    zeroed = lambda log: {tuple(x.split()[1:3]) for x in log if re.match(r"memset .* to 0 ", x)}  # noqa: E731
+    first = lambda log, what: next(i for i, x in enumerate(log) if re.match(what, x))  # noqa: E731
+    counters = {c for c in zeroed(out["set-up"]) if int(c[1]) in (4, 8, 4 * (32 // 8) ** 3)}
+    assert {int(c[1]) for c in counters} == {4, 8, 256}
+    good = out["good"]
+    head = good[:first(good, "capture|launch|replay")]
+    assert counters <= zeroed(head)
+    assert not unfinished([x for x in out["bad"] if not x.endswith("FAILED")] + [x for x in head if "sync" in x])
+    assert not counters & zeroed(out["next"])  # (and a good one needs no clearing)

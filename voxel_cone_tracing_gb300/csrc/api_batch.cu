@@ -103,6 +103,7 @@ struct vct_batch {
   cudaGraphExec_t graph = nullptr;
   bool pending = false, have_frame = false;
   int launches = 0;
+  bool counters_zero = false;  // brick_count, bin_big_count and rbig_count are zero (zero_counters)
 
   ~vct_batch() {
     if (stream) cudaStreamSynchronize(stream);
@@ -245,7 +246,33 @@ struct vct_batch {
     return VCT_OK;
   }
 
+  // The binning and raster counters, which a frame expects to be zero and
+  // leaves so.  Complete on return.
+  vct_status zero_counters() {
+    counters_zero = false;
+    VCT_CUDA(cudaMemsetAsync(brick_count.p, 0, brick_count.n * sizeof(uint32_t), stream));
+    VCT_CUDA(cudaMemsetAsync(bin_big_count.p, 0, sizeof(uint32_t), stream));
+    VCT_CUDA(cudaMemsetAsync(rbig_count.p, 0, sizeof(*rbig_count.p), stream));
+    VCT_CUDA(cudaStreamSynchronize(stream));
+    counters_zero = true;
+    return VCT_OK;
+  }
+
+  // Puts a frame on the streams.  One that fails part of the way may leave
+  // the counters that its later kernels would have cleared: what was launched
+  // is waited for, and the next frame clears them first.
   vct_status submit() {
+    if (!counters_zero) VCT_CHECK(zero_counters());
+    const vct_status s = submit_frame();
+    if (s == VCT_OK) return s;
+    counters_zero = false;
+    for (cudaStream_t st : side)
+      if (cudaStreamSynchronize(st) != cudaSuccess) cudaGetLastError();  // (the frame's own error is the one reported)
+    if (cudaStreamSynchronize(stream) != cudaSuccess) cudaGetLastError();
+    return s;
+  }
+
+  vct_status submit_frame() {
     if (cfg.use_graph) {
       if (!graph) {
         cudaGraph_t g = nullptr;
@@ -512,11 +539,7 @@ vct_status build_batch(vct_batch* b, const vct_batch_scene* descs, uint32_t n) {
   VCT_CHECK(b->tri_rec.ensure(std::max<size_t>(b->tris.total(), 1)));
   VCT_CHECK(b->bin_big_count.ensure(1));
   VCT_CHECK(b->grow_bin_big(1 << 12));
-  // (zero between frames)
-  VCT_CUDA(cudaMemsetAsync(b->brick_count.p, 0, nbk * sizeof(uint32_t), b->stream));
-  VCT_CUDA(cudaMemsetAsync(b->bin_big_count.p, 0, sizeof(uint32_t), b->stream));
   VCT_CHECK(b->rbig_count.ensure(1));
-  VCT_CUDA(cudaMemsetAsync(b->rbig_count.p, 0, sizeof(*b->rbig_count.p), b->stream));
   VCT_CHECK(b->grow_rbig(1 << 16));
   VCT_CHECK(b->queue.ensure(1));
   VCT_CHECK(b->vis.ensure(px));
@@ -539,8 +562,7 @@ vct_status build_batch(vct_batch* b, const vct_batch_scene* descs, uint32_t n) {
   VCT_CHECK(b->d_status.ensure(1));
   VCT_CHECK(b->h_status.ensure(1));
   std::memset(b->h_status.p, 0, sizeof(FrameStatus));
-  VCT_CUDA(cudaStreamSynchronize(b->stream));  // (the set-up memsets, before the caller may change streams)
-  return VCT_OK;
+  return b->zero_counters();  // (waits for the set-up memsets, before the caller may change streams)
 }
 
 }  // namespace

@@ -416,6 +416,7 @@ struct vct_renderer {
   DevBuf<TriRec> tri_rec;           // per triangle: counting pass -> bricks
   DevBuf<uint32_t> bin_big_count;
   uint32_t bin_big_cap = 0;
+  bool counters_zero = false;       // brick_count, bin_big_count and big_count are zero (zero_counters)
   HeavyStore heavy;                 // dense bricks split across CTAs
   DevBuf<FrameStatus> d_status;
   HostBuf<FrameStatus> h_status;
@@ -555,13 +556,22 @@ struct vct_renderer {
     VCT_CHECK(brick_units.ensure(nb + 4));
     VCT_CHECK(brick_dirty.ensure(nb));
     VCT_CHECK(scan_tmp.ensure(scan_tmp_words(nb)));
-    // The binning counters start at zero, and every frame leaves them so.
-    VCT_CUDA(cudaMemsetAsync(brick_count.p, 0, brick_count.n * sizeof(uint32_t), stream));
-    VCT_CUDA(cudaMemsetAsync(bin_big_count.p, 0, sizeof(uint32_t), stream));
     VCT_CHECK(heavy.reserve(nb, 256, 16384, stream));
     if (cfg.keep_counts) VCT_CHECK(counts.ensure((size_t)r * r * r));
     have_frame = false;
-    VCT_CUDA(cudaStreamSynchronize(stream));  // (the memsets, before the caller may change streams)
+    return zero_counters();
+  }
+
+  // The binning and raster counters, which a frame expects to be zero and
+  // leaves so.  Complete on return: the caller may change streams before the
+  // next frame.
+  vct_status zero_counters() {
+    counters_zero = false;
+    VCT_CUDA(cudaMemsetAsync(brick_count.p, 0, brick_count.n * sizeof(uint32_t), stream));
+    VCT_CUDA(cudaMemsetAsync(bin_big_count.p, 0, sizeof(uint32_t), stream));
+    VCT_CUDA(cudaMemsetAsync(big_count.p, 0, sizeof(*big_count.p), stream));
+    VCT_CUDA(cudaStreamSynchronize(stream));
+    counters_zero = true;
     return VCT_OK;
   }
 
@@ -609,7 +619,6 @@ struct vct_renderer {
     VCT_CHECK(h_status.ensure(1));
     std::memset(h_status.p, 0, sizeof(FrameStatus));
     VCT_CHECK(big_count.ensure(1));
-    VCT_CUDA(cudaMemsetAsync(big_count.p, 0, sizeof(*big_count.p), stream));
     VCT_CHECK(grow_big(1 << 16));
     VCT_CHECK(grow_bin_big(1 << 12));
     return alloc_maps((uint32_t)cfg.grid_res);
@@ -649,7 +658,20 @@ struct vct_renderer {
     return VCT_OK;
   }
 
+  // Puts one frame on the streams.  A frame that fails part of the way may
+  // leave the counters that its later kernels would have cleared: what was
+  // launched is waited for, and the next frame clears them first.
   vct_status encode(const FrameInputs& fi) {
+    if (!counters_zero) VCT_CHECK(zero_counters());
+    const vct_status s = encode_frame(fi);
+    if (s == VCT_OK) return s;
+    counters_zero = false;
+    for (cudaStream_t st : {gb_stream, vx_stream, stream})
+      if (cudaStreamSynchronize(st) != cudaSuccess) cudaGetLastError();  // (the frame's own error is the one reported)
+    return s;
+  }
+
+  vct_status encode_frame(const FrameInputs& fi) {
     // Material ids of every queued draw object must exist (the reference
     // indexes m_materials unchecked, renderer.cpp:252).
     uint64_t total = 0;
