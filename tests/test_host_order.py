@@ -76,3 +76,29 @@ def test_counters_are_zero_after_a_failed_frame(tmp_path, kind, kernel):
     assert counters <= zeroed(head)
     assert not unfinished([x for x in out["bad"] if not x.endswith("FAILED")] + [x for x in head if "sync" in x])
     assert not counters & zeroed(out["next"])  # (and a good one needs no clearing)
+
+
+@pytest.mark.parametrize("word,value", [("HEAVY_TOTAL", 5000), ("EXTRA_TOTAL", 100000)])
+def test_graph_is_captured_again_after_the_slots_grew(tmp_path, word, value):
+    """A captured frame holds the split bricks' arrays.  Once a frame's status
+    made them larger, the freed ones must not be replayed."""
+    out = run(tmp_path, f"""
+        b = R.Batch([(scene(), 32, 16, 32, 0)], use_graph=True)
+        b.render()
+        b.render()
+        status({word}, {value})
+        b.render()
+        fake.fake_clear()
+        b.synchronize()
+        take("grow")
+        b.render()
+        take("next")
+        status({word}, 0)
+        b.synchronize()
+        fake.fake_clear()
+        b.render()
+        take("same")
+    """)
+    assert any(x.startswith("free") for x in out["grow"])
+    assert any(x.startswith("capture") for x in out["next"])
+    assert not any(x.startswith("capture") for x in out["same"])

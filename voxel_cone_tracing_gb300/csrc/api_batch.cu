@@ -307,7 +307,13 @@ struct vct_batch {
       VCT_CUDA(cudaStreamSynchronize(stream));
       pending = false;
       const FrameStatus s = *h_status.p;
-      VCT_CHECK(heavy.grow(s, brick_count.n, stream));  // exact either way: no redo
+      const HeavyBricks before = heavy.view();
+      const vct_status grown = heavy.grow(s, brick_count.n, stream);  // exact either way: no redo
+      const HeavyBricks after = heavy.view();
+      if (after.acc != before.acc || after.items != before.items || after.slot_cap != before.slot_cap ||
+          after.item_cap != before.item_cap)
+        drop_graph();  // (it holds the old arrays)
+      VCT_CHECK(grown);
       bool redo = false;
       if (s.pair_total > pair_list.n) {
         VCT_CHECK(pair_list.ensure((size_t)s.pair_total + s.pair_total / 4 + 4096));
