@@ -84,16 +84,14 @@ def test_graph_is_captured_again_after_the_slots_grew(tmp_path, word, value):
     made them larger, the freed ones must not be replayed."""
     out = run(tmp_path, f"""
         b = R.Batch([(scene(), 32, 16, 32, 0)], use_graph=True)
-        b.render()
-        b.render()
         status({word}, {value})
         b.render()
+        status({word}, 0)
         fake.fake_clear()
         b.synchronize()
         take("grow")
         b.render()
         take("next")
-        status({word}, 0)
         b.synchronize()
         fake.fake_clear()
         b.render()
