@@ -42,7 +42,10 @@ cudaError_t copy(const char* what, void* d, const void* s, size_t n, cudaMemcpyK
     for (const auto& w : g_status) static_cast<unsigned*>(d)[w.first] = w.second;
   return cudaSuccess;
 }
-cudaError_t launch(const void* f, size_t smem, cudaStream_t st) {
+cudaError_t launch(const void* f, void** args, size_t smem, cudaStream_t st) {
+  // k_bin's large-triangle records and their capacity
+  if (g_kernels[f].find("5k_binILb") != std::string::npos)
+    g_log += "records " + hex(*static_cast<void**>(args[7])) + " " + std::to_string(*static_cast<unsigned*>(args[8])) + "\n";
   return note("launch", g_kernels[f] + " smem " + std::to_string(smem) + " stream " + hex(st), cudaErrorLaunchOutOfResources);
 }
 cudaError_t g_last = cudaSuccess;
@@ -91,13 +94,13 @@ cudaError_t __cudaPopCallConfiguration(dim3* g, dim3* b, size_t* smem, void* st)
   *(cudaStream_t*)st = g_stream;
   return cudaSuccess;
 }
-cudaError_t __cudaLaunchKernel(cudaKernel_t k, dim3, dim3, void**, size_t smem, cudaStream_t st) {
-  const cudaError_t e = launch((const void*)k, smem, st);
+cudaError_t __cudaLaunchKernel(cudaKernel_t k, dim3, dim3, void** args, size_t smem, cudaStream_t st) {
+  const cudaError_t e = launch((const void*)k, args, smem, st);
   if (e != cudaSuccess) g_last = e;  // (a plain launch reports by cudaGetLastError)
   return e;
 }
-cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void**) {
-  const cudaError_t e = launch(f, c->dynamicSmemBytes, c->stream);
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void** args) {
+  const cudaError_t e = launch(f, args, c->dynamicSmemBytes, c->stream);
   if (e != cudaSuccess) g_last = e;
   return e;
 }

@@ -100,3 +100,35 @@ def test_graph_is_captured_again_after_the_slots_grew(tmp_path, word, value):
     assert any(x.startswith("free") for x in out["grow"])
     assert any(x.startswith("capture") for x in out["next"])
     assert not any(x.startswith("capture") for x in out["same"])
+
+
+def test_what_could_not_be_allocated_is_not_used(tmp_path):
+    """A list that a frame needed larger and that no memory was found for is
+    gone: the next frame's kernels get it with a capacity of 0, and it is
+    allocated again once there is memory.  So are the maps of a new grid."""
+    out = run(tmp_path, """
+        r, s, ids = loaded()
+        status(BIGTRI_TOTAL, 200000)
+        frame(r, s, ids)
+        fake.fake_fail(b"malloc", 0)
+        out["failed"] = [fails(r.synchronize)]
+        fake.fake_clear()
+        status(BIGTRI_TOTAL, 0)
+        frame(r, s, ids)
+        take("without a list")
+        r.synchronize()
+        fake.fake_fail(b"malloc3d", 0)
+        out["failed"].append(fails(r.set_grid_resolution, 64))
+        fake.fake_fail(b"malloc3d", 0)
+        out["failed"].append(fails(frame, r, s, ids))
+        take("without maps")
+        fake.fake_fail(b"", -1)
+        frame(r, s, ids)
+        take("with maps")
+        out["grid"] = r.grid()[0]
+    """)
+    assert out["failed"] == [True, True, True]
+    lists = [x.split()[1:] for x in out["without a list"] if x.startswith("records")]
+    assert lists and all(cap == "0" for _, cap in lists)
+    assert not any(x.startswith("launch") for x in out["without maps"])
+    assert any(x.startswith("malloc3d") for x in out["with maps"]) and out["grid"] == 64

@@ -165,12 +165,15 @@ struct vct_batch {
     return w;
   }
 
+  // (No records, should an allocation fail: the old ones are gone.)
   vct_status grow_bin_big(uint32_t cap) {
+    bin_big_cap = 0;
     VCT_CHECK(bin_big.ensure(cap));
     bin_big_cap = cap;
     return VCT_OK;
   }
   vct_status grow_rbig(uint32_t cap) {
+    rbig_cap = 0;
     VCT_CHECK(rbig.ensure((size_t)cap * big_record_bytes()));
     VCT_CHECK(rbig_first.ensure(cap));
     rbig_cap = cap;

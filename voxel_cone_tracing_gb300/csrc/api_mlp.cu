@@ -173,7 +173,7 @@ extern "C" vct_status vct_mlp_train(vct_renderer* r, const vct_mlp_desc* d, vct_
   vct_mlp_desc dd;
   if (d) dd = *d; else vct_mlp_desc_default(&dd);
   VCT_CHECK(r->finish());
-  if (!r->have_sp || !r->last_sp.total_tris)
+  if (!r->maps_ready || !r->have_sp || !r->last_sp.total_tris)
     return set_error(VCT_ERR_INVALID_VALUE, "render a frame with queued models before training");
   if (!dd.n_samples) return set_error(VCT_ERR_INVALID_VALUE, "n_samples is 0");
   VCT_CHECK(alloc_and_init(r, dd));

@@ -239,7 +239,7 @@ extern "C" vct_status vct_set_grid_resolution(vct_renderer* r, uint32_t res) {
   if (!r) return set_error(VCT_ERR_INVALID_VALUE, "NULL renderer");
   if (!is_pow2(res) || res < 8 || res > 1024)
     return set_error(VCT_ERR_INVALID_VALUE, "grid resolution %u: need a power of two in [8, 1024]", res);
-  if (res == r->res && r->maps.l0_arr) return VCT_OK;
+  if (res == r->res && r->maps_ready) return VCT_OK;
   VCT_CHECK(r->finish());
   r->cfg.grid_res = (int32_t)res;
   return r->alloc_maps(res);

@@ -325,6 +325,7 @@ __global__ void __launch_bounds__(256) k_gb_big(RasterBuffers rb, int W, const B
     rb.status->big_total = records;
     rb.status->big_tiles = total;
   }
+  if (!rb.big_cap) return;  // (no list: reported by big_total)
   // few tiles: up to 8 warps on one, each taking every so many-th row of blocks
   const uint32_t warps = gridDim.x * 8;
   int sh = 0;

@@ -184,6 +184,7 @@ struct HeavyStore {
     VCT_CHECK(counters.ensure(2));
     if (slots > slot_cap) {
       // the slots and their counters start at zero and every frame leaves them so
+      slot_cap = 0;  // (no slots, should one of these fail)
       VCT_CHECK(brick.ensure(slots));
       VCT_CHECK(done.ensure(slots));
       VCT_CHECK(acc.ensure((size_t)slots * slot_bytes()));
@@ -193,6 +194,7 @@ struct HeavyStore {
       slot_cap = slots;
     }
     if (n_items > item_cap) {
+      item_cap = 0;
       VCT_CHECK(items.ensure(n_items));
       item_cap = n_items;
     }
@@ -416,6 +418,7 @@ struct vct_renderer {
   DevBuf<TriRec> tri_rec;           // per triangle: counting pass -> bricks
   DevBuf<uint32_t> bin_big_count;
   uint32_t bin_big_cap = 0;
+  bool maps_ready = false;          // the maps and work arrays of the grid are allocated
   bool counters_zero = false;       // brick_count, bin_big_count and big_count are zero (zero_counters)
   HeavyStore heavy;                 // dense bricks split across CTAs
   DevBuf<FrameStatus> d_status;
@@ -532,6 +535,7 @@ struct vct_renderer {
   // set_grid_resolution (renderer.cpp:178-188): six 3D textures of `levels`
   // mip levels.  Here: level 0 once + one chain (levels 1..L-1) per map.
   vct_status alloc_maps(uint32_t r) {
+    maps_ready = false;
     if (gb_stream) VCT_CUDA(cudaStreamSynchronize(gb_stream));
     if (vx_stream) VCT_CUDA(cudaStreamSynchronize(vx_stream));
     if (stream) VCT_CUDA(cudaStreamSynchronize(stream));
@@ -559,7 +563,9 @@ struct vct_renderer {
     VCT_CHECK(heavy.reserve(nb, 256, 16384, stream));
     if (cfg.keep_counts) VCT_CHECK(counts.ensure((size_t)r * r * r));
     have_frame = false;
-    return zero_counters();
+    VCT_CHECK(zero_counters());
+    maps_ready = true;
+    return VCT_OK;
   }
 
   // The binning and raster counters, which a frame expects to be zero and
@@ -624,7 +630,9 @@ struct vct_renderer {
     return alloc_maps((uint32_t)cfg.grid_res);
   }
 
+  // (No records, should an allocation fail: the old ones are gone.)
   vct_status grow_bin_big(uint32_t cap) {
+    bin_big_cap = 0;
     VCT_CHECK(bin_big.ensure(cap));
     VCT_CHECK(bin_big_count.ensure(1));
     bin_big_cap = cap;
@@ -632,6 +640,7 @@ struct vct_renderer {
   }
 
   vct_status grow_big(uint32_t cap) {
+    big_cap = 0;
     VCT_CHECK(big.ensure((size_t)cap * big_record_bytes()));
     VCT_CHECK(big_first.ensure(cap));
     big_cap = cap;
@@ -662,6 +671,7 @@ struct vct_renderer {
   // leave the counters that its later kernels would have cleared: what was
   // launched is waited for, and the next frame clears them first.
   vct_status encode(const FrameInputs& fi) {
+    if (!maps_ready) VCT_CHECK(alloc_maps((uint32_t)cfg.grid_res));  // (an earlier attempt found no memory)
     if (!counters_zero) VCT_CHECK(zero_counters());
     const vct_status s = encode_frame(fi);
     if (s == VCT_OK) return s;
