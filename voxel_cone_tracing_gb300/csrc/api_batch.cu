@@ -82,7 +82,7 @@ struct vct_batch {
   HeavyStore heavy;
   DevBuf<unsigned char> rbig;
   DevBuf<unsigned long long> rbig_count;
-  DevBuf<uint32_t> rbig_first;
+  DevBuf<unsigned long long> rbig_first;
   uint32_t rbig_cap = 0;
   DevBuf<unsigned long long> vis;
   DevBuf<float4> gb_pos, gb_nrm;

@@ -24,6 +24,7 @@
 #include "vct_internal.h"
 #include "vct_math.cuh"
 #include "vct_snap.h"
+#include "vct_tiles.h"
 
 namespace vct {
 namespace {
@@ -33,8 +34,6 @@ namespace {
 // 120,000 at 1367x771: 8 pixels 172 and 174 us, 16 129 and 96, 32 110 and 89,
 // 64 106 and 84.
 constexpr int kSmallPixels = 64;
-constexpr int kTileBits = 5;  // a large triangle's tile: 32x32 pixels of its box
-constexpr int kTile = 1 << kTileBits;
 constexpr int kAcross = 2;    // blocks of a row in flight
 constexpr int kSetup = 128;   // threads of a setup block
 constexpr float kGuard = 16.0f;
@@ -198,22 +197,22 @@ __device__ __forceinline__ void raster_subtri(const CV v[3], int W, int H, uint3
   // Records and tiles are counted in one word, so the first tiles ascend with
   // the records and need no scan.  The lanes with a single tile, most of them,
   // share one atomic.
-  r.tw = (uint32_t)(nx + kTile - 1) >> kTileBits;
-  const uint32_t tiles = r.tw * ((uint32_t)(ny + kTile - 1) >> kTileBits);
+  r.tw = tiles_across(r.x0, r.x1);
+  const uint32_t tiles = tiles_of(r.x0, r.y0, r.x1, r.y1);
   unsigned long long at;
   if (tiles == 1) {
     const unsigned m = __activemask();
     const int lane = threadIdx.x & 31, lead = __ffs((int)m) - 1;
     unsigned long long base = 0;
-    if (lane == lead) base = atomicAdd(rb.big_count, (1ull << 32 | 1ull) * (unsigned)__popc(m));
-    at = __shfl_sync(m, base, lead) + (1ull << 32 | 1ull) * (unsigned)__popc(m & ((1u << lane) - 1u));
+    if (lane == lead) base = atomicAdd(rb.big_count, big_count_of(1, 1) * (unsigned)__popc(m));
+    at = __shfl_sync(m, base, lead) + big_count_of(1, 1) * (unsigned)__popc(m & ((1u << lane) - 1u));
   } else {
-    at = atomicAdd(rb.big_count, 1ull << 32 | tiles);
+    at = atomicAdd(rb.big_count, big_count_of(1, tiles));
   }
-  const uint32_t slot = (uint32_t)(at >> 32);
+  const uint32_t slot = big_records(at);
   if (slot >= rb.big_cap) return;  // (reported; the frame is encoded again)
   reinterpret_cast<BigRec*>(rb.big)[slot] = r;
-  rb.big_first[slot] = (uint32_t)at;
+  rb.big_first[slot] = big_tiles(at);
 }
 
 // The clipped triangle's fan, called, not inlined: its polygons live in local
@@ -295,7 +294,8 @@ __global__ void __launch_bounds__(kSetup, 8) k_gb_setup_batch(BatchWork w, Raste
 
 // The last of n ascending values that is not above x (the first one is not),
 // found by a warp.
-__device__ __forceinline__ uint32_t warp_last_not_above(const uint32_t* __restrict__ v, uint32_t n, uint32_t x) {
+__device__ __forceinline__ uint32_t warp_last_not_above(const unsigned long long* __restrict__ v, uint32_t n,
+                                                        unsigned long long x) {
   const uint32_t lane = threadIdx.x & 31;
   uint32_t lo = 0, hi = n;
   while (hi - lo > 1) {
@@ -319,31 +319,35 @@ __device__ __forceinline__ uint32_t warp_last_not_above(const uint32_t* __restri
 // (64x64 tiles 155 us for all of the G-buffer, 32x32 210).
 __global__ void __launch_bounds__(256) k_gb_big(RasterBuffers rb, int W, const BatchScene* scenes) {
   follows_previous();
-  const uint32_t total = (uint32_t)*rb.big_count, records = (uint32_t)(*rb.big_count >> 32);
+  const uint32_t records = big_records(*rb.big_count), listed = min(records, rb.big_cap);
+  unsigned long long total = big_tiles(*rb.big_count);
   const int lane = threadIdx.x & 31;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     rb.status->big_total = records;
-    rb.status->big_tiles = total;
+    rb.status->big_tiles = (uint32_t)min(total, 0xffffffffull);
   }
-  if (!rb.big_cap) return;  // (no list: reported by big_total)
+  if (!listed) return;
+  if (listed < records) {  // a full list (reported by big_total): its records' tiles
+    const BigRec& last = reinterpret_cast<const BigRec*>(rb.big)[listed - 1];
+    total = rb.big_first[listed - 1] + tiles_of(last.x0, last.y0, last.x1, last.y1);
+  }
   // few tiles: up to 8 warps on one, each taking every so many-th row of blocks
   const uint32_t warps = gridDim.x * 8;
   int sh = 0;
   while (sh < 3 && total <= warps >> (sh + 1)) ++sh;
-  for (uint32_t j = blockIdx.x * 8 + (threadIdx.x >> 5); j >> sh < total; j += warps) {
-    const uint32_t t = j >> sh;
-    const int strip = (int)(j & ((1u << sh) - 1)) * 4, step = 4 << sh;
-    const uint32_t n = warp_last_not_above(rb.big_first, min(records, rb.big_cap), t);
-    // (past a full list's last record t lies below its box: no rows)
+  for (unsigned long long j = blockIdx.x * 8 + (threadIdx.x >> 5); j >> sh < total; j += warps) {
+    const unsigned long long t = j >> sh;
+    const int strip = (int)((unsigned)j & ((1u << sh) - 1)) * 4, step = 4 << sh;
+    const uint32_t n = warp_last_not_above(rb.big_first, listed, t);
     const BigRec r = reinterpret_cast<const BigRec*>(rb.big)[n];
-    const uint32_t lt = t - rb.big_first[n];
+    int x0, y0;
+    if (!tile_origin(t - rb.big_first[n], r.tw, r.x0, r.y0, r.y1, x0, y0)) continue;
     unsigned long long* vis = rb.vis;
     int w = W;
     if (scenes) {  // a batch: the record's scene
       vis += scenes[r.scene].px_base;
       w = scenes[r.scene].W;
     }
-    const int x0 = r.x0 + (int)(lt % r.tw) * kTile, y0 = r.y0 + (int)(lt / r.tw) * kTile;
     const int x1 = min(r.x1, x0 + kTile - 1), y1 = min(r.y1, y0 + kTile - 1);
     Edges<long long> e;
     e.at(r, x0, y0);

@@ -426,7 +426,7 @@ struct vct_renderer {
   DevBuf<unsigned long long> vis;
   DevBuf<unsigned char> big;
   DevBuf<unsigned long long> big_count;
-  DevBuf<uint32_t> big_first;
+  DevBuf<unsigned long long> big_first;
   uint32_t big_cap = 0;
   DevBuf<float4> gb_pos, gb_nrm;
   DevBuf<uchar4> frame;

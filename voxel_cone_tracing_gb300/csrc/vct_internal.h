@@ -83,7 +83,7 @@ struct SceneParams {
 struct FrameStatus {
   uint32_t pair_total;      // (triangle, brick) pairs needed
   uint32_t big_total;       // raster work records needed
-  uint32_t big_tiles;       // raster tiles of the big-triangle pass
+  uint32_t big_tiles;       // raster tiles of the big-triangle pass (at most 2^32 - 1)
   uint32_t rejected_tris;   // non-finite / out-of-range triangles
   uint32_t count_saturated; // voxels with > 65535 contributions
   uint32_t bigtri_total;    // large-triangle binning records needed
@@ -295,8 +295,8 @@ struct RasterBuffers {
   unsigned long long* vis;  // W*H (depth bits << 32 | triangle id)
   void* big;                // raster work records
   uint32_t big_cap;
-  unsigned long long* big_count;  // records << 32 | tiles; zero between frames
-  uint32_t* big_first;      // a record's first tile (big_cap)
+  unsigned long long* big_count;  // records and tiles (vct_tiles.h); zero between frames
+  unsigned long long* big_first;  // a record's first tile (big_cap)
   float4* gb_pos;           // world position, material id bits in .w
   float4* gb_nrm;           // world normal, triangle id bits in .w
   FrameStatus* status;
