@@ -22,6 +22,7 @@
 #include <vector>
 
 #include "renderer_state.h"
+#include "vct_snap.h"
 
 namespace {
 
@@ -341,7 +342,7 @@ struct vct_batch {
 namespace {
 
 vct_status check_scene(const vct_batch_scene& d, uint32_t i) {
-  if (d.width < 1 || d.height < 1 || d.width > 16384 || d.height > 16384)
+  if (d.width < 1 || d.height < 1 || d.width > kSnapPixels || d.height > kSnapPixels)
     return set_error(VCT_ERR_INVALID_VALUE, "scene %u: frame %dx%d", i, d.width, d.height);
   if (!is_pow2((uint32_t)d.grid_res) || d.grid_res < 16 || d.grid_res > 256)
     return set_error(VCT_ERR_INVALID_VALUE, "scene %u: grid_res %d (need a power of two in [16, 256])", i,

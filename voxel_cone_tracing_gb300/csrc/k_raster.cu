@@ -20,6 +20,7 @@
 //                  visible triangle -> world position, interpolated world
 //                  normal (not renormalised), material id.
 #include <algorithm>
+#include <type_traits>
 
 #include "vct_internal.h"
 #include "vct_math.cuh"
@@ -145,51 +146,66 @@ __device__ __forceinline__ void raster_box(const BigRec& r, unsigned long long* 
   }
 }
 
-// 1/256-pixel coordinate of normalised device coordinate n on K / 128 pixels.
-__device__ __forceinline__ int snap_ndc(float n, int K) {
-  bool close;
-  const int v = snap_scaled(n, (uint32_t)K, close);
-  if (!close) return v;
-  return (int)__double2ll_rn(__dmul_rn(__dadd_rn((double)n, 1.0), (double)K));
+// Screen coordinates while a triangle is set up: 32 bits hold those of a frame
+// within kSnapPixels each way (|n| <= 64: below 2^28, their differences too).
+template <bool WIDE>
+using Coord = typename std::conditional<WIDE, long long, int>::type;
+
+// 1/256-pixel coordinate of normalised device coordinate n on `pixels` pixels.
+template <bool WIDE>
+__device__ __forceinline__ Coord<WIDE> snap_ndc(float n, int pixels) {
+  if constexpr (!WIDE) {
+    bool close;
+    const int v = snap_scaled(n, (uint32_t)pixels * 128u, close);
+    if (!close) return v;
+  }
+  return (Coord<WIDE>)__double2ll_rn(__dmul_rn(__dadd_rn((double)n, 1.0), (double)pixels * 128.0));
 }
 
 // Set up one (possibly clipped) screen triangle; raster it here if small.
+template <bool WIDE>
 __device__ __forceinline__ void raster_subtri(const CV v[3], int W, int H, uint32_t tri, const RasterBuffers& rb,
                                               uint32_t scene) {
+  typedef Coord<WIDE> C;
   BigRec r;
+  C X[3], Y[3];
   for (int k = 0; k < 3; ++k) {
     if (!(v[k].c[3] > 0.0f)) return;
     const float nx = rdiv(v[k].c[0], v[k].c[3]), ny = rdiv(v[k].c[1], v[k].c[3]), nz = rdiv(v[k].c[2], v[k].c[3]);
     if (!(fabsf(nx) <= 64.0f) || !(fabsf(ny) <= 64.0f) || !(nz == nz)) return;
-    r.X[k] = snap_ndc(nx, W * 128);
-    r.Y[k] = snap_ndc(ny, H * 128);
+    X[k] = snap_ndc<WIDE>(nx, W);
+    Y[k] = snap_ndc<WIDE>(ny, H);
     r.z[k] = radd(rmul(0.5f, nz), 0.5f);
   }
-  const long long ax = r.X[1] - r.X[0], ay = r.Y[1] - r.Y[0], bx = r.X[2] - r.X[0], by = r.Y[2] - r.Y[0];
+  const long long ax = X[1] - X[0], ay = Y[1] - Y[0], bx = X[2] - X[0], by = Y[2] - Y[0];
   long long area = ax * by - ay * bx;
   if (area == 0) return;
   if (area < 0) {
-    int t = r.X[1]; r.X[1] = r.X[2]; r.X[2] = t;
-    t = r.Y[1]; r.Y[1] = r.Y[2]; r.Y[2] = t;
+    C t = X[1]; X[1] = X[2]; X[2] = t;
+    t = Y[1]; Y[1] = Y[2]; Y[2] = t;
     float tz = r.z[1]; r.z[1] = r.z[2]; r.z[2] = tz;
     area = -area;
   }
   // the pixels whose centres (256 p + 128) lie in the box
-  const int minx = min(r.X[0], min(r.X[1], r.X[2])), maxx = max(r.X[0], max(r.X[1], r.X[2]));
-  const int miny = min(r.Y[0], min(r.Y[1], r.Y[2])), maxy = max(r.Y[0], max(r.Y[1], r.Y[2]));
-  r.x0 = max(0, (minx + 127) >> 8);
-  r.x1 = min(W - 1, (maxx - 128) >> 8);
-  r.y0 = max(0, (miny + 127) >> 8);
-  r.y1 = min(H - 1, (maxy - 128) >> 8);
+  const C minx = min(X[0], min(X[1], X[2])), maxx = max(X[0], max(X[1], X[2]));
+  const C miny = min(Y[0], min(Y[1], Y[2])), maxy = max(Y[0], max(Y[1], Y[2]));
+  r.x0 = (int)max((C)0, (minx + 127) >> 8);
+  r.x1 = (int)min((C)(W - 1), (maxx - 128) >> 8);
+  r.y0 = (int)max((C)0, (miny + 127) >> 8);
+  r.y1 = (int)min((C)(H - 1), (maxy - 128) >> 8);
   if (r.x1 < r.x0 || r.y1 < r.y0) return;
+  for (int k = 0; k < 3; ++k) {
+    r.X[k] = (int)X[k];
+    r.Y[k] = (int)Y[k];
+  }
   r.farea = __ll2float_rn(area);
-  r.tl = (top_left(r.X[1], r.Y[1], r.X[2], r.Y[2]) ? 1 : 0) | (top_left(r.X[2], r.Y[2], r.X[0], r.Y[0]) ? 2 : 0) |
-         (top_left(r.X[0], r.Y[0], r.X[1], r.Y[1]) ? 4 : 0);
+  r.tl = (top_left(X[1], Y[1], X[2], Y[2]) ? 1 : 0) | (top_left(X[2], Y[2], X[0], Y[0]) ? 2 : 0) |
+         (top_left(X[0], Y[0], X[1], Y[1]) ? 4 : 0);
   r.tri = tri;
   const int nx = r.x1 - r.x0 + 1, ny = r.y1 - r.y0 + 1;
   if (nx * ny <= kSmallPixels) {
     // (within 2^14 the products of two differences stay below 2^29)
-    if (maxx - minx <= (1 << 14) && maxy - miny <= (1 << 14)) raster_box<int>(r, rb.vis, W);
+    if (!WIDE && maxx - minx <= (1 << 14) && maxy - miny <= (1 << 14)) raster_box<int>(r, rb.vis, W);
     else raster_box<long long>(r, rb.vis, W);
     return;
   }
@@ -217,6 +233,7 @@ __device__ __forceinline__ void raster_subtri(const CV v[3], int W, int H, uint3
 
 // The clipped triangle's fan, called, not inlined: its polygons live in local
 // memory, and few triangles need it.
+template <bool WIDE>
 __device__ __noinline__ void raster_clipped(const CV cv[3], int W, int H, uint32_t t, const RasterBuffers& rb,
                                             uint32_t scene) {
   CV a[10], b[10];
@@ -245,10 +262,11 @@ __device__ __noinline__ void raster_clipped(const CV cv[3], int W, int H, uint32
 #pragma unroll 1
   for (int k = 1; k + 1 < n; ++k) {
     const CV tri3[3] = {a[0], a[k], a[k + 1]};
-    raster_subtri(tri3, W, H, t, rb, scene);
+    raster_subtri<WIDE>(tri3, W, H, t, rb, scene);
   }
 }
 
+template <bool WIDE>
 __device__ __forceinline__ void setup_tri(const SceneParams& sp, const CameraParams& cp, const RasterBuffers& rb,
                                           uint32_t t, uint32_t scene) {
   if (t >= sp.total_tris) return;
@@ -261,8 +279,8 @@ __device__ __forceinline__ void setup_tri(const SceneParams& sp, const CameraPar
   for (int pl = 0; pl < 5; ++pl)
     for (int k = 0; k < 3; ++k)
       if (!(plane_eval(pl, cv[k]) >= 0.0f)) all_in = false;
-  if (all_in) raster_subtri(cv, cp.W, cp.H, t, rb, scene);
-  else raster_clipped(cv, cp.W, cp.H, t, rb, scene);
+  if (all_in) raster_subtri<WIDE>(cv, cp.W, cp.H, t, rb, scene);
+  else raster_clipped<WIDE>(cv, cp.W, cp.H, t, rb, scene);
 }
 
 // Latency of the instance, index and vertex loads, so registers decide (64: 32
@@ -270,9 +288,11 @@ __device__ __forceinline__ void setup_tri(const SceneParams& sp, const CameraPar
 // small boxes take 32-bit stepped edge functions and fire-and-forget atomics
 // (reading the visibility word first, to skip the atomic, stalled on every
 // pixel); the clipper is a call.  500,000 triangles, 1920x1080: 86 us with
-// FP64 and the clipper inline (98 registers), 38 now.
+// FP64 and the clipper inline (98 registers), 38 now.  WIDE (snap_wide): with
+// FP64 and 64-bit coordinates.
+template <bool WIDE>
 __global__ void __launch_bounds__(kSetup, 8) k_gb_setup(SceneParams sp, CameraParams cp, RasterBuffers rb) {
-  setup_tri(sp, cp, rb, blockIdx.x * blockDim.x + threadIdx.x, 0u);
+  setup_tri<WIDE>(sp, cp, rb, blockIdx.x * blockDim.x + threadIdx.x, 0u);
 }
 
 // The pixel slice of one batch scene in the batch-wide raster buffers.
@@ -284,11 +304,12 @@ __device__ __forceinline__ RasterBuffers scene_rb(const RasterBuffers& rb, const
   return r;
 }
 
+// (a batch's frames are within kSnapPixels)
 __global__ void __launch_bounds__(kSetup, 8) k_gb_setup_batch(BatchWork w, RasterBuffers rb) {
   for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < w.total; g += gridDim.x * blockDim.x) {
     const int s = batch_scene_of(w, g);
     const BatchScene& S = w.scenes[s];
-    setup_tri(S.sp, w.cams[s], scene_rb(rb, S), g - __ldg(w.prefix + s), (uint32_t)s);
+    setup_tri<false>(S.sp, w.cams[s], scene_rb(rb, S), g - __ldg(w.prefix + s), (uint32_t)s);
   }
 }
 
@@ -459,7 +480,10 @@ cudaError_t launch_gbuffer(const SceneParams& sp, const CameraParams& cp, const 
                            int* launches) {
   cudaError_t e = cudaMemsetAsync(rb.vis, 0xff, (size_t)cp.W * cp.H * sizeof(unsigned long long), st);
   if (e != cudaSuccess) return e;
-  if (sp.total_tris) k_gb_setup<<<(sp.total_tris + kSetup - 1) / kSetup, kSetup, 0, st>>>(sp, cp, rb);
+  if (sp.total_tris) {
+    auto setup = snap_wide(cp.W, cp.H) ? k_gb_setup<true> : k_gb_setup<false>;
+    setup<<<(sp.total_tris + kSetup - 1) / kSetup, kSetup, 0, st>>>(sp, cp, rb);
+  }
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

@@ -59,7 +59,11 @@ VCT_SNAP_HD inline long long snap_fixed(float g, int k) {
 // value is K + m K / 2^s, m K below 2^45; FP64's own rounding moves it by less
 // than 2^-24, so an integer shift rounds alike unless the fraction is that near
 // one half.  `close` reports such a value (and returns nothing of use): the
-// caller then rounds in FP64.
+// caller then rounds in FP64.  A frame wider or higher than kSnapPixels is
+// snapped in FP64 throughout (snap_wide): there FP64's own rounding reaches
+// past that band, and coordinates and their differences past 32 bits.
+constexpr int kSnapPixels = 1 << 14;
+inline bool snap_wide(int W, int H) { return W > kSnapPixels || H > kSnapPixels; }
 VCT_SNAP_HD inline int snap_scaled(float g, uint32_t K, bool& close) {
 #ifdef __CUDA_ARCH__
   const uint32_t bits = __float_as_uint(g);
