@@ -132,3 +132,29 @@ def test_what_could_not_be_allocated_is_not_used(tmp_path):
     assert lists and all(cap == "0" for _, cap in lists)
     assert not any(x.startswith("launch") for x in out["without maps"])
     assert any(x.startswith("malloc3d") for x in out["with maps"]) and out["grid"] == 64
+
+
+def test_a_kernel_has_one_shared_memory_limit(tmp_path):
+    """The limit of a kernel's dynamic shared memory belongs to the process:
+    were it set to what a call needs, a renderer on one thread could lower it
+    between another's setting and launch.  So every call sets the same."""
+    out = run(tmp_path, """
+        rng = np.random.default_rng(0)
+        rows = rng.random((1 << 15, 12), dtype=np.float32)
+        r = R.Renderer(16, 16, grid_res=16)
+        for log2 in (8, 13, 15, 17):
+            r.mlp_init(R.mlp_desc(log2_table=log2))
+            r.mlp_train_samples(rows, R.mlp_desc(log2_table=log2, steps=1))
+            r.mlp_eval(rows[:100])
+        take("train")
+    """)["train"]
+    limits, need = {}, {}
+    for line in out:
+        w = line.split()
+        if w[0] == "attribute":
+            limits.setdefault(w[1], set()).add(int(w[3]))
+        if w[0] == "launch" and int(w[3]) > 48 << 10:
+            need[w[1]] = max(need.get(w[1], 0), int(w[3]))
+    assert any("encode_smem" in k for k in need)
+    for k, n in need.items():
+        assert len(limits[k]) == 1 and n <= min(limits[k]), (k, limits[k], n)

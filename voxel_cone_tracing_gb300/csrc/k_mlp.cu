@@ -1032,7 +1032,9 @@ cudaError_t launch_mlp_train(const MlpParams& p, const MlpBatch& b, uint32_t* wo
   while (b.n >= kSmemRows && in_smem < kMlpLevels && level_entries(p, in_smem) <= kSmemEntries)
     tab = std::max(tab, (size_t)((level_entries(p, in_smem++) + 3) / 4 * 16));
   if (in_smem) {
-    e = cudaFuncSetAttribute(k_mlp_encode_smem, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tab);
+    // (the limit is the process's, so that of the largest level, not of this call's)
+    e = cudaFuncSetAttribute(k_mlp_encode_smem, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)(kSmemEntries * sizeof(uint32_t)));
     if (e != cudaSuccess) return e;
     const int per_sm = std::max(1, std::min(2, (int)(220 * 1024 / (tab + 1024))));
     const dim3 grid((unsigned)std::max(1, sm_count() * per_sm / in_smem), (unsigned)in_smem);
