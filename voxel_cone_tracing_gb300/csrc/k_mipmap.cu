@@ -570,17 +570,17 @@ __device__ __forceinline__ bool occ_raw_cell(const MapSet& ms, int c, int x, int
     for (int dy = 0; dy < f; ++dy) {
       const uint8_t* row = ms.occ_raw[k] + ((size_t)(z * f + dz) * sk + (y * f + dy)) * sk + (size_t)x * f;
       if (f == 4) {
-        any |= __ldg(reinterpret_cast<const uint32_t*>(row));  // 4-byte aligned: x * 4
+        any |= *reinterpret_cast<const uint32_t*>(row);  // 4-byte aligned: x * 4
       } else if (f == 8) {
-        const uint2 v = __ldg(reinterpret_cast<const uint2*>(row));  // 8-byte aligned: x * 8
+        const uint2 v = *reinterpret_cast<const uint2*>(row);  // 8-byte aligned: x * 8
         any |= v.x | v.y;
       } else if (f >= 16) {  // 16-byte aligned: x * f, and every row of level k holds a multiple of 16 bytes
         for (int dx = 0; dx < f; dx += 16) {
-          const uint4 v = __ldg(reinterpret_cast<const uint4*>(row + dx));
+          const uint4 v = *reinterpret_cast<const uint4*>(row + dx);
           any |= v.x | v.y | v.z | v.w;
         }
       } else {
-        for (int dx = 0; dx < f; ++dx) any |= __ldg(row + dx);
+        for (int dx = 0; dx < f; ++dx) any |= row[dx];
       }
     }
   return any != 0u;
@@ -597,7 +597,7 @@ __device__ void occ_pack_word(const MapSet& ms, int c, uint32_t w) {
     const uint4* r = reinterpret_cast<const uint4*>(ms.occ_raw[c] + ((size_t)z * s + y) * s + x0);
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
-      const uint4 v4 = __ldg(r + j);
+      const uint4 v4 = r[j];
       const uint32_t v[4] = {v4.x, v4.y, v4.z, v4.w};
 #pragma unroll
       for (int i = 0; i < 4; ++i)

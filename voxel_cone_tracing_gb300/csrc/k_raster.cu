@@ -315,13 +315,13 @@ __global__ void __launch_bounds__(kSetup, 8) k_gb_setup_batch(BatchWork w, Raste
 
 // The last of n ascending values that is not above x (the first one is not),
 // found by a warp.
-__device__ __forceinline__ uint32_t warp_last_not_above(const unsigned long long* __restrict__ v, uint32_t n,
+__device__ __forceinline__ uint32_t warp_last_not_above(const unsigned long long* v, uint32_t n,
                                                         unsigned long long x) {
   const uint32_t lane = threadIdx.x & 31;
   uint32_t lo = 0, hi = n;
   while (hi - lo > 1) {
     const uint32_t step = (hi - lo + 31) / 32, i = lo + lane * step;
-    const unsigned below = __ballot_sync(0xffffffffu, i < hi && __ldg(v + i) <= x);
+    const unsigned below = __ballot_sync(0xffffffffu, i < hi && v[i] <= x);
     lo += (31 - __clz((int)below)) * step;
     hi = min(hi, lo + step);
   }

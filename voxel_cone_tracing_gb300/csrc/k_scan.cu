@@ -44,7 +44,7 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t& excl) 
   return r;
 }
 
-__global__ void __launch_bounds__(kT) k_scan_tiles(const uint32_t* __restrict__ in, uint32_t* __restrict__ out,
+__global__ void __launch_bounds__(kT) k_scan_tiles(const uint32_t* in, uint32_t* __restrict__ out,
                                                    uint32_t* __restrict__ tile_tot, size_t n, ScanFuse fuse) {
   follows_previous();
   if (blockIdx.x == 0) {  // the counters of the plan and of the list, before k_scan_add
@@ -70,9 +70,9 @@ __global__ void __launch_bounds__(kT) k_scan_tiles(const uint32_t* __restrict__ 
 // Adds each tile the totals of those before it (every CTA sums them itself:
 // at most a few hundred words, against a launch of its own), and plans the
 // bricks.
-__global__ void __launch_bounds__(256) k_scan_add(uint32_t* __restrict__ in, uint32_t* __restrict__ out,
+__global__ void __launch_bounds__(256) k_scan_add(uint32_t* in, uint32_t* out,
                                                   uint32_t* __restrict__ copy_out,
-                                                  const uint32_t* __restrict__ tile_tot, uint32_t ntiles, size_t n,
+                                                  const uint32_t* tile_tot, uint32_t ntiles, size_t n,
                                                   ScanFuse fuse) {
   follows_previous();
   __shared__ uint32_t s_before[8], s_all[8];

@@ -278,7 +278,7 @@ __global__ void __launch_bounds__(kMarchWarps * 32, VCT_MARCH_MIN_BLOCKS)
 // test (with its occupancy load) run while this cone's fetches are in flight.
 template <bool ISO>
 __device__ __forceinline__ V3 shared_diffuse(const MapSet& m, int cone_set, V3 pos, V3 n,
-                                             const float4* __restrict__ far, const ConeStep& first,
+                                             const float4* far, const ConeStep& first,
                                              const ConeRing& ring) {
   const int K = cone_set == VCT_CONES_SIX60 ? 6 : 9;
   const V3 o1 = normalize(tangent(n));
@@ -339,7 +339,7 @@ template <bool ISO, bool SHARE>
 __global__ void __launch_bounds__(256, SHARE ? VCT_SHADE_MIN_BLOCKS : 6)
     k_shade(SceneParams sp, CameraParams cp, const __grid_constant__ MapSet m, TraceParams tp,
             const float4* __restrict__ gb_pos, const float4* __restrict__ gb_nrm, uchar4* __restrict__ frame,
-            float4* __restrict__ frame_f32, TraceWork tw, const float4* __restrict__ diffuse,
+            float4* __restrict__ frame_f32, TraceWork tw, const float4* diffuse,
             const __grid_constant__ ConeStep first, const __grid_constant__ ConeRing ring) {
   follows_previous();  // (the maps it samples were whole before k_march)
   int px, py;

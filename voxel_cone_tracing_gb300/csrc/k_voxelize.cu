@@ -187,8 +187,8 @@ __device__ __forceinline__ bool touches_brick(const float v[3][3], int bx, int b
 // One (triangle, candidate brick) pair of the binning passes.
 template <bool FILL>
 __device__ __forceinline__ void bin_one(const float v[3][3], int bx, int by, int bz, int nb, uint32_t t,
-                                        uint32_t* __restrict__ count, uint32_t* __restrict__ cursor,
-                                        uint32_t* __restrict__ list, uint32_t cap) {
+                                        uint32_t* count, uint32_t* cursor, uint32_t* __restrict__ list,
+                                        uint32_t cap) {
   if (!touches_brick(v, bx, by, bz)) return;
   const uint32_t brick = ((uint32_t)bz * nb + by) * nb + bx;
   if (FILL) {
@@ -218,10 +218,9 @@ constexpr uint32_t kRecAgain = 1u << 31;
 // All 32 lanes of a warp call it together (each with its own triangle t of
 // the same scene; t >= total_tris is an idle lane).
 template <bool FILL>
-__device__ __forceinline__ void bin_tri(const SceneParams& sp, int N, uint32_t t, uint32_t* __restrict__ count,
-                                        uint32_t* __restrict__ cursor, uint32_t* __restrict__ list, uint32_t cap,
-                                        FrameStatus* st, BinRec* __restrict__ big, uint32_t big_cap,
-                                        uint32_t* __restrict__ big_count, uint32_t scene, uint2* __restrict__ rec,
+__device__ __forceinline__ void bin_tri(const SceneParams& sp, int N, uint32_t t, uint32_t* count, uint32_t* cursor,
+                                        uint32_t* __restrict__ list, uint32_t cap, FrameStatus* st, BinRec* big,
+                                        uint32_t big_cap, uint32_t* big_count, uint32_t scene, uint2* __restrict__ rec,
                                         TriRec* __restrict__ recs) {
   const int lane = threadIdx.x & 31;
   const int nb = N / kBrick;
@@ -336,10 +335,9 @@ __device__ __forceinline__ void bin_tri(const SceneParams& sp, int N, uint32_t t
 }
 
 template <bool FILL>
-__global__ void __launch_bounds__(256) k_bin(SceneParams sp, int N, uint32_t* __restrict__ count,
-                                             uint32_t* __restrict__ cursor, uint32_t* __restrict__ list,
-                                             uint32_t cap, FrameStatus* st, BinRec* __restrict__ big,
-                                             uint32_t big_cap, uint32_t* __restrict__ big_count,
+__global__ void __launch_bounds__(256) k_bin(SceneParams sp, int N, uint32_t* count, uint32_t* cursor,
+                                             uint32_t* __restrict__ list, uint32_t cap, FrameStatus* st,
+                                             BinRec* big, uint32_t big_cap, uint32_t* big_count,
                                              uint2* __restrict__ rec, TriRec* __restrict__ recs) {
   follows_previous();
   bin_tri<FILL>(sp, N, blockIdx.x * blockDim.x + threadIdx.x, count, cursor, list, cap, st, big, big_cap, big_count,
@@ -366,9 +364,9 @@ __global__ void __launch_bounds__(256) k_bin_batch(BatchWork w, BatchBuffers bb)
 // the candidate bricks y*256 + tid, stepping by kBigSplit*256.  With
 // `scenes` (a batch) each record bins into its own scene's brick slice.
 template <bool FILL>
-__global__ void __launch_bounds__(256) k_bin_big(int N, const BinRec* __restrict__ big, uint32_t big_cap,
-                                                 const uint32_t* __restrict__ big_count, uint32_t* __restrict__ count,
-                                                 uint32_t* __restrict__ cursor, uint32_t* __restrict__ list,
+__global__ void __launch_bounds__(256) k_bin_big(int N, const BinRec* big, uint32_t big_cap,
+                                                 const uint32_t* big_count, uint32_t* count, uint32_t* cursor,
+                                                 uint32_t* __restrict__ list,
                                                  uint32_t cap, const BatchScene* __restrict__ scenes) {
   follows_previous();
   const uint32_t n = min(*big_count, big_cap);
@@ -814,7 +812,7 @@ static_assert(kRound <= 128, "a queue entry holds the pair in 7 bits");
 // the pairs' loads and setup, a quarter shading.)
 template <int MODE, int STORAGE, bool REC>
 __device__ __forceinline__ void brick_accumulate(const SceneParams& sp, const TriRec* __restrict__ recs, int N, const int b3[3],
-                                                 const uint32_t* __restrict__ list, uint32_t beg, uint32_t end,
+                                                 const uint32_t* list, uint32_t beg, uint32_t end,
                                                  AccT<STORAGE>& acc, RoundOf<MODE>& rd) {
   for (int i = threadIdx.x; i < kBrickVox; i += kThreads) acc.clear(i);
   __syncthreads();
@@ -824,7 +822,7 @@ __device__ __forceinline__ void brick_accumulate(const SceneParams& sp, const Tr
     const uint32_t n = min((uint32_t)kRound, end - b0);
     int cnt = 0;
     if ((uint32_t)threadIdx.x < n) {
-      const uint32_t t = __ldg(list + b0 + threadIdx.x);
+      const uint32_t t = list[b0 + threadIdx.x];
       if constexpr (MODE == VCT_VOX_CONSERVATIVE) cnt = setup_sat<REC>(sp, recs, N, t, b3, rd.setup[threadIdx.x]);
       else cnt = setup_ref<REC>(sp, recs, N, t, b3, rd.setup[threadIdx.x]);
     }
@@ -1104,7 +1102,7 @@ __device__ __forceinline__ void brick_coords(int N, uint32_t brick, int b3[3]) {
 // so that its code exists once per kernel (instruction-cache footprint).
 template <int MODE, int STORAGE, bool SURF = true, bool REC = true>
 __device__ __forceinline__ void brick_unit(const SceneParams& sp, const TriRec* __restrict__ recs, int N, uint32_t brick,
-                                           const uint32_t* __restrict__ offset, const uint32_t* __restrict__ list,
+                                           const uint32_t* offset, const uint32_t* list,
                                            uint32_t cap, cudaSurfaceObject_t l0, uint32_t* __restrict__ counts,
                                            FrameStatus* st, AccT<STORAGE>& acc, RoundOf<MODE>& rd, const InjGrids& inj, void* l0_lin,
                                            const HeavyBricks* hb, uint32_t slot_index, uint32_t chunk, bool item,
@@ -1213,8 +1211,8 @@ __device__ __forceinline__ void for_units(const HeavyBricks& hb, const BrickUnit
 
 // (FUSE: with the fused mips.)
 template <int MODE, int STORAGE, bool FUSE = false>
-__global__ void __launch_bounds__(kThreads, brick_min_blocks<STORAGE>()) k_bricks(SceneParams sp, int N, const uint32_t* __restrict__ offset,
-                                                     const uint32_t* __restrict__ list, uint32_t cap,
+__global__ void __launch_bounds__(kThreads, brick_min_blocks<STORAGE>()) k_bricks(SceneParams sp, int N, const uint32_t* offset,
+                                                     const uint32_t* list, uint32_t cap,
                                                      cudaSurfaceObject_t l0, uint32_t* __restrict__ counts,
                                                      FrameStatus* st, InjGrids inj, void* l0_lin, HeavyBricks hb,
                                                      BrickUnits units, const TriRec* __restrict__ recs,
@@ -1259,7 +1257,7 @@ unsigned resident_grid(K kern, int threads, size_t smem, int sms, int per_sm, ui
 // instead of a surface: the output of vct_voxelize_noalloc.
 template <int MODE>
 __global__ void __launch_bounds__(kThreads, 7)
-    k_bricks_linear(SceneParams sp, int N, const uint32_t* __restrict__ offset, const uint32_t* __restrict__ list,
+    k_bricks_linear(SceneParams sp, int N, const uint32_t* offset, const uint32_t* list,
                     uint32_t cap, uchar4* __restrict__ out, FrameStatus* st, HeavyBricks hb, BrickUnits units) {
   __shared__ Acc acc;
   __shared__ __align__(8) RoundOf<MODE> rd;

@@ -668,7 +668,7 @@ __device__ __forceinline__ void light_dir(const SceneParams& sp, int i, V3 pos, 
 // light, `stride` apart), else they are traced here.
 template <int SAMPLER, bool ISO, int STORAGE, bool SPLIT>
 __device__ V3 direct_light(const SceneParams& sp, const MapSet& m, int enable_shadow, const vct_material_data& mat,
-                           V3 pos, V3 nrm, V3 view_dir, const float* __restrict__ occlusion, size_t stride) {
+                           V3 pos, V3 nrm, V3 view_dir, const float* occlusion, size_t stride) {
   V3 result = v3(0.f, 0.f, 0.f);
   const int nl = min(sp.n_lights, kMaxLights);
   for (int i = 0; i < nl; ++i) {

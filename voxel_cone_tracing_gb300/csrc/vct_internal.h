@@ -16,7 +16,9 @@ namespace vct {
 // kernel's CTAs in early, as well, cost the raster that runs beside: they hold
 // their places while they wait.)  Not for a kernel that reads a texture or
 // surface which the kernel before it writes: those are coherent across whole
-// launches.
+// launches.  And what the kernel before it writes is read by plain loads: a
+// __restrict__ pointer or __ldg promises data that is constant for the kernel's
+// whole life, so such a load could be moved above the wait.
 template <class... P, class... A>
 cudaError_t launch_next(void (*kern)(P...), dim3 grid, unsigned threads, cudaStream_t st, A... args) {
   cudaLaunchAttribute a = {};
