@@ -117,6 +117,7 @@ template <bool ISO>
 __device__ __forceinline__ void march_far(float cube_size, const MapSet& m, const MarchPlan& mp, int tx, int ty, int k,
                                           const float4* __restrict__ gb_pos, const float4* __restrict__ gb_nrm,
                                           float4* __restrict__ far, const ConeSchedule& sched, const ConeRing& ring) {
+  static_assert(trace_far_slots(16, 16) == 32 * 9, "a lane for each group of a tile");
   const int lane = threadIdx.x & 31;
   const int gx = tx * (16 / kShareW) + lane % (16 / kShareW), gy = ty * 8 + lane / (16 / kShareW);
   const int groups_x = (mp.W + kShareW - 1) / kShareW;
@@ -209,6 +210,7 @@ __global__ void __launch_bounds__(kMarchWarps * 32, VCT_MARCH_MIN_BLOCKS)
   }
   if (SHARE) r -= (unsigned)K;
   const int w = (int)(r & 7u);
+  static_assert(kShareWarpW == 8, "group_share's lanes are these pixels");
   const int px = tx * 16 + (w & 1) * 8 + (lane & 7), py = ty * 16 + (w >> 1) * 4 + (lane >> 3);
   const size_t p = (size_t)py * mp.W + px;
   bool valid = false;

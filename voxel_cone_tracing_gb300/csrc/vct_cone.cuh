@@ -615,12 +615,7 @@ __device__ __forceinline__ V3 mixv(V3 a, V3 b, float t) { return a * (1.0f - t) 
 // ---- groups that share far fields -------------------------------------------
 constexpr float kShareCos = 0.99f;
 constexpr float kShareDist = 2.0f;  // voxels
-#ifndef VCT_SHARE_GROUP_W
-#define VCT_SHARE_GROUP_W 4
-#endif
-// A sharing group is kShareW x 2 pixels of a warp's 8x4-pixel block.
-constexpr int kShareW = VCT_SHARE_GROUP_W;
-static_assert(kShareW == 2 || kShareW == 4 || kShareW == 8, "group width divides the 8-pixel block row");
+// (A sharing group: kShareW x 2 pixels of a warp's block.)
 
 // Direction (unnormalised) and aperture of diffuse cone k, as trace_diffuse
 // computes them from the normal n and its frame o1, o2.
@@ -721,15 +716,8 @@ __device__ __forceinline__ unsigned char unorm8(float v) {
 // The pixel of this lane in a 16-pixel-wide CTA tile at (x0, y0) of the
 // shared-far-field kernels: a warp is a kShareWarpW x (32 / kShareWarpW)
 // block (lane = x + kShareWarpW y), 16 / kShareWarpW blocks per row of
-// blocks.  (Measured on the 1080p bench frame, trace ms: 16 x 2 strips
-// 1.235, 8 x 4 blocks 1.217, 4 x 8 blocks 1.221; the same frame: the
-// groups are the same aligned kShareW x 2 pixels whatever the block.)
-#ifndef VCT_SHARE_WARP_W
-#define VCT_SHARE_WARP_W 8
-#endif
-constexpr int kShareWarpW = VCT_SHARE_WARP_W;
-static_assert((kShareWarpW == 4 || kShareWarpW == 8 || kShareWarpW == 16) && kShareWarpW % kShareW == 0,
-              "a warp block holds whole groups");
+// blocks.  (One kernel with every phase inside, on the 1920x1080 bench frame,
+// trace ms: 16 x 2 strips 1.235, 8 x 4 blocks 1.217, 4 x 8 blocks 1.221.)
 __device__ __forceinline__ void share_tile_px(int x0, int y0, int& px, int& py) {
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   px = x0 + (w % (16 / kShareWarpW)) * kShareWarpW + lane % kShareWarpW;

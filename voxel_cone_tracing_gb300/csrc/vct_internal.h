@@ -324,6 +324,12 @@ struct TraceParams {
   int far_share;
 };
 
+// The layout of the shared far fields, one for every kernel and buffer that
+// holds them: a warp's block of kShareWarpW x (32 / kShareWarpW) pixels is made
+// of groups of kShareW x 2 pixels.
+constexpr int kShareW = 4, kShareWarpW = 8;
+static_assert(kShareWarpW % kShareW == 0 && 32 / kShareWarpW % 2 == 0, "a warp's block holds whole groups");
+
 // Work arrays between the passes of one frame's trace (launch_trace).  Every
 // frame that may be in flight at the same time has its own.
 struct TraceWork {
@@ -333,7 +339,9 @@ struct TraceWork {
   float4* refracted;  // W * H: the refracted cone
   float* shadow;      // W * H per light: occlusion of its shadow cone
 };
-inline size_t trace_far_slots(int W, int H) { return (size_t)((W + 3) / 4) * (size_t)((H + 1) / 2) * 9; }
+constexpr size_t trace_far_slots(int W, int H) {  // nine cones a group
+  return (size_t)((W + kShareW - 1) / kShareW) * (size_t)((H + 1) / 2) * 9;
+}
 
 // ---- batched rendering (api_batch.cu) --------------------------------------
 // One scene of a batch, device-resident.  Scenes own their voxel maps; the
