@@ -110,6 +110,8 @@ struct MarchPlan {
   int cone_set;
 };
 
+static_assert(trace_far_slots(16, 16) == 32 * 9, "march_far: a lane for each group of a tile");
+
 // The far field of one cone of a tile's 32 groups: lane = group, marched in
 // lockstep, so that the lanes read neighbouring texels of the same maps at
 // the same step of the schedule.
@@ -117,7 +119,6 @@ template <bool ISO>
 __device__ __forceinline__ void march_far(float cube_size, const MapSet& m, const MarchPlan& mp, int tx, int ty, int k,
                                           const float4* __restrict__ gb_pos, const float4* __restrict__ gb_nrm,
                                           float4* __restrict__ far, const ConeSchedule& sched, const ConeRing& ring) {
-  static_assert(trace_far_slots(16, 16) == 32 * 9, "a lane for each group of a tile");
   const int lane = threadIdx.x & 31;
   const int gx = tx * (16 / kShareW) + lane % (16 / kShareW), gy = ty * 8 + lane / (16 / kShareW);
   const int groups_x = (mp.W + kShareW - 1) / kShareW;
