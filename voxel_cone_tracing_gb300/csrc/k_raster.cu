@@ -154,12 +154,15 @@ using Coord = typename std::conditional<WIDE, long long, int>::type;
 // 1/256-pixel coordinate of normalised device coordinate n on `pixels` pixels.
 template <bool WIDE>
 __device__ __forceinline__ Coord<WIDE> snap_ndc(float n, int pixels) {
-  if constexpr (!WIDE) {
+  if constexpr (WIDE) {
+    return __double2ll_rn(__dmul_rn(__dadd_rn((double)n, 1.0), (double)pixels * 128.0));
+  } else {
+    const int K = pixels * 128;
     bool close;
-    const int v = snap_scaled(n, (uint32_t)pixels * 128u, close);
+    const int v = snap_scaled(n, (uint32_t)K, close);
     if (!close) return v;
+    return (int)__double2ll_rn(__dmul_rn(__dadd_rn((double)n, 1.0), (double)K));
   }
-  return (Coord<WIDE>)__double2ll_rn(__dmul_rn(__dadd_rn((double)n, 1.0), (double)pixels * 128.0));
 }
 
 // Set up one (possibly clipped) screen triangle; raster it here if small.
