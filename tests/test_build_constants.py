@@ -9,7 +9,7 @@ TUNING = {
     "VCT_BRICK_THREADS", "VCT_BRICK_ROUND",  # static_asserts bound them
     "VCT_MARCH_MIN_BLOCKS", "VCT_MARCH_WARPS", "VCT_SHADE_MIN_BLOCKS", "VCT_TRACE_BATCH_MIN_BLOCKS",
     "VCT_TRACE_BATCH_SHARE_MIN_BLOCKS", "VCT_MIP_TMA_MIN_BLOCKS",  # residency
-    "VCT_SHADOW_UNROLL", "VCT_FIRST_UNROLL", "VCT_TRACE_PIPE", "VCT_FAR_PIPE", "VCT_FAR_SHORT_TAIL", "VCT_LOD_FTZ",
+    "VCT_SHADOW_UNROLL", "VCT_FIRST_UNROLL", "VCT_TRACE_PIPE", "VCT_FAR_SHORT_TAIL", "VCT_LOD_FTZ",
     "VCT_SKIP_EMPTY_RGBA", "VCT_SKIP_MAX_LOD", "VCT_HEAVY_SPLIT", "VCT_FUSE_BRICK_MIPS"}  # forms of one result
 
 

@@ -1,12 +1,13 @@
-// k_trace.cu -- the ConeTracer in one kernel, a thread per pixel
-// (voxel_cone_tracing.frag main, :246-275, over the G-buffer): the FP32
-// software sampler, the voxel debug view and a batch's one-launch traces;
+// k_trace.cu -- the ConeTracer in one kernel (voxel_cone_tracing.frag main,
+// :246-275, over the G-buffer): the FP32 software sampler (k_trace_exact), the
+// voxel debug view (k_view) and a batch's one-launch traces (k_trace_batch*);
 // also the learned term's training targets and judge.  A frame with the
 // texture-unit sampler is traced by k_trace_frame.cu.
 //
-// A k_trace CTA covers a 16x8-pixel tile of 8x4 warp blocks, a one-launch
-// batch trace a 16x16 tile of them, so that neighbouring lanes march
-// neighbouring, nearly parallel cones and hit the same texture-cache lines.
+// A batch's one-launch trace takes a thread per pixel, in 16x16-pixel tiles of
+// 8x4 warp blocks where far fields are shared, so that neighbouring lanes
+// march neighbouring, nearly parallel cones and hit the same texture-cache
+// lines.
 #include <algorithm>
 
 #include "vct_cone.cuh"
@@ -21,10 +22,10 @@ namespace {
 // values in registers, so it is compiled for its own occupancy.
 constexpr int kTraceBatchMinBlocks = VCT_TRACE_BATCH_MIN_BLOCKS;
 
-// trace_diffuse, :140-168 (9 equal-weight cones); cone set SIX60 (no
+// trace_diffuse, :140-168 (9 equal-weight cones), texture unit; cone set SIX60 (no
 // reference counterpart): the normal plus 5 cones 60 degrees off it in the
 // same tangent frame, aperture 2 tan(30 deg), equal weights.
-template <int SAMPLER, bool ISO, int STORAGE>
+template <bool ISO>
 __device__ V3 trace_diffuse(const MapSet& m, int cone_set, V3 origin, V3 n) {
   const V3 o1 = normalize(tangent(n));
   const V3 o2 = normalize(cross(o1, n));
@@ -32,24 +33,24 @@ __device__ V3 trace_diffuse(const MapSet& m, int cone_set, V3 origin, V3 n) {
   if (cone_set == VCT_CONES_SIX60) {
     const float ap = kSixAperture;
     const V3 nn = normalize(n);
-    acc = trace_cone<SAMPLER, ISO, STORAGE>(m, origin, nn, ap, kMaxDistance);
+    acc = trace_cone<VCT_SAMPLER_HW, ISO, VCT_STORAGE_RGBA8>(m, origin, nn, ap, kMaxDistance);
 #pragma unroll 1
     for (int k = 0; k < 5; ++k) {
       const float sphi = m.sched->ring.sphi[k], cphi = m.sched->ring.cphi[k];
       const V3 d = nn * 0.5f + (o1 * cphi + o2 * sphi) * 0.86602540378f;
-      acc = acc + trace_cone<SAMPLER, ISO, STORAGE>(m, origin, d, ap, kMaxDistance);
+      acc = acc + trace_cone<VCT_SAMPLER_HW, ISO, VCT_STORAGE_RGBA8>(m, origin, d, ap, kMaxDistance);
     }
     return v3(acc.x, acc.y, acc.z) * (1.0f / 6.0f);
   }
   const V3 c1 = (o1 + o2) * 0.5f, c2 = (o1 - o2) * 0.5f;
-  acc = trace_cone<SAMPLER, ISO, STORAGE>(m, origin, n, kTan22_5, kMaxDistance);
+  acc = trace_cone<VCT_SAMPLER_HW, ISO, VCT_STORAGE_RGBA8>(m, origin, n, kTan22_5, kMaxDistance);
   // Side cones o1, -o1, o2, -o2, c1, -c1, c2, -c2 (:156-165), selected
   // arithmetically so that no local-memory array is needed.
 #pragma unroll 1
   for (int k = 0; k < 8; ++k) {
     const V3 b = k < 2 ? o1 : (k < 4 ? o2 : (k < 6 ? c1 : c2));
     const V3 side = (k & 1) ? -b : b;
-    acc = acc + trace_cone<SAMPLER, ISO, STORAGE>(m, origin, mixv(n, side, 0.5f), kTan22_5, kMaxDistance);
+    acc = acc + trace_cone<VCT_SAMPLER_HW, ISO, VCT_STORAGE_RGBA8>(m, origin, mixv(n, side, 0.5f), kTan22_5, kMaxDistance);
   }
   return v3(acc.x, acc.y, acc.z) * (1.0f / 9.0f);
 }
@@ -75,10 +76,6 @@ __device__ V3 trace_diffuse(const MapSet& m, int cone_set, V3 origin, V3 n) {
 // filter weights being 71 dB): 2x2 groups 80.6 dB, 4x2 groups 73.1 dB, with
 // the diffuse cones' two-level texture fetches cut from 238 to 60 and 31
 // per pixel.
-#ifndef VCT_FAR_PIPE
-#define VCT_FAR_PIPE 1
-#endif
-constexpr bool kFarPipe = VCT_FAR_PIPE != 0;  // software-pipelined far-field march
 #ifndef VCT_FIRST_UNROLL
 #define VCT_FIRST_UNROLL 1  // the per-pixel first samples of the diffuse cones: cones in flight together
 #endif
@@ -109,7 +106,6 @@ struct FarWarp {
 // cone ends (alpha 1, the grid's edge) takes the next job while the others
 // march on.  The march starts at the second step of the schedule (dist1,
 // diam1) with nothing accumulated.  Results go to fw.far[q * K + k].
-template <bool ISO>
 __device__ void far_fields(const MapSet& m, FarWarp& fw, int cone_set, int nq, float dist1, float diam1) {
   const int lane = threadIdx.x & 31;
   const int K = cone_set == VCT_CONES_SIX60 ? 6 : 9;
@@ -170,119 +166,68 @@ __device__ void far_fields(const MapSet& m, FarWarp& fw, int cone_set, int nq, f
   int res = 0;
   bool active = false;
   V3 origin = v3(0.f, 0.f, 0.f), dir = v3(0.f, 0.f, 1.f), ad = v3(0.f, 0.f, 1.f);
-  int ix = 1, iy = 3, iz = 5;
   float dist = 0.f, diam = 0.f, stop = 0.f;
   bool check = false;
   float4 acc = f4(0.f, 0.f, 0.f, 0.f);
-  if constexpr (kFarPipe && !ISO) {
-    // Software-pipelined like trace_cone_pipe (anisotropic maps; the
-    // isotropic march below samples one chain): a lane computes its next step
-    // (position, lod, empty-space test with its occupancy load) while the
-    // current step's texture fetches are in flight, and issues the next
-    // step's fetches as soon as the current one is added.  Same samples, same
-    // arithmetic as the loop below.
-    float mip = 0.f;
-    bool live = false;
-    Taps t;
-    for (;;) {
-      const unsigned need = __ballot_sync(0xffffffffu, !active);
-      if (need && next < n_jobs) {
-        const int job = next + __popc(need & ((1u << lane) - 1u));
-        if (!active && job < n_jobs) {
-          const int jo = fw.order[job];
-          const int k = jo / nq, q = jo - k * nq;
-          res = q * K + k;
-          const float4 jb = fw.job[jo];
-          dir = v3(jb.x, jb.y, jb.z);
-          stop = jb.w;
-          origin = v3(fw.origin[q][0], fw.origin[q][1], fw.origin[q][2]);
-          ix = dir.x < 0.0f ? 0 : 1;
-          iy = dir.y < 0.0f ? 2 : 3;
-          iz = dir.z < 0.0f ? 4 : 5;
-          ad = vabs(dir);
-          dist = dist1;
-          diam = diam1;
-          check = !march_sane(origin, dir, stop);
-          acc = f4(0.f, 0.f, 0.f, 0.f);
-          active = dist < stop;
-          if (!active) {
-            fw.far[res] = acc;
-          } else {
-            const V3 sp = march_pos(origin, dir, dist);
-            mip = cone_lod(diam * cube_res);
-            live = !(kSkipEmptyRGBA && m.skip_empty && mip < kSkipMaxLod && sample_empty(m, sp, mip)) &&
-                   !(check && !u_sane(sp));
-            if (live) issue_taps<false>(m, sp, octant(dir), ad, mip, t);
-          }
-        }
-        next += __popc(need);
-      }
-      if (!__any_sync(0xffffffffu, active)) break;
-      if (active) {
-        const float step = fmaxf(diam * 0.5f, voxel_size);
-        const float dist_n = dist + step;
-        const float diam_n = dist_n * ap;
-        const V3 sp_n = march_pos(origin, dir, dist_n);
-        const bool more = dist_n < stop;
-        const float mip_n = cone_lod(diam_n * cube_res);
-        const bool live_n = more &&
-                            !(kSkipEmptyRGBA && m.skip_empty && mip_n < kSkipMaxLod && sample_empty(m, sp_n, mip_n)) &&
-                            !(check && !u_sane(sp_n));
-        if (live) acc = fma4(combine_taps(t, ad, mip), 1.0f - acc.w, acc);
-        if (!(acc.w < 1.0f) || !more) {
+  // Software-pipelined like trace_cone_pipe: a lane computes its next step
+  // (position, lod, empty-space test with its occupancy load) while the
+  // current step's texture fetches are in flight, and issues the next
+  // step's fetches as soon as the current one is added.  Same samples, same
+  // arithmetic as trace_cone.
+  float mip = 0.f;
+  bool live = false;
+  Taps t;
+  for (;;) {
+    const unsigned need = __ballot_sync(0xffffffffu, !active);
+    if (need && next < n_jobs) {
+      const int job = next + __popc(need & ((1u << lane) - 1u));
+      if (!active && job < n_jobs) {
+        const int jo = fw.order[job];
+        const int k = jo / nq, q = jo - k * nq;
+        res = q * K + k;
+        const float4 jb = fw.job[jo];
+        dir = v3(jb.x, jb.y, jb.z);
+        stop = jb.w;
+        origin = v3(fw.origin[q][0], fw.origin[q][1], fw.origin[q][2]);
+        ad = vabs(dir);
+        dist = dist1;
+        diam = diam1;
+        check = !march_sane(origin, dir, stop);
+        acc = f4(0.f, 0.f, 0.f, 0.f);
+        active = dist < stop;
+        if (!active) {
           fw.far[res] = acc;
-          active = false;
         } else {
-          dist = dist_n;
-          diam = diam_n;
-          mip = mip_n;
-          live = live_n;
-          if (live) issue_taps<false>(m, sp_n, octant(dir), ad, mip, t);
+          const V3 sp = march_pos(origin, dir, dist);
+          mip = cone_lod(diam * cube_res);
+          live = !(kSkipEmptyRGBA && m.skip_empty && mip < kSkipMaxLod && sample_empty(m, sp, mip)) &&
+                 !(check && !u_sane(sp));
+          if (live) issue_taps<false>(m, sp, octant(dir), ad, mip, t);
         }
       }
+      next += __popc(need);
     }
-  } else {
-    for (;;) {
-      const unsigned need = __ballot_sync(0xffffffffu, !active);
-      if (need && next < n_jobs) {
-        const int job = next + __popc(need & ((1u << lane) - 1u));
-        if (!active && job < n_jobs) {
-          const int jo = fw.order[job];
-          const int k = jo / nq, q = jo - k * nq;
-          res = q * K + k;
-          const float4 jb = fw.job[jo];
-          dir = v3(jb.x, jb.y, jb.z);
-          stop = jb.w;
-          origin = v3(fw.origin[q][0], fw.origin[q][1], fw.origin[q][2]);
-          ix = dir.x < 0.0f ? 0 : 1;
-          iy = dir.y < 0.0f ? 2 : 3;
-          iz = dir.z < 0.0f ? 4 : 5;
-          ad = vabs(dir);
-          dist = dist1;
-          diam = diam1;
-          check = !march_sane(origin, dir, stop);
-          acc = f4(0.f, 0.f, 0.f, 0.f);
-          active = dist < stop;
-          if (!active) fw.far[res] = acc;
-        }
-        next += __popc(need);
-      }
-      if (!__any_sync(0xffffffffu, active)) break;
-      if (active) {
-        const V3 sp = march_pos(origin, dir, dist);
-        const float mip = cone_lod(diam * cube_res);
-        if (!(kSkipEmptyRGBA && m.skip_empty && mip < kSkipMaxLod && sample_empty(m, sp, mip)) &&
-            !(check && !u_sane(sp))) {
-          const float4 smp = sample_voxel<VCT_SAMPLER_HW, ISO, VCT_STORAGE_RGBA8, false>(m, sp, ix, iy, iz, ad, mip);
-          acc = fma4(smp, 1.0f - acc.w, acc);
-        }
-        const float step = fmaxf(diam * 0.5f, voxel_size);
-        dist += step;
-        diam = dist * ap;
-        if (!(acc.w < 1.0f) || !(dist < stop)) {
-          fw.far[res] = acc;
-          active = false;
-        }
+    if (!__any_sync(0xffffffffu, active)) break;
+    if (active) {
+      const float step = fmaxf(diam * 0.5f, voxel_size);
+      const float dist_n = dist + step;
+      const float diam_n = dist_n * ap;
+      const V3 sp_n = march_pos(origin, dir, dist_n);
+      const bool more = dist_n < stop;
+      const float mip_n = cone_lod(diam_n * cube_res);
+      const bool live_n = more &&
+                          !(kSkipEmptyRGBA && m.skip_empty && mip_n < kSkipMaxLod && sample_empty(m, sp_n, mip_n)) &&
+                          !(check && !u_sane(sp_n));
+      if (live) acc = fma4(combine_taps(t, ad, mip), 1.0f - acc.w, acc);
+      if (!(acc.w < 1.0f) || !more) {
+        fw.far[res] = acc;
+        active = false;
+      } else {
+        dist = dist_n;
+        diam = diam_n;
+        mip = mip_n;
+        live = live_n;
+        if (live) issue_taps<false>(m, sp_n, octant(dir), ad, mip, t);
       }
     }
   }
@@ -291,7 +236,6 @@ __device__ void far_fields(const MapSet& m, FarWarp& fw, int cone_set, int nq, f
 // trace_diffuse with the group's far fields (far: this group's K results):
 // each cone takes its first sample (step 0 of trace_cone) itself, then the
 // far field behind it.
-template <bool ISO>
 __device__ V3 trace_diffuse_shared(const MapSet& m, int cone_set, V3 origin, V3 n, const float4* far) {
   const V3 o1 = normalize(tangent(n));
   const V3 o2 = normalize(cross(o1, n));
@@ -305,20 +249,20 @@ __device__ V3 trace_diffuse_shared(const MapSet& m, int cone_set, V3 origin, V3 
     // (the origin is a surface point inside the grid and the first step
     // three voxels: the sample position is sane, and one beyond the grid's
     // exit margin reads border texels, 0, as the unshortened march would)
-    float4 c = cone_first<ISO>(m, origin, dir, e);
+    float4 c = cone_first<false>(m, origin, dir, e);
     if (c.w < 1.0f) c = fma4(far[k], 1.0f - c.w, c);
     acc = acc + c;
   }
   return v3(acc.x, acc.y, acc.z) * (1.0f / (float)K);
 }
 
-// Shades pixel (px, py) of one frame (main, voxel_cone_tracing.frag:246-275).
-template <int SAMPLER, bool ISO, int STORAGE, bool SHARE = false>
+// Shades pixel (px, py) of one batch scene's frame (main,
+// voxel_cone_tracing.frag:246-275): texture unit, anisotropic RGBA8 maps.
+template <bool SHARE = false>
 __device__ __forceinline__ void trace_px(const SceneParams& sp, const CameraParams& cp, const MapSet& m,
                                          const TraceParams& tp, const float4* __restrict__ gb_pos,
-                                         const float4* __restrict__ gb_nrm, uchar4* __restrict__ frame,
-                                         float4* __restrict__ frame_f32, int px, int py,
-                                         const float4* far = nullptr) {
+                                         const float4* __restrict__ gb_nrm, uchar4* __restrict__ frame, int px,
+                                         int py, const float4* far = nullptr) {
   if (px >= cp.W || py >= cp.H) return;
   const size_t p = (size_t)py * cp.W + px;
   float4 out = f4(0.15f, 0.25f, 0.25f, 1.0f);  // glClearColor, renderer.cpp:398
@@ -340,23 +284,23 @@ __device__ __forceinline__ void trace_px(const SceneParams& sp, const CameraPara
           const float4 d = tp.diffuse_in[p];
           fd = mulv(mat3v(mat.diffuse), v3(d.x, d.y, d.z));
         } else if (SHARE && far) {
-          fd = mulv(mat3v(mat.diffuse), trace_diffuse_shared<ISO>(m, tp.cone_set, pos, nrm, far));
+          fd = mulv(mat3v(mat.diffuse), trace_diffuse_shared(m, tp.cone_set, pos, nrm, far));
         } else {
-          fd = mulv(mat3v(mat.diffuse), trace_diffuse<SAMPLER, ISO, STORAGE>(m, tp.cone_set, pos, nrm));
+          fd = mulv(mat3v(mat.diffuse), trace_diffuse<false>(m, tp.cone_set, pos, nrm));
         }
       }
       if (tp.enable_direct)
-        fdir = direct_light<SAMPLER, ISO, STORAGE, false>(sp, m, tp.enable_shadow, mat, pos, nrm, view_dir, nullptr, 0);
+        fdir = direct_light<false>(sp, m, tp.enable_shadow, mat, pos, nrm, view_dir, nullptr, 0);
       const float sap = specular_aperture(mat.shininess);
       if (tp.enable_specular) {
         const V3 sd = normalize(reflect(-view_dir, nrm));
-        const float4 c = trace_cone<SAMPLER, ISO, STORAGE>(m, pos, sd, sap, kMaxDistance);
+        const float4 c = trace_cone<VCT_SAMPLER_HW, false, VCT_STORAGE_RGBA8>(m, pos, sd, sap, kMaxDistance);
         fs = mulv(mat3v(mat.specular), v3(c.x, c.y, c.z));
       }
       V3 f = fs + fd + fdir;
       if (refracts(mat) && tp.enable_specular) {
         const V3 rd = refract(view_dir, nrm, 1.0f / mat.ior);
-        const float4 c = trace_cone<SAMPLER, ISO, STORAGE>(m, pos, rd, sap, kMaxDistance);
+        const float4 c = trace_cone<VCT_SAMPLER_HW, false, VCT_STORAGE_RGBA8>(m, pos, rd, sap, kMaxDistance);
         const V3 tr = mulv(mat3v(mat.transmittance), v3(c.x, c.y, c.z));
         f = tr * (1.0f - mat.dissolve) + f * mat.dissolve;
       }
@@ -364,7 +308,6 @@ __device__ __forceinline__ void trace_px(const SceneParams& sp, const CameraPara
     }
   }
   frame[p] = make_uchar4(unorm8(out.x), unorm8(out.y), unorm8(out.z), unorm8(out.w));
-  if (frame_f32) frame_f32[p] = out;
 }
 
 // The voxel debug view (:253-257): one lookup a pixel.
@@ -490,8 +433,7 @@ __global__ void __launch_bounds__((9 + 1 + kExactLights) * 32, 4)
       fd = mulv(mat3v(mat.diffuse), d);
     }
     if (tp.enable_direct)
-      fdir = direct_light<VCT_SAMPLER_EXACT, ISO, STORAGE, true>(sp, m, tp.enable_shadow, mat, pos, nrm, view_dir,
-                                                                 &s_occ[0][lane], 32);
+      fdir = direct_light<true>(sp, m, tp.enable_shadow, mat, pos, nrm, view_dir, &s_occ[0][lane], 32);
     if (tp.enable_specular) fs = mulv(mat3v(mat.specular), cone(9));
     V3 f = fs + fd + fdir;
     if (refracts(mat) && tp.enable_specular) {
@@ -508,13 +450,12 @@ __global__ void __launch_bounds__((9 + 1 + kExactLights) * 32, 4)
 // rows starting at an even frame row; share_tile_px) first picks each group's
 // representative (its first pixel, row by row, whose diffuse cones are
 // traced) and the pixels that share with it, marches the groups' far fields
-// together (far_fields), then shades its pixels as k_trace does.  Called by
+// together (far_fields), then shades its pixels (trace_px).  Called by
 // all 32 lanes of a warp together; fw is the warp's shared-memory block.
-template <bool ISO>
 __device__ __forceinline__ void trace_px_share(const SceneParams& sp, const CameraParams& cp, const MapSet& m,
                                                const TraceParams& tp, const float4* __restrict__ gb_pos,
                                                const float4* __restrict__ gb_nrm, uchar4* __restrict__ frame,
-                                               float4* __restrict__ frame_f32, int px, int py, FarWarp& fw) {
+                                               int px, int py, FarWarp& fw) {
   const int lane = threadIdx.x & 31;
   bool valid = false;
   V3 pos = v3(0.f, 0.f, 0.f), nrm = v3(0.f, 0.f, 1.f);
@@ -548,10 +489,9 @@ __device__ __forceinline__ void trace_px_share(const SceneParams& sp, const Came
   const float voxel_size = 1.0f / (float)m.N;
   const float dist0 = 3.0f * voxel_size;
   const float dist1 = dist0 + fmaxf(dist0 * ap * 0.5f, voxel_size);
-  if (repmask) far_fields<ISO>(m, fw, tp.cone_set, __popc(repmask), dist1, dist1 * ap);
+  if (repmask) far_fields(m, fw, tp.cone_set, __popc(repmask), dist1, dist1 * ap);
   __syncwarp();
-  trace_px<VCT_SAMPLER_HW, ISO, VCT_STORAGE_RGBA8, true>(sp, cp, m, tp, gb_pos, gb_nrm, frame, frame_f32, px, py,
-                                                         share ? fw.far + slot * K : nullptr);
+  trace_px<true>(sp, cp, m, tp, gb_pos, gb_nrm, frame, px, py, share ? fw.far + slot * K : nullptr);
   __syncwarp();  // fw is free for the warp's next use
 }
 
@@ -570,11 +510,9 @@ __device__ __forceinline__ void trace_px_share(const SceneParams& sp, const Came
 __shared__ BatchScene s_batch_scene;
 __shared__ CameraParams s_batch_cam;
 
-template <bool ISO>
 __device__ VCT_BATCH_PX_FN void trace_batch_px(const float4* __restrict__ gb_pos, const float4* __restrict__ gb_nrm,
                                             uchar4* __restrict__ frame, int px, int py) {
-  trace_px<VCT_SAMPLER_HW, ISO, VCT_STORAGE_RGBA8>(s_batch_scene.sp, s_batch_cam, s_batch_scene.ms,
-                                                   s_batch_scene.tp, gb_pos, gb_nrm, frame, nullptr, px, py);
+  trace_px(s_batch_scene.sp, s_batch_cam, s_batch_scene.ms, s_batch_scene.tp, gb_pos, gb_nrm, frame, px, py);
 }
 
 // trace_px_share on the CTA's current batch scene (k_trace_batch_share);
@@ -582,8 +520,8 @@ __device__ VCT_BATCH_PX_FN void trace_batch_px(const float4* __restrict__ gb_pos
 __device__ VCT_BATCH_PX_FN void trace_batch_px_share(const float4* __restrict__ gb_pos,
                                                   const float4* __restrict__ gb_nrm, uchar4* __restrict__ frame,
                                                   int px, int py, FarWarp& fw) {
-  trace_px_share<false>(s_batch_scene.sp, s_batch_cam, s_batch_scene.ms, s_batch_scene.tp, gb_pos, gb_nrm, frame,
-                        nullptr, px, py, fw);
+  trace_px_share(s_batch_scene.sp, s_batch_cam, s_batch_scene.ms, s_batch_scene.tp, gb_pos, gb_nrm, frame, px, py,
+                 fw);
 }
 
 // The 16x16 tiles of every scene of a batch in one persistent launch.  With
@@ -592,7 +530,6 @@ __device__ VCT_BATCH_PX_FN void trace_batch_px_share(const float4* __restrict__ 
 // keeps its current scene's descriptor and camera in shared memory, so the
 // shading code addresses them at fixed offsets (as kernel parameters are in
 // the one-scene kernel) instead of holding pointers in registers.
-template <bool ISO>
 __global__ void __launch_bounds__(256, kTraceBatchMinBlocks) k_trace_batch(BatchWork w, BatchBuffers bb) {
   __shared__ uint32_t s_next;
   __shared__ int s_cur;
@@ -621,8 +558,8 @@ __global__ void __launch_bounds__(256, kTraceBatchMinBlocks) k_trace_batch(Batch
       if (threadIdx.x == 0) s_cur = s;
     }
     const uint32_t lt = g - __ldg(w.prefix + s), tiles_x = (uint32_t)(s_sc.W + 15) / 16;
-    trace_batch_px<ISO>(bb.rb.gb_pos + s_sc.px_base, bb.rb.gb_nrm + s_sc.px_base, bb.frame + s_sc.px_base,
-                        (int)(lt % tiles_x) * 16 + (threadIdx.x & 15), (int)(lt / tiles_x) * 16 + (threadIdx.x >> 4));
+    trace_batch_px(bb.rb.gb_pos + s_sc.px_base, bb.rb.gb_nrm + s_sc.px_base, bb.frame + s_sc.px_base,
+                   (int)(lt % tiles_x) * 16 + (threadIdx.x & 15), (int)(lt / tiles_x) * 16 + (threadIdx.x >> 4));
     if (w.queue) {
       __syncthreads();  // every thread has read s_next
       if (threadIdx.x == 0) s_next = atomicAdd(w.queue, 1u);
@@ -635,7 +572,7 @@ __global__ void __launch_bounds__(256, kTraceBatchMinBlocks) k_trace_batch(Batch
 }
 
 // k_trace_batch with shared far fields (the batch's far_share): every 16x16
-// tile is eight 8x4 warps, as in k_trace_share, so each scene's frame equals
+// tile is eight 8x4 warps, as in k_march and k_shade, so each scene's frame equals
 // a Renderer's with far_share 1.  Anisotropic maps (the batch's).
 #ifndef VCT_TRACE_BATCH_SHARE_MIN_BLOCKS
 #define VCT_TRACE_BATCH_SHARE_MIN_BLOCKS 4
@@ -712,9 +649,9 @@ __global__ void __launch_bounds__(256, SHARE ? kTraceBatchShareMinBlocks : kTrac
   const float4* gn = bb.rb.gb_nrm + s_sc.px_base;
   uchar4* fr = bb.frame + s_sc.px_base;
   if constexpr (SHARE)
-    trace_px_share<false>(s_sc.sp, s_cam, s_sc.ms, s_sc.tp, gp, gn, fr, nullptr, px, py, s_far[threadIdx.x >> 5]);
+    trace_px_share(s_sc.sp, s_cam, s_sc.ms, s_sc.tp, gp, gn, fr, px, py, s_far[threadIdx.x >> 5]);
   else
-    trace_px<VCT_SAMPLER_HW, false, VCT_STORAGE_RGBA8>(s_sc.sp, s_cam, s_sc.ms, s_sc.tp, gp, gn, fr, nullptr, px, py);
+    trace_px(s_sc.sp, s_cam, s_sc.ms, s_sc.tp, gp, gn, fr, px, py);
 }
 
 template <int SAMPLER, bool ISO, int STORAGE>
@@ -748,7 +685,7 @@ __global__ void __launch_bounds__(256) k_trace_points(MapSet m, int cone_set, fl
   if (i >= n) return;
   float* q = samples + (size_t)i * 12;
   const V3 pos = v3(q[0], q[1], q[2]), nrm = v3(q[3], q[4], q[5]);
-  const V3 d = trace_diffuse<VCT_SAMPLER_HW, ISO, VCT_STORAGE_RGBA8>(m, cone_set, pos, nrm);
+  const V3 d = trace_diffuse<ISO>(m, cone_set, pos, nrm);
   q[9] = d.x;
   q[10] = d.y;
   q[11] = d.z;
@@ -868,7 +805,7 @@ cudaError_t launch_trace_batch(const BatchWork& tiles, const BatchBuffers& bb, c
   }
   const int per_sm = std::min(std::max(shape.trace_ctas_per_sm, 1), kTraceBatchMinBlocks);
   const unsigned grid = (unsigned)std::max(1, std::min<int>(sms * per_sm, (int)tiles.total));
-  k_trace_batch<false><<<grid, 256, 0, st>>>(w, bb);
+  k_trace_batch<<<grid, 256, 0, st>>>(w, bb);
   if (launches) ++*launches;
   return cudaGetLastError();
 }

@@ -384,8 +384,8 @@ __global__ void __launch_bounds__(256, SHARE ? VCT_SHADE_MIN_BLOCKS : 6)
     if (tp.enable_diffuse) fd = mulv(mat3v(mat.diffuse), fd);
     const V3 view_dir = normalize(v3(g0.x, g0.y, g0.z) - v3(cp.cam_pos[0], cp.cam_pos[1], cp.cam_pos[2]));
     if (tp.enable_direct)
-      fdir = direct_light<VCT_SAMPLER_HW, ISO, VCT_STORAGE_RGBA8, true>(sp, m, tp.enable_shadow, mat, pos, nrm, view_dir,
-                                                                        tw.shadow + p, (size_t)cp.W * cp.H);
+      fdir = direct_light<true>(sp, m, tp.enable_shadow, mat, pos, nrm, view_dir, tw.shadow + p,
+                                (size_t)cp.W * cp.H);
     if (tp.enable_specular) {
       const float4 c = tw.specular[p];
       fs = mulv(mat3v(mat.specular), v3(c.x, c.y, c.z));

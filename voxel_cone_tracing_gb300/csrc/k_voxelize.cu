@@ -1267,6 +1267,7 @@ __global__ void __launch_bounds__(kThreads, 7)
   });
 }
 
+// CTAs of a kernel resident on one SM.
 template <class K>
 int resident_per_sm(K kern) {
   int f = 1;
@@ -1348,8 +1349,6 @@ void dispatch_bricks(int mode, int storage, bool attr, F&& f) {
     else f(RAS(), F16());
   }
 }
-
-// CTAs of a kernel resident on one SM (cached per kernel).
 
 cudaError_t launch_voxelize(const SceneParams& sp, int N, int mode, int storage, const VoxBuffers& vb,
                             cudaSurfaceObject_t l0, cudaStream_t st, int* launches, const InjGrids* inj) {

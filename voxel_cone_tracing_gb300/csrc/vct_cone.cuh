@@ -659,9 +659,10 @@ __device__ __forceinline__ void light_dir(const SceneParams& sp, int i, V3 pos, 
 }
 
 // direct_light, :175-218.
-// SPLIT: the shadow cones' occlusion comes from `shadow` (one value per
-// light, `stride` apart), else they are traced here.
-template <int SAMPLER, bool ISO, int STORAGE, bool SPLIT>
+// SPLIT: the shadow cones' occlusion comes from `occlusion` (one value per
+// light, `stride` apart), else they are traced here through a batch's maps
+// (texture unit, anisotropic RGBA8, alpha chains, empty-space skipping).
+template <bool SPLIT>
 __device__ V3 direct_light(const SceneParams& sp, const MapSet& m, int enable_shadow, const vct_material_data& mat,
                            V3 pos, V3 nrm, V3 view_dir, const float* occlusion, size_t stride) {
   V3 result = v3(0.f, 0.f, 0.f);
@@ -677,10 +678,7 @@ __device__ V3 direct_light(const SceneParams& sp, const MapSet& m, int enable_sh
     if (enable_shadow) {
       float occ;
       if constexpr (SPLIT) occ = occlusion[i * stride];
-      else if constexpr (SAMPLER == VCT_SAMPLER_HW)  // (a batch's maps: alpha chains, empty-space skipping)
-        occ = trace_shadow<SAMPLER, ISO, STORAGE, true, true>(m, m.sched->shadow.group, pos, ld, d);
-      else if (m.skip_empty) occ = trace_shadow<SAMPLER, ISO, STORAGE, false, true>(m, m.sched->shadow.group, pos, ld, d);
-      else occ = trace_shadow<SAMPLER, ISO, STORAGE, false, false>(m, m.sched->shadow.group, pos, ld, d);
+      else occ = trace_shadow<VCT_SAMPLER_HW, false, VCT_STORAGE_RGBA8, true, true>(m, m.sched->shadow.group, pos, ld, d);
       shadow = fmaxf(0.0f, 1.0f - occ);
     }
     const float lambert = fmaxf(dot(ld, nrm), 0.0f);
