@@ -360,7 +360,7 @@ vct_status vct_mlp_get_judge(vct_renderer* r, vct_mlp_judge_report* out);
  * their frame loop (those calls can synchronise the device and stall the
  * frame, or are simply not theirs to make).  Everything below is caller
  * memory; the voxelizer's intermediates live in a fixed device array inside
- * the library (about 9 MB per GPU, held while the library is loaded).
+ * the library (29 MB per GPU, held while the library is loaded).
  *
  * A mesh already on the device: vertices (vert_data_t layout), u32
  * indices, a material id per triangle (< n_materials), its model matrix. */

@@ -73,6 +73,9 @@ struct NoAllocScratch {
   alignas(16) unsigned char heavy_acc[kNaSlots * kNaSlotBytes];
 };
 
+// (the 29 MB that include/vct.h tells callers who budget device memory)
+static_assert(sizeof(NoAllocScratch) > 28 * 1000 * 1000 && sizeof(NoAllocScratch) <= 29 * 1000 * 1000,
+              "the documented size of the voxelizer's scratch");
 static __device__ __align__(256) unsigned char g_scratch[sizeof(NoAllocScratch)];
 
 std::once_flag g_identity_once;
