@@ -87,7 +87,8 @@ __device__ __forceinline__ void level_corners(const MlpParams& p, int l, V3 pos,
 // Hash features of one (row, level) pair; `tab`: the level's entries (global
 // or shared memory).  (Loading a pair of corners along x as one 8-byte word
 // where they are neighbours, 6 loads instead of 8, was slower: 432 -> 465 us
-// for the bench frame's inference, whose encoders are bound by instructions.)
+// for the bench frame's inference, whose encoders wait for the gathers with
+// issue 65% busy: the choice between the two forms costs instructions.)
 __device__ __forceinline__ float2 corner_features(const Corners& c, const uint32_t* tab) {
   float f0 = 0.f, f1 = 0.f;
 #pragma unroll

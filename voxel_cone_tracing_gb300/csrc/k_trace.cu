@@ -344,7 +344,7 @@ __global__ void __launch_bounds__(256) k_view(SceneParams sp, CameraParams cp, c
 // idle: a CTA takes an 8x4-pixel block with a warp per cone -- the diffuse
 // cones, the specular (and refracted) one, the lights' shadow cones shared by
 // up to kExactLights warps -- and its first warp puts them together.
-// 320x180, 64^3, one light (GB300, trace): 1741 us with a thread per pixel
+// 320x180, 64^3, one light (GB300, the trace alone): 1741 us with a thread per pixel
 // (255 registers, 8 warps an SM), 958 as here at 128 registers, 700 at 48,
 // 647 at 40 (it spills 0.8 KB; more resident warps are worth it).  Bound by
 // instructions (unpacking and weighting texels: ALU pipe 56%).
